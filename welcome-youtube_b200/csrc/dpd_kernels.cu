@@ -944,9 +944,10 @@ __device__ __noinline__ int pair_hist_bin(float2 pi, float2 pj, double L, double
 // image may be another: the counts are those of binning every pair in FP64.
 // The counts go to shared memory: per lane a column of its own (no two lanes
 // of a warp on one address or bank) while that fits, else one column per CTA;
-// the CTAs' sums are added to the global bins once.  786,432 beads, 30 bins to
-// 3.0: 5.77 ms before (FP64 hypot and division per pair, one global atomic per
-// pair); see the launch for the figure of this form.
+// the CTAs' sums are added to the global bins once.  786,432 beads at density 3,
+// 30 bins to 3.0, all beads and the tails alone: 0.17 ms a call on average,
+// against 5.77 ms with FP64 hypot and division per pair and one global atomic
+// per pair.
 template <bool LANES>
 __global__ void __launch_bounds__(BEAD_TPB) k_pair_hist(Bufs b, int cur, const RepDev *__restrict__ reps,
                                                         const Chunk *__restrict__ ch, int rep_index, int ta, int tb,
