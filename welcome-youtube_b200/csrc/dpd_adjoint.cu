@@ -34,6 +34,8 @@
 //
 // Stirring (f_x,i = A sin(2 pi k y_i) minus its replica mean): the VJP on y_m
 // is A 2 pi k cos(2 pi k y_m) (g_x,m - mean of g_x), the mean from k_gsum.
+#include <algorithm>
+
 #include "dpd_device.cuh"
 
 #define NGRAD DPD_NGRAD
@@ -128,103 +130,250 @@ __global__ void __launch_bounds__(BEAD_TPB) k_gsum(const RepDev *__restrict__ re
     if (lane_id() == 0 && v != 0.0) atomicAdd(gsum + c.rep, v);
 }
 
-__global__ void __launch_bounds__(BEAD_TPB) k_force_vjp(StateView sv, long long step, const RepDev *__restrict__ reps,
-                                                        const Chunk *__restrict__ ch, const float2 *__restrict__ g,
-                                                        float2 *__restrict__ xbar, float2 *__restrict__ vbar,
-                                                        double *__restrict__ grad, const double *__restrict__ gsum,
-                                                        const long long *__restrict__ step_base) {
-    if (step_base) step += *step_base;  // the step relative to a step number kept on the device
+#define VJP_TPB 256
+#define VJP_LIST 32         // hits a bead collects before they are evaluated
+#define VJP_TYPES 4         // types whose pairs have lane-private gradient sums
+#define VJP_COMBOS (VJP_TYPES * (VJP_TYPES + 1) / 2)
+
+// LPB lanes share a bead: they take its 3 x 3 cells' slots in turn (cells are
+// column-major: three contiguous ranges, and three more where the rows wrap),
+// list the ones inside the cutoff, then take the listed pairs in turn, so that
+// the noise and the derivative run on lanes that all have a pair.  Each pair is
+// evaluated by both of its beads: every bead's sums are made by its own lanes
+// in a fixed order, with no atomics on floats.  The sums of the parameters'
+// gradient are FP64: per lane and pair of types in shared memory for the first
+// four types (no two lanes on one word), through an atomic for the others.
+// A CTA takes a run of consecutive tasks (256 / LPB beads of a chunk) and hands
+// its gradient sums over when the replica changes and at its end.
+// What bounds it: instruction issue (175 warp instructions a bead at density 4,
+// 2.2 of 4 a cycle: half of them the 12.6 evaluations, 40 of whose 130
+// instructions are the noise) and the fullest list of a warp, 1.6 times the
+// mean.  24 boxes of 65,536 beads: 374 us, against 939 with a thread per bead
+// and an FP64 shared atomic per pair; one box: 32 against 68, of 16,384: 14
+// against 60, of 4,096: 11 against 61.
+template <int LPB, int MINB>
+__global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long long step, const RepDev *__restrict__ reps,
+                                                       const Chunk *__restrict__ ch, int ntask,
+                                                       const float2 *__restrict__ g, float2 *__restrict__ xbar,
+                                                       float2 *__restrict__ vbar,
+                                                       double *__restrict__ grad, const double *__restrict__ gsum,
+                                                       const long long *__restrict__ step_base) {
+    constexpr int BEADS = VJP_TPB / LPB;
+    __shared__ int list[BEADS][VJP_LIST + 1];
+    __shared__ double acc[VJP_COMBOS][VJP_TPB];
     __shared__ double sgrad[NGRAD];
-    for (int k = threadIdx.x; k < NGRAD; k += blockDim.x) sgrad[k] = 0.0;
-    __syncthreads();
-    const Chunk c = ch[blockIdx.x];
-    const RepDev &R = reps[c.rep];
-    const int d = c.begin + (int)threadIdx.x;
-    if (d < c.end) {
-        const float2 pi = sv.pos[d], vi = sv.vt[d], gi2 = g[d];
-        const uint32_t tgi = sv.tg[d], gi = tgi & GID_MASK;
-        const int ti = (int)(tgi >> TYPE_SHIFT);
-        const float L = R.L, h = R.halfL, gam = R.gamma, s = sdt_at(R, step);
-        const NoiseKey nk = make_noise_key(R, step);
+    __shared__ float a_sh[DPD_MAXT * DPD_MAXT];
+    const int tid = (int)threadIdx.x, lane = (int)lane_id(), sub = tid % LPB, bead = tid / LPB;
+    for (int k = tid; k < NGRAD; k += VJP_TPB) sgrad[k] = 0.0;
+#pragma unroll
+    for (int k = 0; k < VJP_COMBOS; k++) acc[k][tid] = 0.0;
+    double ggam = 0.0, gkb = 0.0;
+    if (step_base) step += *step_base;  // the step relative to a step number kept on the device
+    const int t0 = (int)((long long)ntask * blockIdx.x / gridDim.x);
+    const int t1 = (int)((long long)ntask * (blockIdx.x + 1) / gridDim.x);
+    int rep = -1;
+    float gam = 0.0f, s = 0.0f, sg = 0.0f;  // sg = s / (2 gamma): d s / d gamma
+    NoiseKey nk;
+    // the CTA's gradient sums of replica `rep`, added to the global ones
+    auto hand_over = [&]() {
+        auto add = [&](double v, int slot) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0 && v != 0.0) atomicAdd(&sgrad[slot], v);
+        };
+        int k = 0;
+#pragma unroll 1
+        for (int i = 0; i < VJP_TYPES; i++)
+#pragma unroll 1
+            for (int j = i; j < VJP_TYPES; j++, k++) {
+                add(acc[k][tid], i * DPD_MAXT + j);
+                acc[k][tid] = 0.0;
+            }
+        add(ggam, DPD_MAXT * DPD_MAXT);
+        add(gkb, DPD_MAXT * DPD_MAXT + 1);
+        ggam = gkb = 0.0;
+        __syncthreads();
+        for (int q = tid; q < NGRAD; q += VJP_TPB)
+            if (sgrad[q] != 0.0) {
+                atomicAdd(&grad[(size_t)rep * NGRAD + q], sgrad[q]);
+                sgrad[q] = 0.0;
+            }
+        __syncthreads();
+    };
+    for (int task = t0; task < t1; task++) {
+        const Chunk c = ch[task / LPB];
+        const RepDev &R = reps[c.rep];
+        if (c.rep != rep) {  // uniform over the CTA
+            if (rep >= 0) hand_over();
+            rep = c.rep;
+            if (tid < DPD_MAXT * DPD_MAXT) a_sh[tid] = R.a[tid];
+            gam = R.gamma;
+            s = sdt_at(R, step);
+            sg = gam > 0.0f ? s / (2.0f * gam) : 0.0f;
+            nk = make_noise_key(R, step);
+            __syncthreads();
+        }
+        const int d = c.begin + task % LPB * BEADS + bead;
+        const bool act = d < c.end;
+        const float L = R.L, h = R.halfL;
         const int ncx = R.ncx, ncy = R.ncy;
-        const int32_t *cs = sv.cstart + R.c0;
-        int cx, cy;
-        cell_xy(R, pi.x, pi.y, cx, cy);
+        const int32_t *__restrict__ cs = sv.cstart + R.c0;
+        float2 pi = make_float2(0.f, 0.f), vi = pi, gi2 = pi;
+        uint32_t tgi = 0;
+        int cx = 0, cy = 0;
+        if (act) {
+            pi = sv.pos[d];
+            vi = sv.vt[d];
+            gi2 = g[d];
+            tgi = sv.tg[d];
+            cell_xy(R, pi.x, pi.y, cx, cy);
+        }
+        const uint32_t gi = tgi & GID_MASK;
+        const int ti = (int)(tgi >> TYPE_SHIFT);
+        // does some bead of the warp sit in an edge cell (its neighbours' images matter)
+        const bool wrap = __any_sync(0xffffffffu, act && (cx == 0 || cx == ncx - 1 || cy == 0 || cy == ncy - 1));
         float xbx = 0.f, xby = 0.f, vbx = 0.f, vby = 0.f;
-        double ggam = 0.0;
-        for (int ox = -1; ox <= 1; ox++)
-            for (int oy = -1; oy <= 1; oy++) {
-                const int cc = ((cx + ox + ncx) % ncx) * ncy + (cy + oy + ncy) % ncy;
-                for (int j = cs[cc]; j < cs[cc + 1]; j++) {
-                    if (j == d) continue;
-                    const float2 pj = sv.pos[j];
-                    const float dx = minimg(__fsub_rn(pi.x, pj.x), L, h), dy = minimg(__fsub_rn(pi.y, pj.y), L, h);
-                    const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
-                    if (!(r2 < 1.0f && r2 > 1e-24f)) continue;
-                    const float2 vj = sv.vt[j], gj = g[j];
-                    const uint32_t tgj = sv.tg[j];
-                    const int tj = (int)(tgj >> TYPE_SHIFT);
-                    float r, ir;
-                    r_and_ir(r2, r, ir);
-                    const float w = 1.0f - r;
-                    const float dvx = vi.x - vj.x, dvy = vi.y - vj.y;
-                    const float rv = (dx * dvx + dy * dvy) * ir;
-                    const float th = theta_of(nk, gi, tgj & GID_MASK);
-                    const float a = R.a[ti * DPD_MAXT + tj];
-                    const float A = a - gam * w * rv + s * th;
-                    const float fm = w * A * ir;
-                    const float cxv = gi2.x - gj.x, cyv = gi2.y - gj.y;
-                    const float cd = cxv * dx + cyv * dy;
-                    const float dfr = (-A + w * gam * rv) * ir - w * A * ir * ir;
-                    const float dfv = -gam * w * w * ir;
-                    const float hx = dx * ir, hy = dy * ir;
-                    xbx += cd * (dfr * hx + dfv * (dvx - rv * hx) * ir) + fm * cxv;
-                    xby += cd * (dfr * hy + dfv * (dvy - rv * hy) * ir) + fm * cyv;
-                    vbx += cd * dfv * hx;
-                    vby += cd * dfv * hy;
-                    if (gi < (tgj & GID_MASK)) {  // parameter gradients: each pair once
-                        const int lo = min(ti, tj), hi = max(ti, tj);
-                        atomicAdd(&sgrad[lo * DPD_MAXT + hi], (double)(cd * w * ir));
-                        ggam += (double)(cd * w * (-w * rv + (gam > 0.0f ? s * th / (2.0f * gam) : 0.0f)) * ir);
-                    }
+        int n = 0;  // listed hits of the bead (the same in its lanes)
+        auto evaluate = [&]() {
+            __syncwarp();
+            for (int k = sub; k < n; k += LPB) {
+                const int j = list[bead][k];
+                const float2 pj = sv.pos[j], vj = sv.vt[j], gj = g[j];
+                const uint32_t tgj = sv.tg[j];
+                const int tj = (int)(tgj >> TYPE_SHIFT);
+                float dx = __fsub_rn(pi.x, pj.x), dy = __fsub_rn(pi.y, pj.y);
+                if (wrap) {
+                    dx = minimg(dx, L, h);
+                    dy = minimg(dy, L, h);
+                }
+                const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+                float r, ir;
+                r_and_ir(r2, r, ir);
+                const float w = 1.0f - r;
+                const float dvx = vi.x - vj.x, dvy = vi.y - vj.y;
+                const float rv = (dx * dvx + dy * dvy) * ir;
+                const float th = pair_theta(nk, gi, tgj & GID_MASK);
+                const float a = a_sh[ti * DPD_MAXT + tj];
+                const float A = a - gam * w * rv + s * th;
+                const float fm = w * A * ir;
+                const float cxv = gi2.x - gj.x, cyv = gi2.y - gj.y;
+                const float cd = cxv * dx + cyv * dy;
+                const float dfr = (-A + w * gam * rv) * ir - w * A * ir * ir;
+                const float dfv = -gam * w * w * ir;
+                const float hx = dx * ir, hy = dy * ir;
+                xbx += cd * (dfr * hx + dfv * (dvx - rv * hx) * ir) + fm * cxv;
+                xby += cd * (dfr * hy + dfv * (dvy - rv * hy) * ir) + fm * cyv;
+                vbx += cd * dfv * hx;
+                vby += cd * dfv * hy;
+                if (gi < (tgj & GID_MASK)) {  // parameter gradients: each pair once
+                    const int lo = min(ti, tj), hi = max(ti, tj);
+                    const double da = (double)(cd * w * ir);
+                    if (hi < VJP_TYPES) acc[lo * (2 * VJP_TYPES - 1 - lo) / 2 + hi][tid] += da;
+                    else atomicAdd(&sgrad[lo * DPD_MAXT + hi], da);
+                    ggam += (double)(cd * w * (-w * rv + sg * th) * ir);
                 }
             }
-        // bonds: f_i = kb (1 - r0/r) d with d = x_p - x_i (linear chains; the
-        // branched shapes' bonds and angles are k_mol_vjp's)
-        const int2 lk = R.arch == 0 ? sv.link[d] : make_int2(-1, -1);
-        double gkb = 0.0;
-        for (int q = 0; q < 2; q++) {
-            const int p = q ? lk.y : lk.x;
-            if (p < 0) continue;
-            const float2 pp = sv.pos[p], gp = g[p];
-            const float dx = minimg(pp.x - pi.x, L, h), dy = minimg(pp.y - pi.y, L, h);
-            const float r = sqrtf(dx * dx + dy * dy);
-            const float cxv = gi2.x - gp.x, cyv = gi2.y - gp.y;
-            const float cd = cxv * dx + cyv * dy;
-            const float u = 1.0f - R.r0 / r;
-            const float k0 = R.kb * R.r0 / (r * r) * cd / r;
-            xbx -= k0 * dx + R.kb * u * cxv;
-            xby -= k0 * dy + R.kb * u * cyv;
-            if (q == 1) gkb += (double)(u * cd);  // each bond once, from its prev end
+            n = 0;
+            __syncwarp();
+        };
+        // the slots of rows [ra, rb] of the three columns, taken by the bead's lanes
+        // in turn, VJP_LIST a block: each lane marks its hits in a word, then lists them
+        auto sweep = [&](bool on, int ra, int rb) {
+            int s0 = 0, s1 = 0, s2 = 0, l0 = 0, l1 = 0, l2 = 0;
+            if (on) {
+                const int32_t *c0 = cs + (cx > 0 ? cx - 1 : ncx - 1) * ncy, *c1 = cs + cx * ncy;
+                const int32_t *c2 = cs + (cx + 1 < ncx ? cx + 1 : 0) * ncy;
+                s0 = c0[ra];
+                s1 = c1[ra];
+                s2 = c2[ra];
+                l0 = c0[rb + 1] - s0;
+                l1 = l0 + (c1[rb + 1] - s1);
+                l2 = l1 + (c2[rb + 1] - s2);
+                s1 -= l0;
+                s2 -= l1;
+            }
+            const int most = __reduce_max_sync(0xffffffffu, l2);
+            for (int kb = 0; kb < most; kb += VJP_LIST) {
+                uint32_t mark = 0;
+                const int rounds = min(VJP_LIST / LPB, (most - kb + LPB - 1) / LPB);
+#pragma unroll 4
+                for (int u = 0; u < rounds; u++) {
+                    const int k = kb + u * LPB + sub;
+                    const int j = k + (k < l0 ? s0 : (k < l1 ? s1 : s2));
+                    const float2 pj = sv.pos[k < l2 ? j : 0];
+                    float dx = __fsub_rn(pi.x, pj.x), dy = __fsub_rn(pi.y, pj.y);
+                    if (wrap) {
+                        dx = minimg(dx, L, h);
+                        dy = minimg(dy, L, h);
+                    }
+                    const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+                    mark |= (k < l2 && r2 < 1.0f && r2 > 1e-24f && j != d ? 1u : 0u) << u;
+                }
+                int at = __popc(mark), all = at;  // this lane's place in its bead's list
+#pragma unroll
+                for (int o = 1; o < LPB; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, at, o, LPB);
+                    if (sub >= o) at += t;
+                }
+                const int end = __shfl_sync(0xffffffffu, at, LPB - 1, LPB);
+                at -= all;
+                if (__any_sync(0xffffffffu, n + end > VJP_LIST)) evaluate();
+                at += n;
+                while (mark) {
+                    const int k = kb + (__ffs(mark) - 1) * LPB + sub;
+                    mark &= mark - 1;
+                    list[bead][at++] = k + (k < l0 ? s0 : (k < l1 ? s1 : s2));
+                }
+                n += end;
+            }
+        };
+        sweep(act, max(cy - 1, 0), min(cy + 1, ncy - 1));
+        const bool low = act && cy == 0, high = act && cy == ncy - 1;  // ncy >= 3
+        if (__any_sync(0xffffffffu, low || high)) sweep(low || high, low ? ncy - 1 : 0, low ? ncy - 1 : 0);
+        evaluate();
+        if (act) {
+            // bonds: f_i = kb (1 - r0/r) d with d = x_p - x_i (linear chains; the
+            // branched shapes' bonds and angles are k_mol_vjp's), a lane per end
+            const int2 lk = R.arch == 0 ? sv.link[d] : make_int2(-1, -1);
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int p = q ? lk.y : lk.x;
+                if (p < 0 || sub != q % LPB) continue;
+                const float2 pp = sv.pos[p], gp = g[p];
+                const float dx = minimg(pp.x - pi.x, L, h), dy = minimg(pp.y - pi.y, L, h);
+                const float r = sqrtf(dx * dx + dy * dy);
+                const float cxv = gi2.x - gp.x, cyv = gi2.y - gp.y;
+                const float cd = cxv * dx + cyv * dy;
+                const float u = 1.0f - R.r0 / r;
+                const float k0 = R.kb * R.r0 / (r * r) * cd / r;
+                xbx -= k0 * dx + R.kb * u * cxv;
+                xby -= k0 * dy + R.kb * u * cyv;
+                if (q == 1) gkb += (double)(u * cd);  // each bond once, from its prev end
+            }
+            if (R.ka != 0.0f && (lk.x >= 0 || lk.y >= 0) && sub == 2 % LPB) {
+                const float2 t = angle_vjp(sv, g, R, pi, gi2, lk);
+                xbx += t.x;
+                xby += t.y;
+            }
+            if (R.stir_A != 0.0f && sub == 3 % LPB) {
+                const double w2 = 2.0 * R.stir_k;
+                const double dfy = (double)R.stir_A * M_PI * w2 * cospi(w2 * (double)pi.y);
+                xby += (float)(dfy * ((double)gi2.x - gsum[c.rep] / (double)R.n));
+            }
         }
-        if (R.ka != 0.0f && (lk.x >= 0 || lk.y >= 0)) {
-            const float2 t = angle_vjp(sv, g, R, pi, gi2, lk);
-            xbx += t.x;
-            xby += t.y;
+#pragma unroll
+        for (int o = LPB / 2; o > 0; o >>= 1) {
+            xbx += __shfl_xor_sync(0xffffffffu, xbx, o);
+            xby += __shfl_xor_sync(0xffffffffu, xby, o);
+            vbx += __shfl_xor_sync(0xffffffffu, vbx, o);
+            vby += __shfl_xor_sync(0xffffffffu, vby, o);
         }
-        if (R.stir_A != 0.0f) {
-            const double w2 = 2.0 * R.stir_k;
-            const double dfy = (double)R.stir_A * M_PI * w2 * cospi(w2 * (double)pi.y);
-            xby += (float)(dfy * ((double)gi2.x - gsum[c.rep] / (double)R.n));
+        if (act && sub == 0) {
+            xbar[d] = make_float2(xbx, xby);
+            vbar[d] = make_float2(vbx, vby);
         }
-        xbar[d] = make_float2(xbx, xby);
-        vbar[d] = make_float2(vbx, vby);
-        if (ggam != 0.0) atomicAdd(&sgrad[DPD_MAXT * DPD_MAXT], ggam);
-        if (gkb != 0.0) atomicAdd(&sgrad[DPD_MAXT * DPD_MAXT + 1], gkb);
     }
-    __syncthreads();
-    for (int k = threadIdx.x; k < NGRAD; k += blockDim.x)
-        if (sgrad[k] != 0.0) atomicAdd(&grad[(size_t)c.rep * NGRAD + k], sgrad[k]);
+    if (rep >= 0) hand_over();
 }
 
 // Gaussian-smoothed distribution of (ta, tb) pairs: h_b += K(r - r_b) dr for
@@ -557,7 +706,18 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
         cudaMemsetAsync(gsum, 0, (size_t)nrep * sizeof(double), s);
         k_gsum<<<nbch, BEAD_TPB, 0, s>>>(rep, bch, g, gsum);
     }
-    k_force_vjp<<<nbch, BEAD_TPB, 0, s>>>(sv, step, rep, bch, g, xbar, vbar, grad, gsum, step_base);
+    // lanes per bead: eight or four while the tasks fit the GPU at once (a small box is latency: 4,096 beads take
+    // 10.8 us with eight against 13.3 with four and 17.3 with two; 16,384 beads 14.1 with four, 17.4 with two), else two,
+    // whose lanes wait less for the fullest list (24 boxes of 65,536: 374 us, 455 with four, 585 with eight); then
+    // three CTAs an SM at 80 registers, two otherwise
+    auto go = [&](auto kern, int lpb, int per_sm) {
+        const int ntask = nbch * lpb;
+        kern<<<std::min(ntask, per_sm * 148), VJP_TPB, 0, s>>>(sv, step, rep, bch, ntask, g, xbar, vbar, grad, gsum,
+                                                             step_base);
+    };
+    if (nbch * 8 <= 2 * 148) go(k_force_vjp<8, 2>, 8, 2);
+    else if (nbch * 4 <= 2 * 148) go(k_force_vjp<4, 2>, 4, 2);
+    else go(k_force_vjp<2, 3>, 2, 3);
     if (mol) k_mol_vjp<<<nbch, BEAD_TPB, 0, s>>>(sv, rep, bch, mol, g, xbar, grad);
 }
 
