@@ -7,9 +7,13 @@
 //                noise theta is replayed from its key (frozen noise).
 // k_rdf          Gaussian-smoothed pair distribution of two bead types
 //                (the structural target of a fit) and its gradient (VJP).
-// k_adj_update   the adjoint of the Groot-Warren update, with the adjoint
-//                state kept in gid order so the sort of every step does not
-//                matter.
+// adj_update     the adjoint of the Groot-Warren update, applied by the VJP
+//                kernel itself.  The adjoint state lies in the slots of the
+//                configuration it belongs to and moves from step to step
+//                through the steps' stored sorts, so that its accesses are as
+//                local as the sort is (in gid order every access was a sector
+//                of its own: 82 us a step on 24 boxes of 65,536 beads, and 11
+//                for the gather of the force cotangents).
 //
 // Pair term (w = 1 - r, A = a - gamma w rv + s theta, s = sigma / sqrt(dt)):
 //   f = fm d,  fm = w A / r,  rv = d . dv / r
@@ -135,6 +139,19 @@ __global__ void __launch_bounds__(BEAD_TPB) k_gsum(const RepDev *__restrict__ re
 #define VJP_TYPES 4         // types whose pairs have lane-private gradient sums
 #define VJP_COMBOS (VJP_TYPES * (VJP_TYPES + 1) / 2)
 
+//   x_bar(n)  = x_bar(n+1) + J_x^T F_bar
+//   vh_bar(n) = dt x_bar(n) + vh_bar(n+1) + J_v^T F_bar
+//   F_bar(n)  = dt^2 x_bar(n) + dt vh_bar(n+1) + cvt J_v^T F_bar
+// of bead d of the configuration n+1; xf = J_x^T F_bar, vf = J_v^T F_bar
+__device__ __forceinline__ void adj_update(const AdjUpdate &u, const RepDev &R, int d, float2 xf, float2 vf) {
+    const float2 x0 = u.X[d], v0 = u.V[d];
+    const int o = u.src[d];
+    const float2 x = make_float2(x0.x + xf.x, x0.y + xf.y);
+    u.X2[o] = x;
+    u.V2[o] = make_float2(R.dt * x.x + v0.x + vf.x, R.dt * x.y + v0.y + vf.y);
+    u.F2[o] = make_float2(R.dt2 * x.x + R.dt * v0.x + R.cvt * vf.x, R.dt2 * x.y + R.dt * v0.y + R.cvt * vf.y);
+}
+
 // LPB lanes share a bead: they take its 3 x 3 cells' slots in turn (cells are
 // column-major: three contiguous ranges, and three more where the rows wrap),
 // list the ones inside the cutoff, then take the listed pairs in turn, so that
@@ -144,18 +161,20 @@ __global__ void __launch_bounds__(BEAD_TPB) k_gsum(const RepDev *__restrict__ re
 // gradient are FP64: per lane and pair of types in shared memory for the first
 // four types (no two lanes on one word), through an atomic for the others.
 // A CTA takes a run of consecutive tasks (256 / LPB beads of a chunk) and hands
-// its gradient sums over when the replica changes and at its end.
+// its gradient sums over when the replica changes and at its end.  UPDATE: the
+// adjoint of the step's update is applied at once (adj_update); else the
+// products go to xbar and vbar.
 // What bounds it: instruction issue (175 warp instructions a bead at density 4,
 // 2.2 of 4 a cycle: half of them the 12.6 evaluations, 40 of whose 130
 // instructions are the noise) and the fullest list of a warp, 1.6 times the
 // mean.  24 boxes of 65,536 beads: 374 us, against 939 with a thread per bead
 // and an FP64 shared atomic per pair; one box: 32 against 68, of 16,384: 14
 // against 60, of 4,096: 11 against 61.
-template <int LPB, int MINB>
+template <int LPB, int MINB, bool UPDATE>
 __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long long step, const RepDev *__restrict__ reps,
                                                        const Chunk *__restrict__ ch, int ntask,
                                                        const float2 *__restrict__ g, float2 *__restrict__ xbar,
-                                                       float2 *__restrict__ vbar,
+                                                       float2 *__restrict__ vbar, AdjUpdate up,
                                                        double *__restrict__ grad, const double *__restrict__ gsum,
                                                        const long long *__restrict__ step_base) {
     constexpr int BEADS = VJP_TPB / LPB;
@@ -369,8 +388,12 @@ __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long 
             vby += __shfl_xor_sync(0xffffffffu, vby, o);
         }
         if (act && sub == 0) {
-            xbar[d] = make_float2(xbx, xby);
-            vbar[d] = make_float2(vbx, vby);
+            if (UPDATE) {
+                adj_update(up, R, d, make_float2(xbx, xby), make_float2(vbx, vby));
+            } else {
+                xbar[d] = make_float2(xbx, xby);
+                vbar[d] = make_float2(vbx, vby);
+            }
         }
     }
     if (rep >= 0) hand_over();
@@ -491,8 +514,7 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
     };
     for (int it = w; it < n;) {
         const int d = list[it];
-        const uint32_t tgd = sv.tg[d];
-        const int ti = (int)(tgd >> TYPE_SHIFT);
+        const int ti = (int)(sv.tg[d] >> TYPE_SHIFT);
         const float2 pi = sv.pos[d];
         int cx, cy;
         cell_xy(R, pi.x, pi.y, cx, cy);
@@ -545,9 +567,8 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
                 gy += __shfl_xor_sync(0xffffffffu, gy, o);
             }
             if (lane == 0) {
-                const uint32_t gg = (tgd & GID_MASK) + (uint32_t)R.b0;
-                const float2 x = xadd[gg];
-                xadd[gg] = make_float2(x.x + gx, x.y + gy);
+                const float2 x = xadd[d];
+                xadd[d] = make_float2(x.x + gx, x.y + gy);
             }
             gx = gy = 0.0f;
         }
@@ -568,63 +589,31 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
     }
 }
 
-// Adjoint of one Groot-Warren step, slot order of the configuration n+1 mapped
-// to gid order (packed: gid + b0 of the replica):
-//   x_bar(n)  = x_bar(n+1) + J_x^T F_bar
-//   vh_bar(n) = dt x_bar(n) + vh_bar(n+1) + J_v^T F_bar
-//   F_bar(n)  = dt^2 x_bar(n) + dt vh_bar(n+1) + cvt J_v^T F_bar
-// (X, V, F hold x_bar, vh_bar, F_bar in gid order; xb, vb are J_x^T F_bar, J_v^T F_bar in slot order)
-__global__ void __launch_bounds__(BEAD_TPB) k_adj_update(const uint32_t *__restrict__ tg, const RepDev *__restrict__ reps,
-                                                         const Chunk *__restrict__ ch, const float2 *__restrict__ xb,
-                                                         const float2 *__restrict__ vb, float2 *__restrict__ X,
-                                                         float2 *__restrict__ V, float2 *__restrict__ F) {
+// the adjoint of the update alone, after the branched shapes' k_mol_vjp has added its share to xb
+__global__ void __launch_bounds__(BEAD_TPB) k_adj_update(const RepDev *__restrict__ reps, const Chunk *__restrict__ ch,
+                                                         const float2 *__restrict__ xb, const float2 *__restrict__ vb,
+                                                         AdjUpdate up) {
     const Chunk c = ch[blockIdx.x];
     const int d = c.begin + (int)threadIdx.x;
-    if (d >= c.end) return;
-    const RepDev &R = reps[c.rep];
-    const uint32_t g = (tg[d] & GID_MASK) + (uint32_t)R.b0;
-    const float2 x0 = X[g], v0 = V[g], xf = xb[d], vf = vb[d];
-    const float2 x = make_float2(x0.x + xf.x, x0.y + xf.y);
-    X[g] = x;
-    V[g] = make_float2(R.dt * x.x + v0.x + vf.x, R.dt * x.y + v0.y + vf.y);
-    F[g] = make_float2(R.dt2 * x.x + R.dt * v0.x + R.cvt * vf.x, R.dt2 * x.y + R.dt * v0.y + R.cvt * vf.y);
+    if (d < c.end) adj_update(up, reps[c.rep], d, xb[d], vb[d]);
 }
 
-// gather F_bar (gid order) into slot order of one configuration
-__global__ void __launch_bounds__(BEAD_TPB) k_adj_gather(const uint32_t *__restrict__ tg, const RepDev *__restrict__ reps,
-                                                         const Chunk *__restrict__ ch, const float2 *__restrict__ F,
-                                                         float2 *__restrict__ g) {
-    const Chunk c = ch[blockIdx.x];
-    const int d = c.begin + (int)threadIdx.x;
-    if (d >= c.end) return;
-    g[d] = F[(tg[d] & GID_MASK) + (uint32_t)reps[c.rep].b0];
-}
-
-// cotangents of the window's start state in gid order: x_bar(0) gains the part
+// cotangents of the window's start state into gid order: x_bar(0) gains the part
 // that flows through the start forces (xb = J_x^T F_bar(0)), and the predicted
 // velocity's cotangent is that force VJP's vb; vh_bar(0) is V as it stands
 __global__ void __launch_bounds__(BEAD_TPB) k_adj_state(const uint32_t *__restrict__ tg, const RepDev *__restrict__ reps,
-                                                        const Chunk *__restrict__ ch, const float2 *__restrict__ xb,
-                                                        const float2 *__restrict__ vb, float2 *__restrict__ X,
-                                                        float2 *__restrict__ VT) {
+                                                        const Chunk *__restrict__ ch, const float2 *__restrict__ X,
+                                                        const float2 *__restrict__ V, const float2 *__restrict__ xb,
+                                                        const float2 *__restrict__ vb, float2 *__restrict__ oX,
+                                                        float2 *__restrict__ oV, float2 *__restrict__ oVT) {
     const Chunk c = ch[blockIdx.x];
     const int d = c.begin + (int)threadIdx.x;
     if (d >= c.end) return;
     const uint32_t g = (tg[d] & GID_MASK) + (uint32_t)reps[c.rep].b0;
-    const float2 x = X[g], a = xb[d];
-    X[g] = make_float2(x.x + a.x, x.y + a.y);
-    VT[g] = vb[d];
-}
-
-// copy a configuration out of the engine's buffers (for recomputation)
-__global__ void k_adj_save(int n, const float2 *pos, const float2 *vt, const uint32_t *tg, const int2 *link,
-                           float2 *opos, float2 *ovt, uint32_t *otg, int2 *olink) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    opos[k] = pos[k];
-    ovt[k] = vt[k];
-    otg[k] = tg[k];
-    olink[k] = link[k];
+    const float2 x = X[d], a = xb[d];
+    oX[g] = make_float2(x.x + a.x, x.y + a.y);
+    oV[g] = V[d];
+    oVT[g] = vb[d];
 }
 
 // The bonded terms of the branched shapes (the template terms of
@@ -701,7 +690,7 @@ __global__ void __launch_bounds__(BEAD_TPB) k_mol_vjp(StateView sv, const RepDev
 
 void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, const Chunk *bch, int nbch,
                       const float2 *g, float2 *xbar, float2 *vbar, double *grad, double *gsum, int nrep, bool stir,
-                      const dpd_template *mol, cudaStream_t s, const long long *step_base) {
+                      const dpd_template *mol, cudaStream_t s, const long long *step_base, const AdjUpdate *up) {
     if (stir) {
         cudaMemsetAsync(gsum, 0, (size_t)nrep * sizeof(double), s);
         k_gsum<<<nbch, BEAD_TPB, 0, s>>>(rep, bch, g, gsum);
@@ -710,15 +699,20 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
     // 10.8 us with eight against 13.3 with four and 17.3 with two; 16,384 beads 14.1 with four, 17.4 with two), else two,
     // whose lanes wait less for the fullest list (24 boxes of 65,536: 374 us, 455 with four, 585 with eight); then
     // three CTAs an SM at 80 registers, two otherwise
+    const bool update = up && !mol;  // the branched shapes add their share first
+    const AdjUpdate none{};
     auto go = [&](auto kern, int lpb, int per_sm) {
         const int ntask = nbch * lpb;
-        kern<<<std::min(ntask, per_sm * 148), VJP_TPB, 0, s>>>(sv, step, rep, bch, ntask, g, xbar, vbar, grad, gsum,
-                                                             step_base);
+        kern<<<std::min(ntask, per_sm * 148), VJP_TPB, 0, s>>>(sv, step, rep, bch, ntask, g, xbar, vbar,
+                                                             update ? *up : none, grad, gsum, step_base);
     };
-    if (nbch * 8 <= 2 * 148) go(k_force_vjp<8, 2>, 8, 2);
-    else if (nbch * 4 <= 2 * 148) go(k_force_vjp<4, 2>, 4, 2);
-    else go(k_force_vjp<2, 3>, 2, 3);
-    if (mol) k_mol_vjp<<<nbch, BEAD_TPB, 0, s>>>(sv, rep, bch, mol, g, xbar, grad);
+    if (nbch * 8 <= 2 * 148) go(update ? k_force_vjp<8, 2, true> : k_force_vjp<8, 2, false>, 8, 2);
+    else if (nbch * 4 <= 2 * 148) go(update ? k_force_vjp<4, 2, true> : k_force_vjp<4, 2, false>, 4, 2);
+    else go(update ? k_force_vjp<2, 3, true> : k_force_vjp<2, 3, false>, 2, 3);
+    if (mol) {
+        k_mol_vjp<<<nbch, BEAD_TPB, 0, s>>>(sv, rep, bch, mol, g, xbar, grad);
+        if (up) k_adj_update<<<nbch, BEAD_TPB, 0, s>>>(rep, bch, xbar, vbar, *up);
+    }
 }
 
 // CTAs per chunk of beads: the whole chunk, or halves, quarters or eighths of
@@ -742,31 +736,22 @@ void launch_rdf(const StateView &sv, const RepDev *rep, const Chunk *bch, int nb
 }
 
 void launch_rdf_vjp(const StateView &sv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
-                    float rmax, float sigma, const double *wgt, float2 *xadd_gid, cudaStream_t s) {
+                    float rmax, float sigma, const double *wgt, float2 *xadd, cudaStream_t s) {
     RdfConst q{ta, tb, nbin, rmax, sigma};
     const int split = rdf_split(nbch);
-    k_rdf<true, 1><<<nbch * split, BEAD_TPB, nbin * sizeof(float), s>>>(sv, rep, bch, split, q, nullptr, wgt, xadd_gid);
+    k_rdf<true, 1><<<nbch * split, BEAD_TPB, nbin * sizeof(float), s>>>(sv, rep, bch, split, q, nullptr, wgt, xadd);
 }
 
-void launch_adj_update(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *xb,
-                       const float2 *vb, float2 *X, float2 *V, float2 *F, cudaStream_t s) {
-    k_adj_update<<<nbch, BEAD_TPB, 0, s>>>(tg, rep, bch, xb, vb, X, V, F);
+void launch_adj_state(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *X,
+                      const float2 *V, const float2 *xb, const float2 *vb, float2 *oX, float2 *oV, float2 *oVT,
+                      cudaStream_t s) {
+    k_adj_state<<<nbch, BEAD_TPB, 0, s>>>(tg, rep, bch, X, V, xb, vb, oX, oV, oVT);
 }
 
-void launch_adj_gather(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *F, float2 *g,
-                       cudaStream_t s) {
-    k_adj_gather<<<nbch, BEAD_TPB, 0, s>>>(tg, rep, bch, F, g);
-}
+// the device's step number, on the stream and without a copy or a wait
+__global__ void k_set_step(long long *__restrict__ step, long long v) { *step = v; }
 
-void launch_adj_state(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *xb,
-                      const float2 *vb, float2 *X, float2 *VT, cudaStream_t s) {
-    k_adj_state<<<nbch, BEAD_TPB, 0, s>>>(tg, rep, bch, xb, vb, X, VT);
-}
-
-void launch_adj_save(int n, const float2 *pos, const float2 *vt, const uint32_t *tg, const int2 *link, float2 *opos,
-                     float2 *ovt, uint32_t *otg, int2 *olink, cudaStream_t s) {
-    k_adj_save<<<(n + 255) / 256, 256, 0, s>>>(n, pos, vt, tg, link, opos, ovt, otg, olink);
-}
+void launch_set_step(long long *step, long long v, cudaStream_t s) { k_set_step<<<1, 1, 0, s>>>(step, v); }
 
 // ---------------------------------------------------------------- a fit iteration without the host
 //

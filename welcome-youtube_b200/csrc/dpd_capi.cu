@@ -48,18 +48,21 @@ struct FullCk {  // a full configuration of the engine's current buffer
     int2 *link;
     int32_t *cstart;
 };
-struct SegState {  // what a force VJP needs of one configuration
+struct SegState {  // what a force VJP needs of one configuration, and the sort that made it
     float2 *pos, *vt;
     uint32_t *tg;
     int2 *link;
-    int32_t *cstart;
+    int32_t *cstart, *src;
 };
 struct AdjBufs {
-    std::vector<FullCk> ck;  // checkpoints + the end of the window (last)
-    std::vector<SegState> seg;
-    float2 *X, *V, *F, *g, *xb, *vb;
+    std::vector<FullCk> ck;     // the start of each segment
+    std::vector<SegState> seg;  // the configurations of one segment after its start
+    float2 *vh[2], *f[2];       // the half-step velocities and forces of a segment's steps, in turn
+    float2 *X[2], *V[2], *F[2]; // the adjoint state of one configuration and of the one before, in turn
+    float2 *xb, *vb;
     double *hist, *wgt, *grad;
     double *gsum;            // per replica: the sum of the x cotangents (stirring)
+    long long *stir;         // per replica: the stirring sums of a segment's steps
 };
 }  // namespace
 
@@ -371,30 +374,30 @@ static int build_tiles(dpd_handle *h) {
 }
 
 // the exclusive scan of the cell counts, in the form the handle's tuning picked
-static void enqueue_scan(dpd_handle *h, bool step_inc) {
-    if (h->sort_mode == 1) launch_scan_lb(h->b, h->C, step_inc, h->s);
-    else launch_scan(h->b, h->C, step_inc, h->s);
+static void enqueue_scan(dpd_handle *h, const Bufs &b, bool step_inc) {
+    if (h->sort_mode == 1) launch_scan_lb(b, h->C, step_inc, h->s);
+    else launch_scan(b, h->C, step_inc, h->s);
 }
 
 // the sort of the counted keys into cell order (cell starts, src, dest)
-static void enqueue_cell_sort(dpd_handle *h, bool step_inc) {
+static void enqueue_cell_sort(dpd_handle *h, const Bufs &b, bool step_inc) {
     if (h->sort_mode == 2 && sort_pfx_fits(h->C)) {
-        launch_sort_pfx(h->b, h->C, step_inc, h->d_bch, h->nbch, h->d_cch, h->ncch, -1, h->s);
+        launch_sort_pfx(b, h->C, step_inc, h->d_bch, h->nbch, h->d_cch, h->ncch, -1, h->s);
         return;
     }
-    enqueue_scan(h, step_inc);
-    launch_place(h->b, h->d_bch, h->nbch, h->s);
-    launch_cellfix(h->b, h->d_cch, h->ncch, h->s);
+    enqueue_scan(h, b, step_inc);
+    launch_place(b, h->d_bch, h->nbch, h->s);
+    launch_cellfix(b, h->d_cch, h->ncch, h->s);
 }
 
-// row: a stats row the tile kernel assembles on the way (the other kernels
-// leave it to the caller)
-static void enqueue_forces(dpd_handle *h, bool next_keys, RowOut row = RowOut{-1, 0, nullptr}) {
-    if (h->any_mol) launch_mol_forces(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->s);
+// forces of buffer cur of b.  row: a stats row the tile kernel assembles on the
+// way (the other kernels leave it to the caller)
+static void enqueue_forces(dpd_handle *h, const Bufs &b, int cur, bool next_keys, RowOut row = RowOut{-1, 0, nullptr}) {
+    if (h->any_mol) launch_mol_forces(b, cur, h->d_rep, h->d_bch, h->nbch, h->s);
     if (h->force_kernel == 0)
-        launch_forces_tile(h->b, h->cur, h->d_rep, h->d_tiles, h->ntiles, h->tile_threads, next_keys, h->s, row);
-    else if (h->force_kernel == 2) launch_forces_bulk(h->b, h->cur, h->d_rep, h->d_tiles, h->ntiles, next_keys, h->s);
-    else launch_forces(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, true, true, next_keys, h->s);
+        launch_forces_tile(b, cur, h->d_rep, h->d_tiles, h->ntiles, h->tile_threads, next_keys, h->s, row);
+    else if (h->force_kernel == 2) launch_forces_bulk(b, cur, h->d_rep, h->d_tiles, h->ntiles, next_keys, h->s);
+    else launch_forces(b, cur, h->d_rep, h->d_bch, h->nbch, true, true, next_keys, h->s);
 }
 
 static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, const int32_t *n_beads) {
@@ -713,24 +716,23 @@ extern "C" int dpd_set_dynamics(dpd_handle *h, int32_t r, const float *vhx, cons
 // ---------------------------------------------------------------- phases
 
 // the stirring sums are accumulated by the permute kernel and read by the forces
-static void clear_stir(dpd_handle *h) {
-    if (h->any_stir) cudaMemsetAsync(h->b.stir, 0, (size_t)h->nrep * sizeof(long long), h->s);
+static void clear_stir(dpd_handle *h, const Bufs &b) {
+    if (h->any_stir) cudaMemsetAsync(b.stir, 0, (size_t)h->nrep * sizeof(long long), h->s);
 }
 
 static void enqueue_sort(dpd_handle *h, PermuteMode mode) {
     // counts of the CURRENT positions
     cudaMemsetAsync(h->b.count, 0, (size_t)(h->C + 4) * sizeof(uint32_t), h->s);
     launch_keys(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, false, h->s);
-    enqueue_cell_sort(h, false);
-    clear_stir(h);
+    enqueue_cell_sort(h, h->b, false);
+    clear_stir(h, h->b);
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, mode, h->s);
     h->cur ^= 1;
 }
 
 static int set_device_step(dpd_handle *h, int64_t step) {
-    long long v = (long long)step;
-    CK(cudaMemcpyAsync(h->b.step, &v, sizeof v, cudaMemcpyHostToDevice, h->s));
-    CK(cudaStreamSynchronize(h->s));
+    launch_set_step(h->b.step, (long long)step, h->s);
+    CK(cudaGetLastError());
     h->step = step;
     return DPD_OK;
 }
@@ -744,7 +746,7 @@ static void enqueue_next_keys(dpd_handle *h) {
 extern "C" int dpd_prime(dpd_handle *h) {
     if (!h) return fail(DPD_E_ARG, "null handle");
     enqueue_sort(h, PERM_PRIME);
-    enqueue_forces(h, false);
+    enqueue_forces(h, h->b, h->cur, false);
     launch_halfkick(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->s);
     enqueue_next_keys(h);
     CK(cudaGetLastError());
@@ -794,7 +796,7 @@ extern "C" int dpd_get_cells(dpd_handle *h, int32_t r, int32_t *cstart) {
 extern "C" int dpd_forces(dpd_handle *h, int64_t step) {
     if (!h) return fail(DPD_E_ARG, "null handle");
     TRY(set_device_step(h, step));
-    enqueue_forces(h, false);
+    enqueue_forces(h, h->b, h->cur, false);
     h->keys_valid = false;
     CK(cudaGetLastError());
     return check_status(h);
@@ -881,11 +883,11 @@ static bool cat_at(const dpd_handle *h, int64_t s) {
 static void enqueue_step(dpd_handle *h, int64_t s) {
     const bool cat = cat_at(h, s);
     if (!cat) {
-        enqueue_cell_sort(h, true);
+        enqueue_cell_sort(h, h->b, true);
     } else {
         launch_step_begin(h->b, h->nrep, h->s);
     }
-    clear_stir(h);
+    clear_stir(h, h->b);
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, cat ? PERM_KEEP : PERM_STEP, h->s);
     h->cur ^= 1;
     if (h->any_lipid) launch_chem_lists(h->b, h->cur, h->d_rep, -1, h->s);
@@ -897,9 +899,9 @@ static void enqueue_step(dpd_handle *h, int64_t s) {
     // the step's stats row into the ring: assembled by the tile force kernel's
     // epilogue from the beads it holds anyway, else by a pass of its own
     if (h->ring && h->force_kernel == 0) {
-        enqueue_forces(h, true, RowOut{h->ring_rep, h->ring_slots, h->ring});
+        enqueue_forces(h, h->b, h->cur, true, RowOut{h->ring_rep, h->ring_slots, h->ring});
     } else {
-        enqueue_forces(h, true);
+        enqueue_forces(h, h->b, h->cur, true);
         if (h->ring)
             launch_observables(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->ring_rep, false, h->ring, h->ring_slots,
                                h->s);
@@ -1056,7 +1058,7 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
         else launch_cellfix(h->b, h->d_cch, h->ncch, h->s);
     }
     CK(cudaEventRecord(ev[k++], h->s));
-    clear_stir(h);
+    clear_stir(h, h->b);
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, cat ? PERM_KEEP : PERM_STEP, h->s);
     CK(cudaEventRecord(ev[k++], h->s));
     h->cur ^= 1;
@@ -1071,7 +1073,7 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
         enqueue_sort(h, PERM_SORT);
         CK(cudaEventRecord(ev[k++], h->s));
     }
-    enqueue_forces(h, true);
+    enqueue_forces(h, h->b, h->cur, true);
     CK(cudaEventRecord(ev[k++], h->s));
     CK(cudaGetLastError());
     CK(cudaEventSynchronize(ev[nk]));
@@ -1408,17 +1410,22 @@ static int adj_setup(dpd_handle *h, int nck, int nseg, int nbin, AdjBufs &A) {
         want(&c.tg, N);
         want(&c.link, N);
         want(&c.cstart, C + 1);
+        want(&c.src, N);
     }
-    want(&A.X, N);
-    want(&A.V, N);
-    want(&A.F, N);
-    want(&A.g, N);
+    for (int k = 0; k < 2; k++) {
+        want(&A.vh[k], N);
+        want(&A.f[k], N);
+        want(&A.X[k], N);
+        want(&A.V[k], N);
+        want(&A.F[k], N);
+    }
     want(&A.xb, N);
     want(&A.vb, N);
     want(&A.hist, (size_t)h->nrep * nbin);
     want(&A.wgt, (size_t)h->nrep * nbin);
     want(&A.grad, (size_t)h->nrep * DPD_NGRAD);
     want(&A.gsum, (size_t)h->nrep);
+    want(&A.stir, (size_t)h->nrep);
     size_t total = 0;
     for (auto &q : plan) total += (q.second + 64 + 255) & ~(size_t)255;
     char *base = nullptr;
@@ -1448,26 +1455,15 @@ static void ck_save(dpd_handle *h, const FullCk &c) {
     cudaMemcpyAsync(c.cstart, h->b.cstart, (C + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, h->s);
 }
 
-static void ck_restore(dpd_handle *h, const FullCk &c) {
-    const size_t N = (size_t)h->N, C = (size_t)h->C;
-    const int k = h->cur;
-    cudaMemcpyAsync(h->b.pos[k], c.pos, N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
-    cudaMemcpyAsync(h->b.vh[k], c.vh, N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
-    cudaMemcpyAsync(h->b.vt[k], c.vt, N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
-    cudaMemcpyAsync(h->b.f[k], c.f, N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
-    cudaMemcpyAsync(h->b.tg[k], c.tg, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->s);
-    cudaMemcpyAsync(h->b.link[k], c.link, N * sizeof(int2), cudaMemcpyDeviceToDevice, h->s);
-    cudaMemcpyAsync(h->b.cstart, c.cstart, (C + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, h->s);
-    h->keys_valid = false;
+// the configuration at step s of segment sg (0: its checkpoint)
+static StateView seg_view(const AdjBufs &A, int sg, int s) {
+    if (s == 0) {
+        const FullCk &c = A.ck[sg];
+        return StateView{c.pos, c.vt, c.tg, c.link, c.cstart};
+    }
+    const SegState &c = A.seg[s - 1];
+    return StateView{c.pos, c.vt, c.tg, c.link, c.cstart};
 }
-
-static void seg_save(dpd_handle *h, const SegState &c) {
-    const int k = h->cur;
-    launch_adj_save((int)h->N, h->b.pos[k], h->b.vt[k], h->b.tg[k], h->b.link[k], c.pos, c.vt, c.tg, c.link, h->s);
-    cudaMemcpyAsync(c.cstart, h->b.cstart, (size_t)(h->C + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, h->s);
-}
-
-static StateView view_of(const SegState &c) { return StateView{c.pos, c.vt, c.tg, c.link, c.cstart}; }
 
 static StateView view_cur(dpd_handle *h) {
     const int k = h->cur;
@@ -1475,11 +1471,148 @@ static StateView view_cur(dpd_handle *h) {
 }
 
 static void enqueue_plain_step(dpd_handle *h) {  // one step without chemistry (windows require chem off)
-    enqueue_cell_sort(h, true);
-    clear_stir(h);
+    enqueue_cell_sort(h, h->b, true);
+    clear_stir(h, h->b);
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, PERM_STEP, h->s);
     h->cur ^= 1;
-    enqueue_forces(h, true);
+    enqueue_forces(h, h->b, h->cur, true);
+}
+
+// The handle's buffers with the configurations at steps s - 1 (buffer
+// (s - 1) & 1) and s (buffer s & 1) of segment sg in their place: a step of a
+// segment reads one stored configuration and writes the next, and nothing is
+// copied.  Keys, counts and the sort's scratch are the handle's own.
+static Bufs seg_bufs(dpd_handle *h, AdjBufs &A, int sg, int s) {
+    Bufs b = h->b;
+    const FullCk &c = A.ck[sg];
+    const int from = (s - 1) & 1, to = s & 1;
+    b.pos[from] = s == 1 ? c.pos : A.seg[s - 2].pos;
+    b.vt[from] = s == 1 ? c.vt : A.seg[s - 2].vt;
+    b.tg[from] = s == 1 ? c.tg : A.seg[s - 2].tg;
+    b.link[from] = s == 1 ? c.link : A.seg[s - 2].link;
+    b.vh[from] = s == 1 ? c.vh : A.vh[from];
+    b.f[from] = s == 1 ? c.f : A.f[from];
+    const SegState &t = A.seg[s - 1];
+    b.pos[to] = t.pos;
+    b.vt[to] = t.vt;
+    b.tg[to] = t.tg;
+    b.link[to] = t.link;
+    b.vh[to] = A.vh[to];
+    b.f[to] = A.f[to];
+    b.cstart = t.cstart;
+    b.src = t.src;
+    b.stir = A.stir;
+    return b;
+}
+
+static void enqueue_seg_step(dpd_handle *h, AdjBufs &A, int sg, int s) {
+    const Bufs b = seg_bufs(h, A, sg, s);
+    enqueue_cell_sort(h, b, true);
+    clear_stir(h, b);
+    launch_permute(b, (s - 1) & 1, h->d_rep, h->d_bch, h->nbch, PERM_STEP, h->s);
+    enqueue_forces(h, b, s & 1, true);
+}
+
+// A differentiated window, enqueued: its steps with the loss's histogram, then
+// (after the loss's weights are on the device) its reverse pass.
+struct Window {
+    int64_t nsteps;
+    int ckpt, nseg;
+    const dpd_rdf_spec *spec;
+    int64_t step0;     // the step the window starts from, or
+    const FitDev *fd;  // where the device keeps it (a captured iteration), else null
+    bool backward;
+    int64_t first_loss() const { return nsteps - spec->last_steps + 1; }  // window steps whose state enters the loss
+};
+
+static void window_forward(dpd_handle *h, AdjBufs &A, const Window &w) {
+    const float rmax = (float)w.spec->rmax, sig = (float)w.spec->sigma;
+    const int cur0 = h->cur, nb = w.spec->nbin;
+    cudaMemsetAsync(A.hist, 0, (size_t)h->nrep * nb * sizeof(double), h->s);
+    int last = 0;  // steps of the last segment, whose configurations stay stored for the reverse pass
+    for (int64_t k = 1; k <= w.nsteps; k++) {
+        const int sg = (int)((k - 1) / w.ckpt);
+        if (w.backward && (k - 1) % w.ckpt == 0) ck_save(h, A.ck[sg]);
+        if (w.backward && sg == w.nseg - 1) enqueue_seg_step(h, A, sg, ++last);
+        else enqueue_plain_step(h);
+        if (k >= w.first_loss())
+            launch_rdf(last ? seg_view(A, sg, last) : view_cur(h), h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb,
+                       nb, rmax, sig, A.hist, h->s);
+    }
+    if (!last) return;
+    // the end of the window into the handle's buffers, those it started from (a captured iteration is replayed there)
+    const SegState &e = A.seg[last - 1];
+    const size_t N = (size_t)h->N, C = (size_t)h->C;
+    h->cur = cur0;
+    cudaMemcpyAsync(h->b.pos[cur0], e.pos, N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
+    cudaMemcpyAsync(h->b.vh[cur0], A.vh[last & 1], N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
+    cudaMemcpyAsync(h->b.vt[cur0], e.vt, N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
+    cudaMemcpyAsync(h->b.f[cur0], A.f[last & 1], N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
+    cudaMemcpyAsync(h->b.tg[cur0], e.tg, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->s);
+    cudaMemcpyAsync(h->b.link[cur0], e.link, N * sizeof(int2), cudaMemcpyDeviceToDevice, h->s);
+    cudaMemcpyAsync(h->b.cstart, e.cstart, (C + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, h->s);
+    if (h->any_stir)
+        cudaMemcpyAsync(h->b.stir, A.stir, (size_t)h->nrep * sizeof(long long), cudaMemcpyDeviceToDevice, h->s);
+    h->keys_valid = false;  // the reverse pass uses the handle's keys and counts
+}
+
+// the device's step number to the window's step k
+static void window_set_step(dpd_handle *h, const Window &w, int64_t k) {
+    if (w.fd) launch_set_step_rel(h->b.step, w.fd, k, h->s);
+    else launch_set_step(h->b.step, (long long)(w.step0 + k), h->s);
+}
+
+// The reverse pass: segment by segment, the states of each (but the last,
+// stored by the forward pass) recomputed from its checkpoint, down to the
+// step the horizon leaves.  state[0..2] (may be null) receive the device
+// arrays of the start state's cotangents in gid order.
+static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const float2 **state) {
+    const float rmax = (float)w.spec->rmax, sig = (float)w.spec->sigma;
+    const size_t N = (size_t)h->N;
+    const dpd_template *mol = h->any_mol ? h->b.mol : nullptr;
+    const long long *base = w.fd ? &w.fd->base : nullptr;
+    int p = 0;  // which of X, V, F hold the adjoint state
+    cudaMemsetAsync(A.X[0], 0, N * sizeof(float2), h->s);
+    cudaMemsetAsync(A.V[0], 0, N * sizeof(float2), h->s);
+    cudaMemsetAsync(A.F[0], 0, N * sizeof(float2), h->s);
+    cudaMemsetAsync(A.grad, 0, (size_t)h->nrep * DPD_NGRAD * sizeof(double), h->s);
+    const int64_t first_loss = w.first_loss();
+    const int64_t k_stop = w.spec->horizon > 0 ? std::max<int64_t>(0, first_loss - 1 - w.spec->horizon) : 0;
+    const int sg_stop = (int)(k_stop / w.ckpt), s_stop = (int)(k_stop - (int64_t)sg_stop * w.ckpt);
+    for (int sg = w.nseg - 1; sg >= sg_stop; sg--) {
+        const int64_t k0 = (int64_t)sg * w.ckpt;
+        const int len = (int)std::min<int64_t>(w.ckpt, w.nsteps - k0);
+        if (sg < w.nseg - 1) {
+            window_set_step(h, w, k0);
+            const Bufs b = seg_bufs(h, A, sg, 1);
+            cudaMemsetAsync(b.count, 0, (size_t)(h->C + 4) * sizeof(uint32_t), h->s);
+            launch_keys(b, 0, h->d_rep, h->d_bch, h->nbch, true, h->s);
+            for (int s = 1; s <= len; s++) enqueue_seg_step(h, A, sg, s);
+        }
+        for (int s = len; s > (sg == sg_stop ? s_stop : 0); s--) {
+            const int64_t k = k0 + s;
+            const StateView v = seg_view(A, sg, s);
+            if (k >= first_loss)
+                launch_rdf_vjp(v, h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb, w.spec->nbin, rmax, sig, A.wgt,
+                               A.X[p], h->s);
+            const AdjUpdate up{A.X[p], A.V[p], A.F[p], A.X[p ^ 1], A.V[p ^ 1], A.F[p ^ 1], A.seg[s - 1].src};
+            launch_force_vjp(v, w.step0 + k, h->d_rep, h->d_bch, h->nbch, A.F[p], A.xb, A.vb, A.grad, A.gsum, h->nrep,
+                             h->any_stir, mol, h->s, base, &up);
+            p ^= 1;
+        }
+    }
+    // the forces stored at step k_stop (the window start without a horizon) depend on the parameters too
+    const StateView v0 = seg_view(A, sg_stop, s_stop);
+    launch_force_vjp(v0, w.step0 + k_stop, h->d_rep, h->d_bch, h->nbch, A.F[p], A.xb, A.vb, A.grad, A.gsum, h->nrep,
+                     h->any_stir, mol, h->s, base);
+    if (state) {
+        launch_adj_state(v0.tg, h->d_rep, h->d_bch, h->nbch, A.X[p], A.V[p], A.xb, A.vb, A.X[p ^ 1], A.V[p ^ 1],
+                         A.F[p ^ 1], h->s);
+        state[0] = A.X[p ^ 1];
+        state[1] = A.V[p ^ 1];
+        state[2] = A.F[p ^ 1];
+    }
+    window_set_step(h, w, w.nsteps);
 }
 
 static int check_window(dpd_handle *h, int64_t nsteps, const dpd_rdf_spec *spec, const double *target) {
@@ -1538,88 +1671,35 @@ static int window_impl(dpd_handle *h, int64_t nsteps, int32_t ckpt, const dpd_rd
     TRY(check_window(h, nsteps, spec, target));
     if (state_out && spec->horizon > 0)
         return fail(DPD_E_ARG, "start-state cotangents need the full reverse pass (horizon 0)");
-    if (ckpt < 1) ckpt = (int32_t)nsteps;
+    if (ckpt < 1 || ckpt > nsteps) ckpt = (int32_t)nsteps;
     const int nseg = (int)((nsteps + ckpt - 1) / ckpt);
     const int nb = spec->nbin;
-    const float rmax = (float)spec->rmax, sig = (float)spec->sigma;
     std::vector<long long> npairs;
     TRY(count_pairs(h, spec, npairs));
     AdjBufs A;
-    TRY(adj_setup(h, backward ? nseg + 1 : 0, backward ? ckpt + 1 : 0, nb, A));
+    TRY(adj_setup(h, backward ? nseg : 0, backward ? ckpt : 0, nb, A));
     if (!h->keys_valid) enqueue_next_keys(h);
-    const int64_t step0 = h->step;
-    const int64_t first_loss = nsteps - spec->last_steps + 1;  // window steps whose state enters the loss
-    CK(cudaMemsetAsync(A.hist, 0, (size_t)h->nrep * nb * sizeof(double), h->s));
-    // ---- forward, with a full checkpoint at the start of every segment
-    for (int64_t k = 1; k <= nsteps; k++) {
-        if (backward && (k - 1) % ckpt == 0) ck_save(h, A.ck[(k - 1) / ckpt]);
-        enqueue_plain_step(h);
-        if (k >= first_loss) launch_rdf(view_cur(h), h->d_rep, h->d_bch, h->nbch, spec->ta, spec->tb, nb, rmax, sig, A.hist, h->s);
-    }
+    const Window w{nsteps, ckpt, nseg, spec, h->step, nullptr, backward};
+    window_forward(h, A, w);
     CK(cudaGetLastError());
-    h->step = step0 + nsteps;
+    h->step = w.step0 + nsteps;
     std::vector<double> hist((size_t)h->nrep * nb), wgt((size_t)h->nrep * nb);
     CK(cudaMemcpyAsync(hist.data(), A.hist, hist.size() * sizeof(double), cudaMemcpyDeviceToHost, h->s));
     CK(cudaStreamSynchronize(h->s));
     TRY(check_status(h));
     rdf_loss(h, spec, hist, npairs, target, loss, rdf_out, &wgt);
     if (!backward) return DPD_OK;
-    const FullCk &end = A.ck[nseg];
-    ck_save(h, end);
-    const int cur_end = h->cur;
     CK(cudaMemcpyAsync(A.wgt, wgt.data(), wgt.size() * sizeof(double), cudaMemcpyHostToDevice, h->s));
-    const size_t N = (size_t)h->N;
-    CK(cudaMemsetAsync(A.X, 0, N * sizeof(float2), h->s));
-    CK(cudaMemsetAsync(A.V, 0, N * sizeof(float2), h->s));
-    CK(cudaMemsetAsync(A.F, 0, N * sizeof(float2), h->s));
-    CK(cudaMemsetAsync(A.grad, 0, (size_t)h->nrep * DPD_NGRAD * sizeof(double), h->s));
-    // ---- reverse, segment by segment, recomputing each segment's states, down to k_stop
-    const int64_t k_stop = spec->horizon > 0 ? std::max<int64_t>(0, first_loss - 1 - spec->horizon) : 0;
-    const int sg_stop = (int)(k_stop / ckpt);
-    int stop_slot = 0;  // slot of the configuration k_stop in the last recomputed segment
-    for (int sg = nseg - 1; sg >= sg_stop; sg--) {
-        const int64_t k0 = (int64_t)sg * ckpt;
-        const int len = (int)std::min<int64_t>(ckpt, nsteps - k0);
-        ck_restore(h, A.ck[sg]);
-        TRY(set_device_step(h, step0 + k0));
-        enqueue_next_keys(h);
-        seg_save(h, A.seg[0]);
-        for (int s = 1; s <= len; s++) {
-            enqueue_plain_step(h);
-            seg_save(h, A.seg[s]);
-        }
-        const int s_low = sg == sg_stop ? (int)(k_stop - k0) : 0;
-        stop_slot = s_low;
-        for (int s = len; s > s_low; s--) {
-            const int64_t k = k0 + s;
-            const StateView v = view_of(A.seg[s]);
-            if (k >= first_loss)
-                launch_rdf_vjp(v, h->d_rep, h->d_bch, h->nbch, spec->ta, spec->tb, nb, rmax, sig, A.wgt, A.X, h->s);
-            launch_adj_gather(v.tg, h->d_rep, h->d_bch, h->nbch, A.F, A.g, h->s);
-            launch_force_vjp(v, step0 + k, h->d_rep, h->d_bch, h->nbch, A.g, A.xb, A.vb, A.grad, A.gsum, h->nrep,
-                     h->any_stir, h->any_mol ? h->b.mol : nullptr, h->s);
-            launch_adj_update(v.tg, h->d_rep, h->d_bch, h->nbch, A.xb, A.vb, A.X, A.V, A.F, h->s);
-        }
-    }
-    // the forces stored at step k_stop (the window start without a horizon) depend on the parameters too
-    const StateView v0 = view_of(A.seg[stop_slot]);
-    launch_adj_gather(v0.tg, h->d_rep, h->d_bch, h->nbch, A.F, A.g, h->s);
-    launch_force_vjp(v0, step0 + k_stop, h->d_rep, h->d_bch, h->nbch, A.g, A.xb, A.vb, A.grad, A.gsum, h->nrep,
-                     h->any_stir, h->any_mol ? h->b.mol : nullptr, h->s);
+    const float2 *state[3] = {nullptr, nullptr, nullptr};
+    window_reverse(h, A, w, state_out ? state : nullptr);
     CK(cudaGetLastError());
-    if (state_out) {
-        launch_adj_state(v0.tg, h->d_rep, h->d_bch, h->nbch, A.xb, A.vb, A.X, A.g, h->s);
-        const float2 *src[3] = {A.X, A.V, A.g};
+    if (state_out)
         for (int k = 0; k < 3; k++)
-            if (state_out[k]) CK(cudaMemcpyAsync(state_out[k], src[k], N * sizeof(float2), cudaMemcpyDefault, h->s));
-    }
+            if (state_out[k])
+                CK(cudaMemcpyAsync(state_out[k], state[k], (size_t)h->N * sizeof(float2), cudaMemcpyDefault, h->s));
     if (grad) {
         CK(cudaMemcpyAsync(grad, A.grad, (size_t)h->nrep * DPD_NGRAD * sizeof(double), cudaMemcpyDefault, h->s));
     }
-    // back to the end of the window
-    h->cur = cur_end;
-    ck_restore(h, end);
-    TRY(set_device_step(h, step0 + nsteps));
     CK(cudaStreamSynchronize(h->s));
     return check_status(h);
 }
@@ -1653,9 +1733,7 @@ extern "C" int dpd_window_adjoint_state(dpd_handle *h, int64_t nsteps, int32_t c
 // ends with the window's last state in the buffers of the parity it started
 // from, so the captured graph can be replayed for the next iteration.
 struct FitArgs {
-    int64_t nsteps;
-    int ckpt, nseg, nb;
-    const dpd_rdf_spec *spec;
+    Window w;
     FitDev *fd;
     const long long *npairs;
     const double *target;
@@ -1663,66 +1741,13 @@ struct FitArgs {
 };
 
 static void enqueue_fit_iteration(dpd_handle *h, AdjBufs &A, const FitArgs &a) {
-    const dpd_rdf_spec *spec = a.spec;
-    const int nb = a.nb, ckpt = a.ckpt, nseg = a.nseg;
-    const int64_t nsteps = a.nsteps;
-    const float rmax = (float)spec->rmax, sig = (float)spec->sigma;
-    const int cur0 = h->cur;
+    const dpd_rdf_spec *spec = a.w.spec;
     launch_fit_begin(h->b.step, a.fd, h->s);
-    cudaMemsetAsync(A.hist, 0, (size_t)h->nrep * nb * sizeof(double), h->s);
     enqueue_next_keys(h);
-    const int64_t first_loss = nsteps - spec->last_steps + 1;
-    for (int64_t k = 1; k <= nsteps; k++) {
-        if ((k - 1) % ckpt == 0) ck_save(h, A.ck[(k - 1) / ckpt]);
-        enqueue_plain_step(h);
-        if (k >= first_loss) launch_rdf(view_cur(h), h->d_rep, h->d_bch, h->nbch, spec->ta, spec->tb, nb, rmax, sig, A.hist, h->s);
-    }
-    const FullCk &end = A.ck[nseg];
-    ck_save(h, end);
-    launch_rdf_loss(h->d_rep, h->nrep, A.hist, a.npairs, a.target, nb, spec->rmax, spec->last_steps, a.loss, A.wgt,
-                    a.fd, h->s);
-    const size_t N = (size_t)h->N;
-    cudaMemsetAsync(A.X, 0, N * sizeof(float2), h->s);
-    cudaMemsetAsync(A.V, 0, N * sizeof(float2), h->s);
-    cudaMemsetAsync(A.F, 0, N * sizeof(float2), h->s);
-    cudaMemsetAsync(A.grad, 0, (size_t)h->nrep * DPD_NGRAD * sizeof(double), h->s);
-    const long long *base = &a.fd->base;
-    const int64_t k_stop = spec->horizon > 0 ? std::max<int64_t>(0, first_loss - 1 - spec->horizon) : 0;
-    const int sg_stop = (int)(k_stop / ckpt);
-    int stop_slot = 0;
-    const dpd_template *mol = h->any_mol ? h->b.mol : nullptr;
-    for (int sg = nseg - 1; sg >= sg_stop; sg--) {
-        const int64_t k0 = (int64_t)sg * ckpt;
-        const int len = (int)std::min<int64_t>(ckpt, nsteps - k0);
-        ck_restore(h, A.ck[sg]);
-        launch_set_step_rel(h->b.step, a.fd, k0, h->s);
-        enqueue_next_keys(h);
-        seg_save(h, A.seg[0]);
-        for (int s = 1; s <= len; s++) {
-            enqueue_plain_step(h);
-            seg_save(h, A.seg[s]);
-        }
-        const int s_low = sg == sg_stop ? (int)(k_stop - k0) : 0;
-        stop_slot = s_low;
-        for (int s = len; s > s_low; s--) {
-            const int64_t k = k0 + s;
-            const StateView v = view_of(A.seg[s]);
-            if (k >= first_loss)
-                launch_rdf_vjp(v, h->d_rep, h->d_bch, h->nbch, spec->ta, spec->tb, nb, rmax, sig, A.wgt, A.X, h->s);
-            launch_adj_gather(v.tg, h->d_rep, h->d_bch, h->nbch, A.F, A.g, h->s);
-            launch_force_vjp(v, k, h->d_rep, h->d_bch, h->nbch, A.g, A.xb, A.vb, A.grad, A.gsum, h->nrep, h->any_stir,
-                             mol, h->s, base);
-            launch_adj_update(v.tg, h->d_rep, h->d_bch, h->nbch, A.xb, A.vb, A.X, A.V, A.F, h->s);
-        }
-    }
-    const StateView v0 = view_of(A.seg[stop_slot]);
-    launch_adj_gather(v0.tg, h->d_rep, h->d_bch, h->nbch, A.F, A.g, h->s);
-    launch_force_vjp(v0, k_stop, h->d_rep, h->d_bch, h->nbch, A.g, A.xb, A.vb, A.grad, A.gsum, h->nrep, h->any_stir,
-                     mol, h->s, base);
-    // the window's end into the starting parity's buffers, the step after the window
-    h->cur = cur0;
-    ck_restore(h, end);
-    launch_set_step_rel(h->b.step, a.fd, nsteps, h->s);
+    window_forward(h, A, a.w);
+    launch_rdf_loss(h->d_rep, h->nrep, A.hist, a.npairs, a.target, spec->nbin, spec->rmax, spec->last_steps, a.loss,
+                    A.wgt, a.fd, h->s);
+    window_reverse(h, A, a.w, nullptr);
     launch_fit_update(h->d_rep, h->nrep, A.grad, a.fd, a.grad, a.value, h->s);
 }
 
@@ -1754,12 +1779,12 @@ extern "C" int dpd_fit_graph(dpd_handle *h, int64_t nsteps, int32_t ckpt, const 
             if (h->params[r].a[s] != F.value[k])
                 return fail(DPD_E_ARG, "fit: a shared slot (%d) must start equal in every replica", s);
     }
-    if (ckpt < 1) ckpt = (int32_t)nsteps;
+    if (ckpt < 1 || ckpt > nsteps) ckpt = (int32_t)nsteps;
     const int nseg = (int)((nsteps + ckpt - 1) / ckpt), nb = spec->nbin, nrep = h->nrep;
     std::vector<long long> npairs;
     TRY(count_pairs(h, spec, npairs));
     AdjBufs A;
-    TRY(adj_setup(h, nseg + 1, ckpt + 1, nb, A));
+    TRY(adj_setup(h, nseg, ckpt, nb, A));
     // the fit's own device memory, freed before returning
     char *mem = nullptr;
     const size_t o_np = ((sizeof(FitDev) + 255) / 256) * 256, o_tg = o_np + (((size_t)nrep * 8 + 255) / 256) * 256;
@@ -1769,11 +1794,7 @@ extern "C" int dpd_fit_graph(dpd_handle *h, int64_t nsteps, int32_t ckpt, const 
     const size_t total = o_val + (((size_t)iters * fit->n * 8 + 255) / 256) * 256;
     if (cudaMalloc(&mem, total) != cudaSuccess) return fail(DPD_E_NOMEM, "cudaMalloc(%zu) for the fit", total);
     FitArgs a;
-    a.nsteps = nsteps;
-    a.ckpt = ckpt;
-    a.nseg = nseg;
-    a.nb = nb;
-    a.spec = spec;
+    a.w = Window{nsteps, ckpt, nseg, spec, 0, (FitDev *)mem, true};
     a.fd = (FitDev *)mem;
     a.npairs = (const long long *)(mem + o_np);
     a.target = (const double *)(mem + o_tg);
@@ -1847,16 +1868,16 @@ extern "C" int dpd_force_vjp(dpd_handle *h, int32_t r, int64_t step, const float
     const size_t n = (size_t)R.n, N = (size_t)h->N, a = ((n * 4 + 255) / 256) * 256;
     AdjBufs A;
     TRY(adj_setup(h, 0, 0, 1, A));
-    CK(cudaMemsetAsync(A.g, 0, N * sizeof(float2), h->s));
+    CK(cudaMemsetAsync(A.F[0], 0, N * sizeof(float2), h->s));
     CK(cudaMemsetAsync(A.grad, 0, (size_t)h->nrep * DPD_NGRAD * sizeof(double), h->s));
     float *sx = (float *)h->stage, *sy = (float *)(h->stage + a);
     CK(cudaMemcpyAsync(sx, gx, n * 4, cudaMemcpyDefault, h->s));
     CK(cudaMemcpyAsync(sy, gy, n * 4, cudaMemcpyDefault, h->s));
     // pack the cotangent into the replica's slots via the state packer's force field
     Bufs u = h->b;
-    u.f[h->cur] = A.g;
+    u.f[h->cur] = A.F[0];
     launch_set_dynamics(u, h->cur, R.b0, (int)n, nullptr, nullptr, sx, sy, nullptr, nullptr, h->s);
-    launch_force_vjp(view_cur(h), step, h->d_rep, h->d_bch, h->nbch, A.g, A.xb, A.vb, A.grad, A.gsum, h->nrep,
+    launch_force_vjp(view_cur(h), step, h->d_rep, h->d_bch, h->nbch, A.F[0], A.xb, A.vb, A.grad, A.gsum, h->nrep,
                      h->any_stir, h->any_mol ? h->b.mol : nullptr, h->s);
     CK(cudaGetLastError());
     float *outs[4] = {xbar_x, xbar_y, vbar_x, vbar_y};

@@ -275,11 +275,22 @@ size_t tile_smem_bytes();
 size_t bulk_smem_bytes();
 void launch_forces_bulk(const Bufs &b, int cur, const RepDev *rep, const TileDesc *tiles, int ntiles,
                         bool next_keys, cudaStream_t s);
+// The adjoint of the Groot-Warren update that made a configuration from the
+// one before: (X, V, F) hold x_bar, vh_bar and F_bar in its slots, (X2, V2, F2)
+// take them in the slots of the configuration before (old slot = src[slot],
+// the step's sort).
+struct AdjUpdate {
+    const float2 *X, *V, *F;
+    float2 *X2, *V2, *F2;
+    const int32_t *src;
+};
 // gsum: nrep doubles of scratch (the mean x cotangent of the stirring term), used when stir;
-// mol: the replicas' lipid templates when some replica has branched lipids, else null
+// mol: the replicas' lipid templates when some replica has branched lipids, else null;
+// up: the update's adjoint, applied with the products at once (xbar and vbar are then scratch), or null
 void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, const Chunk *bch, int nbch,
                       const float2 *g, float2 *xbar, float2 *vbar, double *grad, double *gsum, int nrep, bool stir,
-                      const dpd_template *mol, cudaStream_t s, const long long *step_base = nullptr);
+                      const dpd_template *mol, cudaStream_t s, const long long *step_base = nullptr,
+                      const AdjUpdate *up = nullptr);
 // the device side of a fit iteration that runs without the host (dpd_fit_graph); FitDev is in device memory
 struct FitDev {
     long long base;             // the device step at the start of the iteration's window
@@ -299,15 +310,13 @@ void launch_fit_update(RepDev *rep, int nrep, const double *grad, FitDev *fd, do
 void launch_rdf(const StateView &sv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
                 float rmax, float sigma, double *hist, cudaStream_t s);
 void launch_rdf_vjp(const StateView &sv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
-                    float rmax, float sigma, const double *wgt, float2 *xadd_gid, cudaStream_t s);
-void launch_adj_update(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *xb,
-                       const float2 *vb, float2 *X, float2 *V, float2 *F, cudaStream_t s);
-void launch_adj_gather(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *F, float2 *g,
-                       cudaStream_t s);
-void launch_adj_state(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *xb,
-                      const float2 *vb, float2 *X, float2 *VT, cudaStream_t s);
-void launch_adj_save(int n, const float2 *pos, const float2 *vt, const uint32_t *tg, const int2 *link, float2 *opos,
-                     float2 *ovt, uint32_t *otg, int2 *olink, cudaStream_t s);
+                    float rmax, float sigma, const double *wgt, float2 *xadd, cudaStream_t s);
+// the start-state cotangents of slot-order X, V, xb, vb into gid-order arrays: positions, half-step velocities,
+// predicted velocities
+void launch_adj_state(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *X,
+                      const float2 *V, const float2 *xb, const float2 *vb, float2 *oX, float2 *oV, float2 *oVT,
+                      cudaStream_t s);
+void launch_set_step(long long *step, long long v, cudaStream_t s);
 int chem_kernel_count();
 int lib_error(int code, const char *msg);  // sets dpd_last_error() and returns code
 // the break stage and the candidate draws on the current sorted state (phase entry point)
