@@ -175,9 +175,11 @@ typedef struct dpd_handle dpd_handle;
  * graph_steps: steps per captured CUDA graph.  sort_mode: the cell sort's
  * exclusive scan of the cell counts in two passes (0), in one pass with
  * decoupled look-back between blocks (1), or as a block-local pass whose
- * block prefixes the placement and fix-up kernels add themselves (2: one
- * kernel fewer; boxes of up to 4,194,304 cells, else as 0); the same cell
- * starts and order.  tile_threads: threads per CTA of force_kernel 0, 256
+ * block prefixes the later kernels add themselves (2: boxes of up to 4,194,304
+ * cells, else as 0; up to 196,608 cells and ten beads a cell the force kernel
+ * also bins the beads by their next cell, and one kernel, with a scan of its
+ * own up to 32,768 cells, takes the place of scan, placement and fix-up); the
+ * same cell starts and order.  tile_threads: threads per CTA of force_kernel 0, 256
  * (four CTAs per SM) or 512 (two per SM, tiles of up to 512 cells with their
  * halo, so less halo per owned cell). */
 typedef struct {

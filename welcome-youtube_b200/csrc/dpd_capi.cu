@@ -81,6 +81,8 @@ struct dpd_handle {
     // force kernel: 0 = cell tiles in shared memory (half shell), 1 = one thread per bead (full shell)
     int force_kernel = 0;      // 0 cell tiles, 1 thread per bead, 2 cell tiles staged by bulk copies
     int sort_mode = 2;
+    uint32_t *count2[2] = {nullptr, nullptr};  // counts of next positions, one array per buffer parity
+    int32_t *bins = nullptr;    // the cells' rows of beads (see k_binfix), null where the density is too high for them
     int tile_threads = 256;    // threads per CTA of the tile kernel (256 or 512: tiles of up to that many local cells)         // 0 two scan passes, 1 one scan pass (k_scan_lb), 2 no second pass (block prefixes in place/cellfix)
     int tile_w = 8, tile_h = 16;
     TileDesc *d_tiles = nullptr;
@@ -380,7 +382,20 @@ static void enqueue_scan(dpd_handle *h, const Bufs &b, bool step_inc) {
 }
 
 // the sort of the counted keys into cell order (cell starts, src, dest)
-static void enqueue_cell_sort(dpd_handle *h, const Bufs &b, bool step_inc) {
+// b with the counts of buffer parity cur and, in sort_mode 2, the bins
+static Bufs at_parity(const dpd_handle *h, Bufs b, int cur) {
+    b.count = h->count2[cur];
+    b.bins = h->sort_mode == 2 ? h->bins : nullptr;
+    return b;
+}
+
+// the sort of buffer cur's counted keys into cell order (cell starts, src, dest); part: see dpd_profile_step
+static void enqueue_cell_sort(dpd_handle *h, const Bufs &b0, int cur, bool step_inc) {
+    const Bufs b = at_parity(h, b0, cur);
+    if (b.bins) {
+        launch_sort_bins(b, h->count2[cur ^ 1], h->C, step_inc, h->d_rep, h->d_cch, h->ncch, -1, h->s);
+        return;
+    }
     if (h->sort_mode == 2 && sort_pfx_fits(h->C)) {
         launch_sort_pfx(b, h->C, step_inc, h->d_bch, h->nbch, h->d_cch, h->ncch, -1, h->s);
         return;
@@ -390,9 +405,25 @@ static void enqueue_cell_sort(dpd_handle *h, const Bufs &b, bool step_inc) {
     launch_cellfix(b, h->d_cch, h->ncch, h->s);
 }
 
+// the handle's buffers for a sort by the placement kernels (no bins)
+static Bufs plain_counts(const dpd_handle *h) {
+    Bufs b = h->b;
+    b.count = h->count2[h->cur];
+    b.bins = nullptr;
+    return b;
+}
+
+// clear the counts (both parities) and count the current (or the next) positions of buffer cur of b
+static void enqueue_keys(dpd_handle *h, const Bufs &b0, int cur, bool next) {
+    cudaMemsetAsync(h->count2[0], 0, 2 * (size_t)(h->C + 64) * sizeof(uint32_t), h->s);
+    launch_keys(at_parity(h, b0, cur), cur, h->d_rep, h->d_bch, h->nbch, next, h->s);
+}
+
 // forces of buffer cur of b.  row: a stats row the tile kernel assembles on the
 // way (the other kernels leave it to the caller)
-static void enqueue_forces(dpd_handle *h, const Bufs &b, int cur, bool next_keys, RowOut row = RowOut{-1, 0, nullptr}) {
+static void enqueue_forces(dpd_handle *h, const Bufs &b0, int cur, bool next_keys,
+                           RowOut row = RowOut{-1, 0, nullptr}) {
+    const Bufs b = at_parity(h, b0, cur);
     if (h->any_mol) launch_mol_forces(b, cur, h->d_rep, h->d_bch, h->nbch, h->s);
     if (h->force_kernel == 0)
         launch_forces_tile(b, cur, h->d_rep, h->d_tiles, h->ntiles, h->tile_threads, next_keys, h->s, row);
@@ -467,7 +498,16 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
     TRY(dalloc(h, &b.fill, C + 4));
     TRY(dalloc(h, &b.src, N));
     TRY(dalloc(h, &b.dest, N));
-    TRY(dalloc(h, &b.count, C + 4));
+    // (both parities in one array, cleared together; each begins on a 16-byte boundary)
+    TRY(dalloc(h, &h->count2[0], 2 * (C + 64)));
+    h->count2[1] = h->count2[0] + (C + 64) / 4 * 4;
+    // Bins up to ten beads a cell: a row of 32 is then too short for about one cell in 10^8 of a random soup (denser
+    // boxes keep the placement kernel); and up to 196,608 cells, where the kernel saved is worth more than the force
+    // kernel's wait for the counts: 13.3 against 18.3 us a step at 1,024 cells, 21.4 (26.1) at 16,384, 44.0 (47.0) at
+    // 65,536, 88.9 (91.0) at 176,400, but 126.2 (120.7) at 262,144.
+    double dense = 0.0;
+    for (int r = 0; r < nrep; r++) dense = std::max(dense, (double)h->rh[r].n / h->rh[r].ncell);
+    if (dense <= 10.0 && C <= 196608) TRY(dalloc(h, &h->bins, C * BIN_CAP));
     TRY(dalloc(h, &b.cstart, C + 4));
     TRY(dalloc(h, &b.bsum, C / SCAN_PER_BLOCK + 2));
     TRY(dalloc(h, &b.scan_state, C / SCAN_PER_BLOCK + 2));
@@ -538,7 +578,7 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
     CK(cudaMemset(b.stir, 0, (size_t)nrep * sizeof(long long)));
     // staging for set/get state: 8 float + 3 int32 + 1 byte arrays of nmax
     TRY(dalloc(h, &h->stage, (size_t)h->nmax * (8 * 4 + 3 * 4 + 1) + 16 * 256));
-    CK(cudaMemset(b.count, 0, (C + 4) * sizeof(uint32_t)));
+    CK(cudaMemset(h->count2[0], 0, 2 * (C + 64) * sizeof(uint32_t)));
     CK(cudaMemset(b.claim, 0xFF, N * sizeof(uint32_t)));
     CK(cudaMemset(b.req, 0xFF, N * sizeof(int32_t)));
     CK(cudaMemset(b.status, 0, sizeof(DevStatus)));
@@ -722,9 +762,8 @@ static void clear_stir(dpd_handle *h, const Bufs &b) {
 
 static void enqueue_sort(dpd_handle *h, PermuteMode mode) {
     // counts of the CURRENT positions
-    cudaMemsetAsync(h->b.count, 0, (size_t)(h->C + 4) * sizeof(uint32_t), h->s);
-    launch_keys(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, false, h->s);
-    enqueue_cell_sort(h, h->b, false);
+    enqueue_keys(h, h->b, h->cur, false);
+    enqueue_cell_sort(h, h->b, h->cur, false);
     clear_stir(h, h->b);
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, mode, h->s);
     h->cur ^= 1;
@@ -738,8 +777,7 @@ static int set_device_step(dpd_handle *h, int64_t step) {
 }
 
 static void enqueue_next_keys(dpd_handle *h) {
-    cudaMemsetAsync(h->b.count, 0, (size_t)(h->C + 4) * sizeof(uint32_t), h->s);
-    launch_keys(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, true, h->s);
+    enqueue_keys(h, h->b, h->cur, true);
     h->keys_valid = true;
 }
 
@@ -883,7 +921,7 @@ static bool cat_at(const dpd_handle *h, int64_t s) {
 static void enqueue_step(dpd_handle *h, int64_t s) {
     const bool cat = cat_at(h, s);
     if (!cat) {
-        enqueue_cell_sort(h, h->b, true);
+        enqueue_cell_sort(h, h->b, h->cur, true);
     } else {
         launch_step_begin(h->b, h->nrep, h->s);
     }
@@ -892,7 +930,7 @@ static void enqueue_step(dpd_handle *h, int64_t s) {
     h->cur ^= 1;
     if (h->any_lipid) launch_chem_lists(h->b, h->cur, h->d_rep, -1, h->s);
     if (cat) {
-        launch_resort(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->d_cch, h->ncch, h->C, h->s);
+        launch_resort(plain_counts(h), h->cur, h->d_rep, h->d_bch, h->nbch, h->d_cch, h->ncch, h->C, h->s);
         launch_catalyst(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->nrep, h->C, h->nmax, h->stream_grid, h->s);
         enqueue_sort(h, PERM_SORT);
     }
@@ -995,6 +1033,7 @@ extern "C" int dpd_set_tuning(dpd_handle *h, const dpd_tuning *t) {
         build_tiles(h);
         return r;
     }
+    if (t->sort_mode != h->sort_mode) h->keys_valid = false;  // the modes keep the next keys differently
     h->sort_mode = t->sort_mode;
     h->gsteps = graph_len(h, t->graph_steps);
     drop_graphs(h);
@@ -1022,8 +1061,8 @@ extern "C" int dpd_set_graph_steps(dpd_handle *h, int32_t steps) {
 
 // One step launched kernel by kernel with CUDA events between the launches on
 // the handle's stream; ms[k] = device time of kernel k (scan1 (the whole scan
-// with sort_mode 1, the block-local scan with 2), scan2 (0 ms with sort_mode 1
-// and 2), place, cellfix, permute, [2 chemistry], [catalyst check + its sort], forces).  The
+// with sort_mode 1, the block-local scan with 2; 0 ms where the sort is one
+// kernel), scan2 (0 ms with sort_mode 1 and 2), place (0 ms with bins), cellfix, permute, [2 chemistry], [catalyst check + its sort], forces).  The
 // step is a real step; on a step with a catalyst check the first entry is the
 // step counter's kernel, the next three are not launched (0 ms) and the
 // permute keeps the slot order.
@@ -1037,25 +1076,29 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
     for (auto &e : ev) CK(cudaEventCreate(&e));
     int k = 0;
     CK(cudaEventRecord(ev[k++], h->s));
+    const Bufs sb = at_parity(h, h->b, h->cur);
+    uint32_t *other = h->count2[h->cur ^ 1];
     const bool pfx = h->sort_mode == 2 && sort_pfx_fits(h->C);
     if (!cat) {
-        if (pfx) launch_sort_pfx(h->b, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 0, h->s);
-        else if (h->sort_mode == 1) launch_scan_lb(h->b, h->C, true, h->s);
-        else launch_scan_part(h->b, h->C, true, 1, h->s);
+        if (sb.bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 0, h->s);
+        else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 0, h->s);
+        else if (h->sort_mode == 1) launch_scan_lb(sb, h->C, true, h->s);
+        else launch_scan_part(sb, h->C, true, 1, h->s);
     } else {
         launch_step_begin(h->b, h->nrep, h->s);
     }
     CK(cudaEventRecord(ev[k++], h->s));
-    if (!cat && h->sort_mode == 0) launch_scan_part(h->b, h->C, true, 2, h->s);
+    if (!cat && h->sort_mode == 0) launch_scan_part(sb, h->C, true, 2, h->s);
     CK(cudaEventRecord(ev[k++], h->s));
-    if (!cat) {
-        if (pfx) launch_sort_pfx(h->b, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 1, h->s);
-        else launch_place(h->b, h->d_bch, h->nbch, h->s);
+    if (!cat && !sb.bins) {
+        if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 1, h->s);
+        else launch_place(sb, h->d_bch, h->nbch, h->s);
     }
     CK(cudaEventRecord(ev[k++], h->s));
     if (!cat) {
-        if (pfx) launch_sort_pfx(h->b, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 2, h->s);
-        else launch_cellfix(h->b, h->d_cch, h->ncch, h->s);
+        if (sb.bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 1, h->s);
+        else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 2, h->s);
+        else launch_cellfix(sb, h->d_cch, h->ncch, h->s);
     }
     CK(cudaEventRecord(ev[k++], h->s));
     clear_stir(h, h->b);
@@ -1068,7 +1111,7 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
             CK(cudaEventRecord(ev[k++], h->s));
         }
     if (cat) {
-        launch_resort(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->d_cch, h->ncch, h->C, h->s);
+        launch_resort(plain_counts(h), h->cur, h->d_rep, h->d_bch, h->nbch, h->d_cch, h->ncch, h->C, h->s);
         launch_catalyst(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->nrep, h->C, h->nmax, h->stream_grid, h->s);
         enqueue_sort(h, PERM_SORT);
         CK(cudaEventRecord(ev[k++], h->s));
@@ -1298,8 +1341,10 @@ extern "C" int dpd_get_rng(dpd_handle *h, int32_t r, uint64_t *state) {
 
 extern "C" int dpd_kernels_per_step(const dpd_handle *h, int32_t *n_plain, int32_t *n_chem) {
     if (!h) return fail(DPD_E_ARG, "null handle");
-    // scan1, scan2, place, cellfix, permute, forces (+ the chemistry kernels)
-    if (n_plain) *n_plain = 6 + (h->any_lipid ? chem_kernel_count() : 0);
+    // the scan, placement and fix-up of the sort mode, permute, forces (+ the chemistry kernels)
+    const int sort = h->sort_mode == 0 || (h->sort_mode == 2 && !sort_pfx_fits(h->C)) ? 4
+                     : h->sort_mode == 2 && h->bins ? (sort_bins_one(h->C) ? 1 : 2) : 3;
+    if (n_plain) *n_plain = sort + 2 + (h->any_lipid ? chem_kernel_count() : 0);
     if (n_chem) *n_chem = chem_kernel_count();
     return DPD_OK;
 }
@@ -1471,21 +1516,21 @@ static StateView view_cur(dpd_handle *h) {
 }
 
 static void enqueue_plain_step(dpd_handle *h) {  // one step without chemistry (windows require chem off)
-    enqueue_cell_sort(h, h->b, true);
+    enqueue_cell_sort(h, h->b, h->cur, true);
     clear_stir(h, h->b);
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, PERM_STEP, h->s);
     h->cur ^= 1;
     enqueue_forces(h, h->b, h->cur, true);
 }
 
-// The handle's buffers with the configurations at steps s - 1 (buffer
-// (s - 1) & 1) and s (buffer s & 1) of segment sg in their place: a step of a
+// The handle's buffers with the configurations at steps s - 1 and s of segment
+// sg in their place (buffer parities par0 + s - 1 and par0 + s): a step of a
 // segment reads one stored configuration and writes the next, and nothing is
 // copied.  Keys, counts and the sort's scratch are the handle's own.
-static Bufs seg_bufs(dpd_handle *h, AdjBufs &A, int sg, int s) {
+static Bufs seg_bufs(dpd_handle *h, AdjBufs &A, int sg, int s, int par0) {
     Bufs b = h->b;
     const FullCk &c = A.ck[sg];
-    const int from = (s - 1) & 1, to = s & 1;
+    const int from = (par0 + s - 1) & 1, to = (par0 + s) & 1;
     b.pos[from] = s == 1 ? c.pos : A.seg[s - 2].pos;
     b.vt[from] = s == 1 ? c.vt : A.seg[s - 2].vt;
     b.tg[from] = s == 1 ? c.tg : A.seg[s - 2].tg;
@@ -1505,12 +1550,13 @@ static Bufs seg_bufs(dpd_handle *h, AdjBufs &A, int sg, int s) {
     return b;
 }
 
-static void enqueue_seg_step(dpd_handle *h, AdjBufs &A, int sg, int s) {
-    const Bufs b = seg_bufs(h, A, sg, s);
-    enqueue_cell_sort(h, b, true);
+static void enqueue_seg_step(dpd_handle *h, AdjBufs &A, int sg, int s, int par0) {
+    const Bufs b = seg_bufs(h, A, sg, s, par0);
+    const int from = (par0 + s - 1) & 1;
+    enqueue_cell_sort(h, b, from, true);
     clear_stir(h, b);
-    launch_permute(b, (s - 1) & 1, h->d_rep, h->d_bch, h->nbch, PERM_STEP, h->s);
-    enqueue_forces(h, b, s & 1, true);
+    launch_permute(b, from, h->d_rep, h->d_bch, h->nbch, PERM_STEP, h->s);
+    enqueue_forces(h, b, from ^ 1, true);
 }
 
 // A differentiated window, enqueued: its steps with the loss's histogram, then
@@ -1529,11 +1575,11 @@ static void window_forward(dpd_handle *h, AdjBufs &A, const Window &w) {
     const float rmax = (float)w.spec->rmax, sig = (float)w.spec->sigma;
     const int cur0 = h->cur, nb = w.spec->nbin;
     cudaMemsetAsync(A.hist, 0, (size_t)h->nrep * nb * sizeof(double), h->s);
-    int last = 0;  // steps of the last segment, whose configurations stay stored for the reverse pass
+    int par0 = 0, last = 0;  // steps of the last segment, whose configurations stay stored for the reverse pass
     for (int64_t k = 1; k <= w.nsteps; k++) {
         const int sg = (int)((k - 1) / w.ckpt);
         if (w.backward && (k - 1) % w.ckpt == 0) ck_save(h, A.ck[sg]);
-        if (w.backward && sg == w.nseg - 1) enqueue_seg_step(h, A, sg, ++last);
+        if (w.backward && sg == w.nseg - 1) enqueue_seg_step(h, A, sg, ++last, par0 = h->cur);
         else enqueue_plain_step(h);
         if (k >= w.first_loss())
             launch_rdf(last ? seg_view(A, sg, last) : view_cur(h), h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb,
@@ -1545,9 +1591,9 @@ static void window_forward(dpd_handle *h, AdjBufs &A, const Window &w) {
     const size_t N = (size_t)h->N, C = (size_t)h->C;
     h->cur = cur0;
     cudaMemcpyAsync(h->b.pos[cur0], e.pos, N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
-    cudaMemcpyAsync(h->b.vh[cur0], A.vh[last & 1], N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
+    cudaMemcpyAsync(h->b.vh[cur0], A.vh[(par0 + last) & 1], N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
     cudaMemcpyAsync(h->b.vt[cur0], e.vt, N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
-    cudaMemcpyAsync(h->b.f[cur0], A.f[last & 1], N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
+    cudaMemcpyAsync(h->b.f[cur0], A.f[(par0 + last) & 1], N * sizeof(float2), cudaMemcpyDeviceToDevice, h->s);
     cudaMemcpyAsync(h->b.tg[cur0], e.tg, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->s);
     cudaMemcpyAsync(h->b.link[cur0], e.link, N * sizeof(int2), cudaMemcpyDeviceToDevice, h->s);
     cudaMemcpyAsync(h->b.cstart, e.cstart, (C + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, h->s);
@@ -1584,10 +1630,8 @@ static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const flo
         const int len = (int)std::min<int64_t>(w.ckpt, w.nsteps - k0);
         if (sg < w.nseg - 1) {
             window_set_step(h, w, k0);
-            const Bufs b = seg_bufs(h, A, sg, 1);
-            cudaMemsetAsync(b.count, 0, (size_t)(h->C + 4) * sizeof(uint32_t), h->s);
-            launch_keys(b, 0, h->d_rep, h->d_bch, h->nbch, true, h->s);
-            for (int s = 1; s <= len; s++) enqueue_seg_step(h, A, sg, s);
+            enqueue_keys(h, seg_bufs(h, A, sg, 1, 0), 0, true);
+            for (int s = 1; s <= len; s++) enqueue_seg_step(h, A, sg, s, 0);
         }
         for (int s = len; s > (sg == sg_stop ? s_stop : 0); s--) {
             const int64_t k = k0 + s;

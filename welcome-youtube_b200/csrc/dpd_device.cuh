@@ -341,9 +341,18 @@ __device__ __forceinline__ bool last_cta(unsigned int *done) {
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
-// count a bead into its next cell (no value returned: the add is fire-and-forget)
-__device__ __forceinline__ void count_key(uint32_t *count, uint32_t key, bool active) {
-    if (active) atomicAdd(count + key, 1u);
+// Count a bead (slot) into its next cell and, with bins, put it into the
+// cell's row at the place the count gives (in arrival order; k_binfix puts the
+// row in slot order).  Without bins no value is returned: the add is
+// fire-and-forget.
+__device__ __forceinline__ void count_key(const Bufs &b, uint32_t key, int slot, bool active) {
+    if (!active) return;
+    if (b.bins) {
+        const uint32_t r = atomicAdd(b.count + key, 1u);
+        if (r < BIN_CAP) b.bins[(size_t)key * BIN_CAP + r] = slot;
+    } else {
+        atomicAdd(b.count + key, 1u);
+    }
 }
 
 __device__ __forceinline__ long long warp_sum_ll(long long v) {

@@ -30,6 +30,7 @@
 #define SCAN_TPB 256
 #define SCAN_PER_THREAD 4
 #define SCAN_PER_BLOCK (SCAN_TPB * SCAN_PER_THREAD)
+#define BIN_CAP 32              // beads a cell's row of bins holds
 
 // status flags raised by kernels (read back once per API call)
 #define DPD_F_OUTSIDE 0x1u      // a bead left [0, L) after integration
@@ -142,7 +143,8 @@ struct Bufs {
     uint32_t *key;
     uint32_t *fill;             // per cell: next free slot while beads are placed (cstart + count so far)
     int32_t *src, *dest;
-    uint32_t *count;
+    uint32_t *count;            // the counts the next force kernel makes or the next sort reads (one array per parity)
+    int32_t *bins;              // per cell BIN_CAP slots: the beads counted into it, or null (see k_binfix)
     int32_t *cstart;            // C + 1
     int32_t *bsum;              // scan block totals
     unsigned long long *scan_state;   // single-pass scan: per block (epoch | flag | value), see k_scan_lb
@@ -230,6 +232,11 @@ void launch_scan_lb(const Bufs &b, int64_t C, bool step_inc, cudaStream_t s);
 bool sort_pfx_fits(int64_t C);
 void launch_sort_pfx(const Bufs &b, int64_t C, bool step_inc, const Chunk *bch, int nbch, const Chunk *cch, int ncch,
                      int part, cudaStream_t s);
+// the sort from the bins the force kernel filled: the scan of the counts (within the one kernel up to
+// BIN_SCAN_CELLS cells) and every cell's row in slot order; other: the counts of the other parity, cleared
+bool sort_bins_one(int64_t C);
+void launch_sort_bins(const Bufs &b, uint32_t *other, int64_t C, bool step_inc, const RepDev *rep, const Chunk *cch,
+                      int ncch, int part, cudaStream_t s);
 void launch_place(const Bufs &b, const Chunk *bch, int nbch, cudaStream_t s);
 void launch_cellfix(const Bufs &b, const Chunk *cch, int ncch, cudaStream_t s);
 void launch_permute(const Bufs &b, int cur, const RepDev *rep, const Chunk *bch, int nbch, PermuteMode mode,

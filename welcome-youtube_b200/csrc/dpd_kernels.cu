@@ -1,9 +1,12 @@
 // dpd_kernels.cu -- cell sort, integrator, pair + bond forces and observables (sm_100a).
 //
 // One step of the production path (dpd_step) is
-//   k_scan1, k_scan2   exclusive scan of the per-cell counts of the NEXT positions
-//   k_place            provisional slot of every bead: an atomic cursor per cell
-//   k_cellfix          per cell: order its beads by old slot (stable sort), dest[]
+//   k_binfix           the beads binned by the cell of their NEXT position, by
+//                      the previous force kernel: cell starts, and every cell's
+//                      beads in old slot order (stable sort), dest[]
+//                      (large or dense boxes: k_scan1, k_scan2 the exclusive
+//                      scan of the counts, k_place a provisional slot from an
+//                      atomic cursor per cell, k_cellfix the order per cell)
 //   k_permute          gather the old slots into the new order AND apply the
 //                      Groot-Warren update (fused; oercel.c:2303-2334 + 832-933)
 //   [chemistry]        dpd_chem.cu
@@ -40,7 +43,7 @@ __global__ void __launch_bounds__(BEAD_TPB) k_keys(Bufs b, int cur, const RepDev
         int cx, cy;
         key = (uint32_t)(R.c0 + cell_xy(R, p.x, p.y, cx, cy));
     }
-    count_key(b.count, key, act);
+    count_key(b, key, i, act);
     if (act) b.key[i] = key;
 }
 
@@ -453,6 +456,115 @@ __global__ void __launch_bounds__(CELL_TPB) k_cellfix(Bufs b, const Chunk *__res
     cellfix_range(b, s, e - s);
 }
 
+// ---------------------------------------------------------------- the sort from bins
+
+// The counts of next positions come with the beads themselves (count_key): a
+// cell's row of bins holds them in arrival order.  A thread takes a cell, sorts
+// its row by old slot in registers (the reference's stable order) and writes
+// src and dest: the placement kernel and its atomics are gone.  ONE: the CTA
+// also adds up the counts before its own (up to BIN_SCAN_CELLS cells, at most
+// 128 KB read per CTA, from L2), so that the sort of a small handle is one
+// kernel; else k_scan1<true> left the cells' starts within its blocks and the
+// block totals.  A cell with more beads than its row holds (at the densities
+// that use bins, none in 10^8 cells) is gathered from the keys of its replica
+// by the whole CTA, once for all such cells it has.
+// What bounds it: latency (a small box: starts, row, stores), else HBM and L2
+// sectors: a row is read 32 bytes at a time, one or two sectors a cell.
+#define BIN_SCAN_CELLS 32768
+
+template <int NP>
+__device__ __forceinline__ void bin_cell(const Bufs &b, int cell, int s, int n) {
+    const int4 *row = reinterpret_cast<const int4 *>(b.bins + (size_t)cell * BIN_CAP);
+    int v[NP];
+#pragma unroll
+    for (int k = 0; k < NP / 4; k++) {
+        const int4 q = 4 * k < n ? row[k] : make_int4(0, 0, 0, 0);
+        v[4 * k] = q.x;
+        v[4 * k + 1] = q.y;
+        v[4 * k + 2] = q.z;
+        v[4 * k + 3] = q.w;
+    }
+#pragma unroll
+    for (int k = 0; k < NP; k++) v[k] = k < n ? v[k] : 0x7fffffff;
+    bitonic<NP>(v);
+#pragma unroll
+    for (int k = 0; k < NP; k++)
+        if (k < n) {
+            b.src[s + k] = v[k];
+            b.dest[v[k]] = s + k;
+        }
+}
+
+template <bool ONE>
+__global__ void __launch_bounds__(CELL_TPB) k_binfix(Bufs b, uint32_t *__restrict__ other,
+                                                     const RepDev *__restrict__ reps, const Chunk *__restrict__ ch,
+                                                     int nb, long long C, int step_inc) {
+    const Chunk c = ch[blockIdx.x];
+    pdl_begin();
+    __shared__ int pfx[ONE ? 1 : PFX_MAX];
+    __shared__ int red[CELL_TPB / 32];
+    __shared__ int ncrowd, cursor[CELL_TPB];
+    const int tid = (int)threadIdx.x, cell = c.begin + tid;
+    const bool act = cell < c.end;
+    if (tid == 0) ncrowd = 0;
+    int s = 0, n = 0;
+    if (ONE) {
+        int part = 0;
+        const int4 *q = reinterpret_cast<const int4 *>(b.count);
+        for (int k = tid; k < c.begin / 4; k += CELL_TPB) {
+            const int4 v = q[k];
+            part += v.x + v.y + v.z + v.w;
+        }
+        if (tid < (c.begin & 3)) part += (int)b.count[(c.begin & ~3) + tid];
+        n = act ? (int)b.count[cell] : 0;
+        part = __reduce_add_sync(0xffffffffu, part);
+        if (lane_id() == 0) red[tid >> 5] = part;
+        int total;
+        s = block_exclusive_scan(n, &total);  // (its barriers order red too)
+#pragma unroll
+        for (int w = 0; w < CELL_TPB / 32; w++) s += red[w];
+        if (act) other[cell] = 0u;
+        if (step_inc && blockIdx.x == 0 && tid == 0) {
+            *b.step += 1;
+            b.status->n_grow = 0u;  // the chemistry candidate lists of the new step start empty
+            b.status->n_bond = 0u;
+        }
+    } else {
+        block_prefixes(b.bsum, nb, pfx);
+        if (act) {
+            s = (int)b.fill[cell] + pfx[cell / SCAN_PER_BLOCK];
+            const int e = cell + 1 < C ? (int)b.fill[cell + 1] + pfx[(cell + 1) / SCAN_PER_BLOCK]
+                                       : pfx[nb - 1] + b.bsum[nb - 1];
+            n = e - s;
+        }
+    }
+    if (act) {
+        b.cstart[cell] = s;
+        if (cell + 1 == C) b.cstart[C] = s + n;
+        if (n > 16) {
+            if (n <= BIN_CAP) bin_cell<32>(b, cell, s, n);
+            else atomicAdd(&ncrowd, 1);
+        } else if (n > 8) {
+            bin_cell<16>(b, cell, s, n);
+        } else if (n > 4) {
+            bin_cell<8>(b, cell, s, n);
+        } else if (n > 0) {
+            bin_cell<4>(b, cell, s, n);
+        }
+    }
+    __syncthreads();
+    if (ncrowd == 0) return;
+    cursor[tid] = n > BIN_CAP ? s : -1;
+    __syncthreads();
+    const RepDev &R = reps[c.rep];
+    for (int i = R.b0 + tid; i < R.b0 + R.n; i += CELL_TPB) {
+        const int k = (int)b.key[i] - c.begin;
+        if (k >= 0 && k < c.end - c.begin && cursor[k] >= 0) b.src[atomicAdd(&cursor[k], 1)] = i;
+    }
+    __syncthreads();
+    if (n > BIN_CAP) cellfix_range(b, s, n);
+}
+
 // ---------------------------------------------------------------- permute (+ integrate)
 
 #define OBS_ITEMS 4  // chunks per round of k_observables
@@ -720,7 +832,7 @@ __global__ void __launch_bounds__(BEAD_TPB) k_forces(Bufs b, int cur, const RepD
         if (lane_id() == 0 && mbb != 0u) atomicMax(b.obs + (size_t)c.rep * OBS_N + 4, (unsigned long long)mbb);
     }
     if (NEXTKEY) {
-        count_key(b.count, key, act);
+        count_key(b, key, d, act);
         if (act) b.key[d] = key;
     }
 }
@@ -1161,6 +1273,20 @@ void launch_sort_pfx(const Bufs &b, int64_t C, bool step_inc, const Chunk *bch, 
     if (part < 0 || part == 1)
         launch_pdl(k_place<true>, (nbch + PLACE_ITEMS - 1) / PLACE_ITEMS, BEAD_TPB, 0, s, b, bch, nbch, no, nb);
     if (part < 0 || part == 2) launch_pdl(k_cellfix<true>, ncch, CELL_TPB, 0, s, b, cch, no, nb, (long long)C);
+}
+
+bool sort_bins_one(int64_t C) { return C <= BIN_SCAN_CELLS; }
+
+void launch_sort_bins(const Bufs &b, uint32_t *other, int64_t C, bool step_inc, const RepDev *rep, const Chunk *cch,
+                      int ncch, int part, cudaStream_t s) {
+    const int nb = (int)((C + SCAN_PER_BLOCK - 1) / SCAN_PER_BLOCK);
+    const bool one = sort_bins_one(C);
+    if (part != 1 && !one)
+        launch_pdl(k_scan1<true>, nb, SCAN_TPB, 0, s, b.count, (int32_t *)b.fill, b.bsum, (long long)C, b.step,
+                   step_inc ? 1 : 0, b.status, (const int32_t *)nullptr);
+    if (part == 0) return;
+    if (one) launch_pdl(k_binfix<true>, ncch, CELL_TPB, 0, s, b, other, rep, cch, nb, (long long)C, step_inc ? 1 : 0);
+    else launch_pdl(k_binfix<false>, ncch, CELL_TPB, 0, s, b, other, rep, cch, nb, (long long)C, 0);
 }
 
 void launch_permute(const Bufs &b, int cur, const RepDev *rep, const Chunk *bch, int nbch, PermuteMode mode,
