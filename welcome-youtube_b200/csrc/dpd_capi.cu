@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <numeric>
 #include <vector>
@@ -110,6 +111,12 @@ struct dpd_handle {
     AdjBufs adj;
     // staging for state in/out
     char *stage = nullptr;
+    int dev = 0;                // the device the handle was made on
+    // pinned host memory the device writes its status and stats rows into (no staging on the way back)
+    struct HostSide {
+        DevStatus st;
+        unsigned long long row[OBS_N];
+    } *host = nullptr;
     // cluster analysis scratch (allocated on first use): union-find parents, sizes, sums
     int *ana_parent = nullptr, *ana_size = nullptr, *ana_min = nullptr;
     int32_t *ana_label = nullptr;
@@ -347,6 +354,8 @@ static void free_all(dpd_handle *h) {
     free_adj(h);
     for (void *p : h->allocs) cudaFree(p);
     h->allocs.clear();
+    if (h->host) cudaFreeHost(h->host);
+    h->host = nullptr;
     if (h->s) cudaStreamDestroy(h->s);
 }
 
@@ -507,65 +516,66 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
         h->force_kernel = strcmp(e, "bead") == 0 ? 1 : (strcmp(e, "bulk") == 0 ? 2 : 0);
 
     choose_tile(h);
-    TRY(dalloc(h, &h->d_rep, nrep));
-    TRY(dalloc(h, &h->d_bch, bch.size()));
-    TRY(dalloc(h, &h->d_cch, cch.size()));
-    CK(cudaMemcpy(h->d_rep, h->rh.data(), nrep * sizeof(RepDev), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->d_bch, bch.data(), bch.size() * sizeof(Chunk), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->d_cch, cch.data(), cch.size() * sizeof(Chunk), cudaMemcpyHostToDevice));
+    CK(cudaGetDevice(&h->dev));
+    CK(cudaHostAlloc((void **)&h->host, sizeof *h->host, cudaHostAllocDefault));
+    // the handle's arrays, carved from one allocation that is cleared as a whole
+    std::vector<std::pair<void **, size_t>> plan;
+    auto want = [&](auto **q, size_t count) { plan.push_back({(void **)q, count * sizeof(**q)}); };
     Bufs &b = h->b;
     const size_t N = (size_t)h->N, C = (size_t)h->C;
+    want(&h->d_rep, nrep);
+    want(&h->d_bch, bch.size());
+    want(&h->d_cch, cch.size());
     for (int k = 0; k < 2; k++) {
-        TRY(dalloc(h, &b.pos[k], N));
-        TRY(dalloc(h, &b.vh[k], N));
-        TRY(dalloc(h, &b.vt[k], N));
-        TRY(dalloc(h, &b.f[k], N));
-        TRY(dalloc(h, &b.tg[k], N));
-        TRY(dalloc(h, &b.link[k], N));
+        want(&b.pos[k], N);
+        want(&b.vh[k], N);
+        want(&b.vt[k], N);
+        want(&b.f[k], N);
+        want(&b.tg[k], N);
+        want(&b.link[k], N);
     }
-    TRY(dalloc(h, &b.key, N));
-    TRY(dalloc(h, &b.fill, C + 4));
-    TRY(dalloc(h, &b.src, N));
-    TRY(dalloc(h, &b.dest, N));
+    want(&b.key, N);
+    want(&b.fill, C + 4);
+    want(&b.src, N);
+    want(&b.dest, N);
     // (both parities in one array, cleared together; each begins on a 16-byte boundary)
-    TRY(dalloc(h, &h->count2[0], 2 * (C + 64)));
-    h->count2[1] = h->count2[0] + (C + 64) / 4 * 4;
+    want(&h->count2[0], 2 * (C + 64));
     // Bins up to ten beads a cell: a row of 32 is then too short for about one cell in 10^8 of a random soup (denser
     // boxes keep the placement kernel); and up to 196,608 cells, where the kernel saved is worth more than the force
     // kernel's wait for the counts: 13.3 against 18.3 us a step at 1,024 cells, 21.4 (26.1) at 16,384, 44.0 (47.0) at
     // 65,536, 88.9 (91.0) at 176,400, but 126.2 (120.7) at 262,144.
     double dense = 0.0;
     for (int r = 0; r < nrep; r++) dense = std::max(dense, (double)h->rh[r].n / h->rh[r].ncell);
-    if (dense <= 10.0 && C <= 196608) TRY(dalloc(h, &h->bins, C * BIN_CAP));
-    TRY(dalloc(h, &b.cstart, C + 4));
-    TRY(dalloc(h, &b.bsum, C / SCAN_PER_BLOCK + 2));
-    TRY(dalloc(h, &b.scan_state, C / SCAN_PER_BLOCK + 2));
-    TRY(dalloc(h, &b.scan_ticket, 1));
-    CK(cudaMemset(b.scan_state, 0, (C / SCAN_PER_BLOCK + 2) * sizeof(unsigned long long)));
-    CK(cudaMemset(b.scan_ticket, 0, sizeof(unsigned long long)));
-    TRY(dalloc(h, &b.claim, N));
-    TRY(dalloc(h, &b.req, N));
-    TRY(dalloc(h, &b.grow_list, N));
-    TRY(dalloc(h, &b.bond_list, N));
+    if (dense <= 10.0 && C <= 196608) want(&h->bins, C * BIN_CAP);
+    want(&b.cstart, C + 4);
+    want(&b.bsum, C / SCAN_PER_BLOCK + 2);
+    want(&b.scan_state, C / SCAN_PER_BLOCK + 2);
+    want(&b.scan_ticket, 1);
+    want(&b.claim, N);
+    want(&b.req, N);
+    want(&b.grow_list, N);
+    want(&b.bond_list, N);
     b.evcap = 1 << 20;
-    TRY(dalloc(h, &b.events, (size_t)b.evcap));
-    TRY(dalloc(h, &b.status, 1));
-    TRY(dalloc(h, &b.step, 1));
-    TRY(dalloc(h, &b.obs, (size_t)nrep * OBS_N));
-    TRY(dalloc(h, &b.obs_out, (size_t)nrep * OBS_N));
-    TRY(dalloc(h, &b.obs_done, (size_t)nrep));
-    TRY(dalloc(h, &b.hist, 4096));
-    TRY(dalloc(h, &b.stir, (size_t)nrep));
-    TRY(dalloc(h, &b.rng, (size_t)4 * nrep));
-    TRY(dalloc(h, &b.cat_list, N));
-    TRY(dalloc(h, &b.cat_cnt, (size_t)h->nbch + 1));
-    TRY(dalloc(h, &b.cat_ncnt, (size_t)h->nbch + 1));
-    TRY(dalloc(h, &b.resort, (size_t)nrep + 1));
-    TRY(dalloc(h, &b.cat_nk, (size_t)nrep));
-    TRY(dalloc(h, &b.cat_near, N));
-    TRY(dalloc(h, &b.cat_cell, N));
-    TRY(dalloc(h, &b.cat_mark, C));
-    TRY(dalloc(h, &b.fmol, N));
+    want(&b.events, (size_t)b.evcap);
+    want(&b.status, 1);
+    want(&b.step, 1);
+    want(&b.obs, (size_t)nrep * OBS_N);
+    want(&b.obs_out, (size_t)nrep * OBS_N);
+    want(&b.obs_done, (size_t)nrep);
+    want(&b.hist, 4096);
+    want(&b.stir, (size_t)nrep);
+    want(&b.rng, (size_t)4 * nrep);
+    want(&b.cat_list, N);
+    want(&b.cat_cnt, (size_t)h->nbch + 1);
+    want(&b.cat_ncnt, (size_t)h->nbch + 1);
+    want(&b.resort, (size_t)nrep + 1);
+    want(&b.cat_nk, (size_t)nrep);
+    want(&b.cat_near, N);
+    want(&b.cat_cell, N);
+    want(&b.cat_mark, C);
+    want(&b.fmol, N);
+    uint64_t *dj = nullptr;
+    std::vector<uint64_t> jt;
     if (h->any_cat) {
         // the catalyst checks' draw streams: 3 n + 4096 draws per replica, 64-draw blocks
         long long so = 0;
@@ -577,51 +587,44 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
             so += dcap;
             nblk = std::max(nblk, dcap / 64);
         }
-        CK(cudaMemcpy(h->d_rep, h->rh.data(), (size_t)nrep * sizeof(RepDev), cudaMemcpyHostToDevice));
-        std::vector<uint64_t> jt;
         if (jump_table(nblk, jt) != 0) return fail(DPD_E_STATE, "xoshiro256** polynomial not found");
-        uint64_t *dj = nullptr;
-        TRY(dalloc(h, &dj, jt.size()));
-        CK(cudaMemcpy(dj, jt.data(), jt.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
-        b.jump = dj;
-        TRY(dalloc(h, &b.stream, (size_t)so));
-        TRY(dalloc(h, &b.sblock, (size_t)so / 16));
-        TRY(dalloc(h, &b.cat_dn, (size_t)nrep));
-        TRY(dalloc(h, &b.shuf, 8 * N));
+        want(&dj, jt.size());
+        want(&b.stream, (size_t)so);
+        want(&b.sblock, (size_t)so / 16);
+        want(&b.cat_dn, (size_t)nrep);
+        want(&b.shuf, 8 * N);
         b.shuf_n = (long long)N;
         h->stream_grid = (nblk + 255) / 256;
     }
-    {
-        std::vector<dpd_template> mols(nrep);
-        for (int r = 0; r < nrep; r++)
-            if (dpd_lipid_template(&h->params[r], &mols[r]) != DPD_OK) std::memset(&mols[r], 0, sizeof(dpd_template));
-        dpd_template *dm = nullptr;
-        TRY(dalloc(h, &dm, (size_t)nrep));
-        CK(cudaMemcpy(dm, mols.data(), (size_t)nrep * sizeof(dpd_template), cudaMemcpyHostToDevice));
-        b.mol = dm;
+    dpd_template *dm = nullptr;
+    want(&dm, (size_t)nrep);
+    // staging for set/get state: 8 float + 3 int32 + 1 byte arrays of nmax
+    want(&h->stage, (size_t)h->nmax * (8 * 4 + 3 * 4 + 1) + 16 * 256);
+    size_t total = 0;
+    for (auto &q : plan) total += (q.second + 64 + 255) & ~(size_t)255;
+    char *base = nullptr;
+    TRY(dalloc(h, &base, total));
+    CK(cudaMemset(base, 0, total));
+    for (auto &q : plan) {
+        *q.first = base;
+        base += (q.second + 64 + 255) & ~(size_t)255;
     }
-    CK(cudaMemset(b.resort, 0, ((size_t)nrep + 1) * sizeof(int32_t)));
-    CK(cudaMemset(b.rng, 0, (size_t)4 * nrep * sizeof(uint64_t)));
+    h->count2[1] = h->count2[0] + (C + 64) / 4 * 4;
+    b.jump = dj;
+    b.mol = dm;
+    CK(cudaMemcpy(h->d_rep, h->rh.data(), nrep * sizeof(RepDev), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(h->d_bch, bch.data(), bch.size() * sizeof(Chunk), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(h->d_cch, cch.data(), cch.size() * sizeof(Chunk), cudaMemcpyHostToDevice));
+    if (dj) CK(cudaMemcpy(dj, jt.data(), jt.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
+    std::vector<dpd_template> mols(nrep);
+    for (int r = 0; r < nrep; r++)
+        if (dpd_lipid_template(&h->params[r], &mols[r]) != DPD_OK) std::memset(&mols[r], 0, sizeof(dpd_template));
+    CK(cudaMemcpy(dm, mols.data(), (size_t)nrep * sizeof(dpd_template), cudaMemcpyHostToDevice));
     if (h->any_cat && catalyst_setup() != 0)
         return fail(DPD_E_CUDA, "cannot reserve shared memory for the catalyst kernel");
-    CK(cudaMemset(b.stir, 0, (size_t)nrep * sizeof(long long)));
-    // staging for set/get state: 8 float + 3 int32 + 1 byte arrays of nmax
-    TRY(dalloc(h, &h->stage, (size_t)h->nmax * (8 * 4 + 3 * 4 + 1) + 16 * 256));
-    CK(cudaMemset(h->count2[0], 0, 2 * (C + 64) * sizeof(uint32_t)));
     CK(cudaMemset(b.claim, 0xFF, N * sizeof(uint32_t)));
     CK(cudaMemset(b.req, 0xFF, N * sizeof(int32_t)));
-    CK(cudaMemset(b.status, 0, sizeof(DevStatus)));
-    CK(cudaMemset(b.step, 0, sizeof(long long)));
-    CK(cudaMemset(b.obs, 0, (size_t)nrep * OBS_N * sizeof(unsigned long long)));
-    CK(cudaMemset(b.obs_done, 0, (size_t)nrep * sizeof(unsigned int)));
-    for (int k = 0; k < 2; k++) {
-        CK(cudaMemset(b.pos[k], 0, N * sizeof(float2)));
-        CK(cudaMemset(b.vh[k], 0, N * sizeof(float2)));
-        CK(cudaMemset(b.vt[k], 0, N * sizeof(float2)));
-        CK(cudaMemset(b.f[k], 0, N * sizeof(float2)));
-        CK(cudaMemset(b.tg[k], 0, N * sizeof(uint32_t)));
-        CK(cudaMemset(b.link[k], 0xFF, N * sizeof(int2)));
-    }
+    for (int k = 0; k < 2; k++) CK(cudaMemset(b.link[k], 0xFF, N * sizeof(int2)));
     // graph length: even (the buffers alternate every step), ~4M bead-steps per replay
     int g = (int)std::max<int64_t>(1, std::min<int64_t>(64, (4 << 20) / std::max<int64_t>(1, h->N)));
     if (const char *e = getenv("DPD_GRAPH_STEPS")) g = atoi(e);
@@ -667,9 +670,9 @@ extern "C" int dpd_sizes(const dpd_handle *h, int32_t r, int64_t *n_total, int32
 // ---------------------------------------------------------------- status
 
 static int check_status(dpd_handle *h) {
-    DevStatus st;
-    CK(cudaMemcpyAsync(&st, h->b.status, sizeof st, cudaMemcpyDeviceToHost, h->s));
+    CK(cudaMemcpyAsync(&h->host->st, h->b.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, h->s));
     CK(cudaStreamSynchronize(h->s));
+    const DevStatus st = h->host->st;
     if (st.flags) {
         CK(cudaMemsetAsync(&h->b.status->flags, 0, sizeof(unsigned), h->s));
         CK(cudaStreamSynchronize(h->s));
@@ -700,6 +703,21 @@ static int ensure_replica(const dpd_handle *h, int r) {
 
 // ---------------------------------------------------------------- state in/out
 
+// are all of these (null ones aside) memory of the handle's device, aligned for
+// its kernels?  They can then be read or written in place; anything else goes
+// through the staging arrays and copies that take any pointer.
+static bool on_device(const dpd_handle *h, std::initializer_list<const void *> ps, size_t align) {
+    bool ok = true;
+    for (const void *p : ps) {
+        if (!p || !ok) continue;
+        cudaPointerAttributes pa;
+        ok = (uintptr_t)p % align == 0 && cudaPointerGetAttributes(&pa, p) == cudaSuccess &&
+             pa.type == cudaMemoryTypeDevice && pa.device == h->dev;
+    }
+    cudaGetLastError();
+    return ok;
+}
+
 extern "C" int dpd_set_state(dpd_handle *h, int32_t r, const float *x, const float *y, const float *vx,
                              const float *vy, const uint8_t *type, const uint32_t *gid, const int32_t *prev,
                              const int32_t *next) {
@@ -712,21 +730,25 @@ extern "C" int dpd_set_state(dpd_handle *h, int32_t r, const float *x, const flo
     uint32_t *sg = (uint32_t *)(p + 4 * a);
     int32_t *sp = (int32_t *)(p + 5 * a), *sn = (int32_t *)(p + 6 * a);
     uint8_t *st = (uint8_t *)(p + 7 * a);
-    CK(cudaMemcpyAsync(sx, x, n * 4, cudaMemcpyDefault, h->s));
-    CK(cudaMemcpyAsync(sy, y, n * 4, cudaMemcpyDefault, h->s));
-    CK(cudaMemcpyAsync(svx, vx, n * 4, cudaMemcpyDefault, h->s));
-    CK(cudaMemcpyAsync(svy, vy, n * 4, cudaMemcpyDefault, h->s));
-    CK(cudaMemcpyAsync(st, type, n, cudaMemcpyDefault, h->s));
-    if (gid) CK(cudaMemcpyAsync(sg, gid, n * 4, cudaMemcpyDefault, h->s));
-    if (prev) CK(cudaMemcpyAsync(sp, prev, n * 4, cudaMemcpyDefault, h->s));
-    if (next) CK(cudaMemcpyAsync(sn, next, n * 4, cudaMemcpyDefault, h->s));
-    launch_pack(h->b, h->cur, R.b0, (int)n, R.L, sx, sy, svx, svy, st, gid ? sg : nullptr, prev ? sp : nullptr,
-                next ? sn : nullptr, h->s);
+    if (on_device(h, {x, y, vx, vy, gid, prev, next}, 4) && on_device(h, {type}, 1)) {
+        launch_pack(h->b, h->cur, R.b0, (int)n, R.L, x, y, vx, vy, type, gid, prev, next, h->s);
+    } else {
+        CK(cudaMemcpyAsync(sx, x, n * 4, cudaMemcpyDefault, h->s));
+        CK(cudaMemcpyAsync(sy, y, n * 4, cudaMemcpyDefault, h->s));
+        CK(cudaMemcpyAsync(svx, vx, n * 4, cudaMemcpyDefault, h->s));
+        CK(cudaMemcpyAsync(svy, vy, n * 4, cudaMemcpyDefault, h->s));
+        CK(cudaMemcpyAsync(st, type, n, cudaMemcpyDefault, h->s));
+        if (gid) CK(cudaMemcpyAsync(sg, gid, n * 4, cudaMemcpyDefault, h->s));
+        if (prev) CK(cudaMemcpyAsync(sp, prev, n * 4, cudaMemcpyDefault, h->s));
+        if (next) CK(cudaMemcpyAsync(sn, next, n * 4, cudaMemcpyDefault, h->s));
+        launch_pack(h->b, h->cur, R.b0, (int)n, R.L, sx, sy, svx, svy, st, gid ? sg : nullptr, prev ? sp : nullptr,
+                    next ? sn : nullptr, h->s);
+    }
     CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&h->host->st, h->b.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, h->s));
     CK(cudaStreamSynchronize(h->s));
     h->keys_valid = false;
-    unsigned flags = 0;
-    CK(cudaMemcpy(&flags, &h->b.status->flags, sizeof flags, cudaMemcpyDeviceToHost));
+    unsigned flags = h->host->st.flags;
     if (flags & DPD_F_INPUT) {
         flags &= ~DPD_F_INPUT;
         CK(cudaMemcpy(&h->b.status->flags, &flags, sizeof flags, cudaMemcpyHostToDevice));
@@ -742,6 +764,12 @@ extern "C" int dpd_get_state(dpd_handle *h, int32_t r, float *x, float *y, float
     TRY(ensure_replica(h, r));
     const RepDev &R = h->rh[r];
     const size_t n = (size_t)R.n, a = ((n * 4 + 255) / 256) * 256;
+    if (on_device(h, {x, y, vhx, vhy, vtx, vty, fx, fy, gid, prev, next}, 4) && on_device(h, {type}, 1)) {
+        launch_unpack(h->b, h->cur, R.b0, (int)n, x, y, vhx, vhy, vtx, vty, fx, fy, type, gid, prev, next, h->s);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(h->s));
+        return DPD_OK;
+    }
     char *p = h->stage;
     float *f8[8];
     for (int k = 0; k < 8; k++) f8[k] = (float *)(p + k * a);
@@ -1288,10 +1316,9 @@ static void decode_observables(const RepDev &R, const unsigned long long *v, dou
 static int observables_impl(dpd_handle *h, int32_t r, bool virial, double *out) {
     TRY(ensure_replica(h, r));
     if (!out) return fail(DPD_E_ARG, "null out");
-    unsigned long long v[OBS_N];
-    TRY(enqueue_observables(h, r, virial, v));
+    TRY(enqueue_observables(h, r, virial, h->host->row));
     CK(cudaStreamSynchronize(h->s));
-    decode_observables(h->rh[r], v, out);
+    decode_observables(h->rh[r], h->host->row, out);
     return DPD_OK;
 }
 
@@ -1727,9 +1754,16 @@ static void rdf_loss(dpd_handle *h, const dpd_rdf_spec *spec, const std::vector<
 // unordered pairs of the loss types per replica (the types do not change in a window)
 static int count_pairs(dpd_handle *h, const dpd_rdf_spec *spec, std::vector<long long> &npairs) {
     npairs.assign(h->nrep, 0);
+    // every replica's row into obs_out, then one copy
+    for (int r = 0; r < h->nrep; r++)
+        launch_observables(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, r, false, nullptr, 0, h->s);
+    CK(cudaGetLastError());
+    std::vector<unsigned long long> rows((size_t)h->nrep * OBS_N);
+    CK(cudaMemcpyAsync(rows.data(), h->b.obs_out, rows.size() * sizeof(rows[0]), cudaMemcpyDeviceToHost, h->s));
+    CK(cudaStreamSynchronize(h->s));
     for (int r = 0; r < h->nrep; r++) {
         double o[16];
-        TRY(observables_impl(h, r, false, o));
+        decode_observables(h->rh[r], rows.data() + (size_t)r * OBS_N, o);
         const long long na = (long long)o[8 + spec->ta], nb = (long long)o[8 + spec->tb];
         npairs[r] = spec->ta == spec->tb ? na * (na - 1) / 2 : na * nb;
     }
@@ -1941,11 +1975,15 @@ extern "C" int dpd_force_vjp(dpd_handle *h, int32_t r, int64_t step, const float
     const size_t n = (size_t)R.n, N = (size_t)h->N, a = ((n * 4 + 255) / 256) * 256;
     AdjBufs A;
     TRY(adj_setup(h, 0, 0, 1, A));
-    CK(cudaMemsetAsync(A.F[0], 0, N * sizeof(float2), h->s));
     CK(cudaMemsetAsync(A.grad, 0, (size_t)h->nrep * DPD_NGRAD * sizeof(double), h->s));
-    float *sx = (float *)h->stage, *sy = (float *)(h->stage + a);
-    CK(cudaMemcpyAsync(sx, gx, n * 4, cudaMemcpyDefault, h->s));
-    CK(cudaMemcpyAsync(sy, gy, n * 4, cudaMemcpyDefault, h->s));
+    if (h->nrep > 1) CK(cudaMemsetAsync(A.F[0], 0, N * sizeof(float2), h->s));  // the other replicas' cotangents
+    const float *sx = gx, *sy = gy;
+    if (!on_device(h, {gx, gy}, 4)) {
+        sx = (float *)h->stage;
+        sy = (float *)(h->stage + a);
+        CK(cudaMemcpyAsync(h->stage, gx, n * 4, cudaMemcpyDefault, h->s));
+        CK(cudaMemcpyAsync(h->stage + a, gy, n * 4, cudaMemcpyDefault, h->s));
+    }
     // pack the cotangent into the replica's slots via the state packer's force field
     Bufs u = h->b;
     u.f[h->cur] = A.F[0];
@@ -1955,7 +1993,8 @@ extern "C" int dpd_force_vjp(dpd_handle *h, int32_t r, int64_t step, const float
     CK(cudaGetLastError());
     float *outs[4] = {xbar_x, xbar_y, vbar_x, vbar_y};
     float *st[4];
-    for (int k = 0; k < 4; k++) st[k] = (float *)(h->stage + k * a);
+    const bool direct = on_device(h, {xbar_x, xbar_y, vbar_x, vbar_y}, 4);
+    for (int k = 0; k < 4; k++) st[k] = direct ? outs[k] : (float *)(h->stage + k * a);
     Bufs w = h->b;
     w.f[h->cur] = A.xb;
     w.vh[h->cur] = A.vb;
@@ -1963,7 +2002,7 @@ extern "C" int dpd_force_vjp(dpd_handle *h, int32_t r, int64_t step, const float
                   nullptr, nullptr, nullptr, h->s);
     CK(cudaGetLastError());
     for (int k = 0; k < 4; k++)
-        if (outs[k]) CK(cudaMemcpyAsync(outs[k], st[k], n * 4, cudaMemcpyDefault, h->s));
+        if (outs[k] && !direct) CK(cudaMemcpyAsync(outs[k], st[k], n * 4, cudaMemcpyDefault, h->s));
     if (grad) CK(cudaMemcpyAsync(grad, A.grad + (size_t)r * DPD_NGRAD, DPD_NGRAD * sizeof(double), cudaMemcpyDefault, h->s));
     CK(cudaStreamSynchronize(h->s));
     return DPD_OK;

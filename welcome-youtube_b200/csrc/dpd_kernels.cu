@@ -1187,21 +1187,36 @@ __global__ void k_unpack(Bufs b, int cur, int b0, int n, float *x, float *y, flo
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int d = b0 + k;
-    const float2 p = b.pos[cur][d], vh = b.vh[cur][d], vt = b.vt[cur][d], f = b.f[cur][d];
-    if (x) x[k] = p.x;
-    if (y) y[k] = p.y;
-    if (vhx) vhx[k] = vh.x;
-    if (vhy) vhy[k] = vh.y;
-    if (vtx) vtx[k] = vt.x;
-    if (vty) vty[k] = vt.y;
-    if (fx) fx[k] = f.x;
-    if (fy) fy[k] = f.y;
-    const uint32_t tg = b.tg[cur][d];
-    if (type) type[k] = (uint8_t)(tg >> TYPE_SHIFT);
-    if (gid) gid[k] = tg & GID_MASK;
-    const int2 lk = b.link[cur][d];
-    if (prev) prev[k] = lk.x >= 0 ? lk.x - b0 : -1;
-    if (next) next[k] = lk.y >= 0 ? lk.y - b0 : -1;
+    if (x || y) {
+        const float2 p = b.pos[cur][d];
+        if (x) x[k] = p.x;
+        if (y) y[k] = p.y;
+    }
+    if (vhx || vhy) {
+        const float2 v = b.vh[cur][d];
+        if (vhx) vhx[k] = v.x;
+        if (vhy) vhy[k] = v.y;
+    }
+    if (vtx || vty) {
+        const float2 v = b.vt[cur][d];
+        if (vtx) vtx[k] = v.x;
+        if (vty) vty[k] = v.y;
+    }
+    if (fx || fy) {
+        const float2 f = b.f[cur][d];
+        if (fx) fx[k] = f.x;
+        if (fy) fy[k] = f.y;
+    }
+    if (type || gid) {
+        const uint32_t tg = b.tg[cur][d];
+        if (type) type[k] = (uint8_t)(tg >> TYPE_SHIFT);
+        if (gid) gid[k] = tg & GID_MASK;
+    }
+    if (prev || next) {
+        const int2 lk = b.link[cur][d];
+        if (prev) prev[k] = lk.x >= 0 ? lk.x - b0 : -1;
+        if (next) next[k] = lk.y >= 0 ? lk.y - b0 : -1;
+    }
 }
 
 __global__ void k_set_dynamics(Bufs b, int cur, int b0, int n, const float *vhx, const float *vhy, const float *fx,
