@@ -41,7 +41,7 @@ def smoothed(x, y, t, L, ta, tb, nbin, rmax, sigma):
     (12.0, 0.3, 2, 2, 64, 2.0, 0.05),     # the fits' shape
     (9.3, 0.95, 2, 2, 64, 2.0, 0.05),     # over 32 neighbours a bead
     (12.0, 0.3, 1, 2, 65, 2.0, 0.05),     # two types, one bin past the two lane rounds
-    (12.0, 0.3, 2, 0, 300, 1.5, 0.02),    # past one block of 128 bins
+    (12.0, 0.3, 2, 0, 300, 1.5, 0.02),    # past one block of bins
 ])
 def test_window_rdf_and_gradient(cuda_ok, L, f_lip, ta, tb, nbin, rmax, sigma):
     e = ob.Engine(ob.Params(L=L, f_lip=f_lip, seed=3, **PHYS))

@@ -422,30 +422,35 @@ struct RdfPair {
 
 // The CTA's part of its chunk (1 / split of it), its beads of the loss's types
 // listed in shared memory and handed to the warps one at a time: the beads of
-// a cluster, with their many neighbours, spread over the CTA.  A warp scans its
-// bead's window 32 slots a round, each column of cells one contiguous slot
-// range (two where it wraps), and queues the pairs it keeps, so that the
-// Gaussians are evaluated by full rounds:
-//   VJP == false  lane = bin: every lane adds one queued pair's Gaussian at its
-//                 own bins (32 G of them, blockIdx.y says which) to sums it
-//                 holds in FP64 registers; each pair once (j > d)
+// a cluster, with their many neighbours, spread over the CTA.  A warp reads the
+// types of its bead's window 32 slots a round (each column of cells one
+// contiguous slot range, two where it wraps, the ranges found by a lane each)
+// and keeps the slots of the types; takes the distances of those 32 at a time
+// and queues the pairs inside the reach; and evaluates the queue:
+//   VJP == false  half a warp per pair, a lane per bin of its reach: FP64 sums
+//                 in shared memory, a copy per half warp, so no two lanes meet
+//                 (of the nsum bins from blockIdx.y nsum on); each pair once
+//                 (j > d)
 //   VJP == true   lane = pair: the derivative of its bins' Gaussians against
-//                 the bin weights, then a warp sum per bead, in a fixed order
+//                 the bin weights; the bead's sum is taken in the order of the
+//                 window's cells and slots
 // What bounds it: the issue of the scan (about 200 slots around each bead of
 // the types, most of another type) and of 13 Gaussians per pair and side.
-// 24 boxes of 65,536 beads: 290 us (VJP: 405) against 766 (783) with a thread
-// per bead and an FP64 shared atomic per pair and bin; one box of 16,384: 14
-// (17) against 100 (87).
-template <bool VJP, int G>
+// 24 boxes of 65,536 beads: 186 us (VJP: 272) against 766 (783) with a thread
+// per bead and an FP64 shared atomic per pair and bin; one box of 16,384: 10
+// (13) against 100 (87).
+template <bool VJP>
 __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__restrict__ reps,
-                                                  const Chunk *__restrict__ ch, int split, RdfConst q,
+                                                  const Chunk *__restrict__ ch, int split, RdfConst q, int nsum,
                                                   double *__restrict__ hist, const double *__restrict__ wgt,
                                                   float2 *__restrict__ xadd) {
     __shared__ int list[BEAD_TPB];
     __shared__ int nlist, next;
     __shared__ RdfPair queue[RDF_WARPS][RDF_QCAP];
-    __shared__ double red[VJP ? 1 : RDF_WARPS][VJP ? 1 : 32 * G];
-    extern __shared__ float wsh[];  // VJP: the bins' weights
+    __shared__ int cand[RDF_WARPS][RDF_QCAP];
+    __shared__ __align__(16) float part_xy[VJP ? RDF_WARPS : 1][2][VJP ? 36 : 1];
+    extern __shared__ __align__(16) double rdf_sh[];
+    float *wsh = reinterpret_cast<float *>(rdf_sh);  // VJP: the bins' weights
     const Chunk c = ch[blockIdx.x / split];
     const RepDev &R = reps[c.rep];
     const int tid = (int)threadIdx.x, lane = (int)lane_id(), w = tid >> 5;
@@ -455,6 +460,8 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
     }
     if (VJP)
         for (int k = tid; k < q.nbin; k += BEAD_TPB) wsh[k] = (float)wgt[(size_t)c.rep * q.nbin + k];
+    else
+        for (int k = tid; k < 2 * RDF_WARPS * nsum; k += BEAD_TPB) rdf_sh[k] = 0.0;
     __syncthreads();
     const int part = BEAD_TPB / split;
     if (tid < part) {
@@ -473,12 +480,11 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
     const int ncx = R.ncx, ncy = R.ncy;
     const int rcell = min((int)ceilf(rc * (float)R.icsx), (min(ncx, ncy) - 1) / 2);
     const int32_t *__restrict__ cs = sv.cstart + R.c0;
-    const int bin0 = VJP ? 0 : (int)blockIdx.y * 32 * G;
-    double acc[G];
-#pragma unroll
-    for (int g = 0; g < G; g++) acc[g] = 0.0;
-    float gx = 0.0f, gy = 0.0f;
-    int waiting = 0;
+    const int bin0 = VJP ? 0 : (int)blockIdx.y * nsum, bin1 = min(bin0 + nsum, q.nbin);
+    double *acc = rdf_sh + (tid >> 4) * nsum;  // !VJP: this half warp's sums
+    float gx = 0.0f;
+    int waiting = 0, ncand = 0;
+    const uint32_t below = (1u << lane) - 1u;
     // the queued pairs [0, cnt)
     auto evaluate = [&](int cnt) {
         __syncwarp();
@@ -492,22 +498,36 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
                     const float k = kn * __expf(-e * e * inv2s2);
                     dldr += wsh[b] * k * (-e * 2.0f * inv2s2);
                 }
-                gx += dldr * p.dx / p.r;
-                gy += dldr * p.dy / p.r;
+                part_xy[w][0][lane] = dldr * p.dx / p.r;
+                part_xy[w][1][lane] = dldr * p.dy / p.r;
+            } else if (lane < ((cnt + 3) & ~3)) {
+                part_xy[w][0][lane] = part_xy[w][1][lane] = 0.0f;
+            }
+            __syncwarp();
+            if (lane < 2) {  // lane 0 sums x, lane 1 sums y, in order
+                const float4 *v = reinterpret_cast<const float4 *>(part_xy[w][lane]);
+                for (int u = 0; 4 * u < cnt; u++) {
+                    const float4 t = v[u];
+                    gx += t.x;
+                    gx += t.y;
+                    gx += t.z;
+                    gx += t.w;
+                }
             }
         } else {
-            for (int u = 0; u < cnt; u++) {
-                const float r = queue[w][u].r;
-                const uint32_t bins = queue[w][u].bins;
-                const int b0 = (int)(bins & 0xFFFFu) - bin0, b1 = (int)(bins >> 16) - bin0;
-#pragma unroll
-                for (int g = 0; g < G; g++) {
-                    if (b1 < 32 * g || b0 > 32 * g + 31) continue;  // uniform over the warp
-                    const int b = bin0 + 32 * g + lane;
-                    const float rb = (b + 0.5f) * dr, e = r - rb;
-                    const float k = kn * __expf(-e * e * inv2s2);
-                    if (32 * g + lane >= b0 && 32 * g + lane <= b1) acc[g] += (double)k;
+            for (int u = 0; u < cnt; u += 2) {
+                const int e = u + (lane >> 4);
+                if (e < cnt) {
+                    const float r = queue[w][e].r;
+                    const uint32_t bins = queue[w][e].bins;
+                    const int b1 = min((int)(bins >> 16), bin1 - 1);
+                    for (int b = max((int)(bins & 0xFFFFu), bin0) + (lane & 15); b <= b1; b += 16) {
+                        const float rb = (b + 0.5f) * dr, e2 = r - rb;
+                        const float k = kn * __expf(-e2 * e2 * inv2s2);
+                        acc[b - bin0] += (double)k;
+                    }
                 }
+                __syncwarp();
             }
         }
         __syncwarp();
@@ -518,59 +538,86 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
         const float2 pi = sv.pos[d];
         int cx, cy;
         cell_xy(R, pi.x, pi.y, cx, cy);
-        for (int ox = -rcell; ox <= rcell; ox++) {
-            const int nx = cx + ox < 0 ? cx + ox + ncx : (cx + ox >= ncx ? cx + ox - ncx : cx + ox);
-            const int32_t *col = cs + nx * ncy;
-            if (!VJP && col[ncy] <= d) continue;  // earlier slots only
-            for (int seg = -1; seg <= 1; seg++) {  // the rows below 0, inside, and past the top
-                const int r0 = max(cy - rcell, seg * ncy), r1 = min(cy + rcell, seg * ncy + ncy - 1);
-                if (r0 > r1) continue;
-                int js = col[r0 - seg * ncy];
-                const int je = col[r1 - seg * ncy + 1];
-                if (!VJP) js = max(js, d + 1);  // the histogram counts each pair once
-                for (int base = js; base < je; base += 32) {
+        // the distances of candidates [0, cnt), the pairs inside the reach queued
+        auto distances = [&](int cnt) {
+            __syncwarp();
+            RdfPair p;
+            bool keep = false;
+            if (lane < cnt) {
+                const float2 pj = sv.pos[cand[w][lane]];
+                p.dx = minimg(pi.x - pj.x, L, h);
+                p.dy = minimg(pi.y - pj.y, L, h);
+                p.r = sqrtf(p.dx * p.dx + p.dy * p.dy);
+                keep = p.r < rc && p.r != 0.0f;
+            }
+            if (keep) {
+                const int b0 = max(0, (int)floorf((p.r - 4.0f * q.sigma) / dr));
+                const int b1 = min(q.nbin - 1, (int)floorf((p.r + 4.0f * q.sigma) / dr));
+                keep = b0 <= b1 && (VJP || (b1 >= bin0 && b0 < bin1));
+                p.bins = (uint32_t)b0 | (uint32_t)b1 << 16;
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, keep);
+            if (keep) queue[w][waiting + __popc(m & below)] = p;
+            waiting += __popc(m);
+            if (waiting >= 32) {  // a full round now, the rest to the front
+                evaluate(32);
+                waiting -= 32;
+                RdfPair t;
+                if (lane < waiting) t = queue[w][32 + lane];
+                __syncwarp();
+                if (lane < waiting) queue[w][lane] = t;
+            }
+        };
+        const int lo = cy - rcell, hi = cy + rcell;  // 2 rcell + 1 <= ncy: the rows wrap at one end at most
+        for (int g0 = -rcell; g0 <= rcell; g0 += 16) {
+            // a lane's range: column g0 + lane / 2, its first rows or, where they wrap, the others
+            const int ox = g0 + (lane >> 1);
+            int js = 0, je = 0;
+            if (ox <= rcell) {
+                const int nx = cx + ox < 0 ? cx + ox + ncx : (cx + ox >= ncx ? cx + ox - ncx : cx + ox);
+                const int32_t *col = cs + nx * ncy;
+                int r0 = max(lo, 0), r1 = min(hi, ncy - 1);  // the rows inside: first unless rows below 0 come before
+                const bool other = (lane & 1) != (lo < 0 ? 1 : 0);
+                if (other) {
+                    r0 = lo < 0 ? lo + ncy : 0;
+                    r1 = lo < 0 ? ncy - 1 : hi - ncy;
+                }
+                if (r0 <= r1) {
+                    js = col[r0];
+                    je = col[r1 + 1];
+                    if (!VJP) js = max(js, d + 1);  // the histogram counts each pair once
+                }
+            }
+            for (uint32_t m = __ballot_sync(0xffffffffu, js < je); m; m &= m - 1) {
+                const int from = __ffs(m) - 1;
+                const int s = __shfl_sync(0xffffffffu, js, from), e = __shfl_sync(0xffffffffu, je, from);
+                for (int base = s; base < e; base += 32) {
                     const int j = base + lane;
-                    RdfPair p;
-                    bool keep = false;
-                    if (j < je && j != d && rdf_types(q, ti, (int)(sv.tg[j] >> TYPE_SHIFT))) {
-                        const float2 pj = sv.pos[j];
-                        p.dx = minimg(pi.x - pj.x, L, h);
-                        p.dy = minimg(pi.y - pj.y, L, h);
-                        p.r = sqrtf(p.dx * p.dx + p.dy * p.dy);
-                        keep = p.r < rc && p.r != 0.0f;
-                    }
-                    if (keep) {
-                        const int b0 = max(0, (int)floorf((p.r - 4.0f * q.sigma) / dr));
-                        const int b1 = min(q.nbin - 1, (int)floorf((p.r + 4.0f * q.sigma) / dr));
-                        keep = b0 <= b1 && (VJP || (b1 >= bin0 && b0 < bin0 + 32 * G));
-                        p.bins = (uint32_t)b0 | (uint32_t)b1 << 16;
-                    }
-                    const uint32_t m = __ballot_sync(0xffffffffu, keep);
-                    if (keep) queue[w][waiting + __popc(m & ((1u << lane) - 1u))] = p;
-                    waiting += __popc(m);
-                    if (waiting >= 32) {  // a full round now, the rest to the front
-                        evaluate(32);
-                        waiting -= 32;
-                        RdfPair t;
-                        if (lane < waiting) t = queue[w][32 + lane];
+                    const bool ok = j < e && j != d && rdf_types(q, ti, (int)(sv.tg[j] >> TYPE_SHIFT));
+                    const uint32_t t = __ballot_sync(0xffffffffu, ok);
+                    if (ok) cand[w][ncand + __popc(t & below)] = j;
+                    ncand += __popc(t);
+                    if (ncand >= 32) {
+                        distances(32);
+                        ncand -= 32;
+                        const int c1 = lane < ncand ? cand[w][32 + lane] : 0;
                         __syncwarp();
-                        if (lane < waiting) queue[w][lane] = t;
+                        if (lane < ncand) cand[w][lane] = c1;
                     }
                 }
             }
         }
+        distances(ncand);
+        ncand = 0;
         if (VJP) {
             evaluate(waiting);
             waiting = 0;
-            for (int o = 16; o > 0; o >>= 1) {
-                gx += __shfl_xor_sync(0xffffffffu, gx, o);
-                gy += __shfl_xor_sync(0xffffffffu, gy, o);
-            }
+            const float gy = __shfl_sync(0xffffffffu, gx, 1);
             if (lane == 0) {
                 const float2 x = xadd[d];
                 xadd[d] = make_float2(x.x + gx, x.y + gy);
             }
-            gx = gy = 0.0f;
+            gx = 0.0f;
         }
         int nxt = 0;
         if (lane == 0) nxt = atomicAdd(&next, 1);
@@ -578,12 +625,10 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
     }
     if (!VJP) {
         evaluate(waiting);
-#pragma unroll
-        for (int g = 0; g < G; g++) red[w][32 * g + lane] = acc[g];
         __syncthreads();
-        for (int k = tid; k < 32 * G && bin0 + k < q.nbin; k += BEAD_TPB) {
+        for (int k = tid; bin0 + k < bin1; k += BEAD_TPB) {
             double sum = 0.0;
-            for (int u = 0; u < RDF_WARPS; u++) sum += red[u][k];
+            for (int u = 0; u < 2 * RDF_WARPS; u++) sum += rdf_sh[u * nsum + k];
             if (sum != 0.0) atomicAdd(&hist[(size_t)c.rep * q.nbin + bin0 + k], sum);
         }
     }
@@ -727,19 +772,17 @@ void launch_rdf(const StateView &sv, const RepDev *rep, const Chunk *bch, int nb
                 float rmax, float sigma, double *hist, cudaStream_t s) {
     RdfConst q{ta, tb, nbin, rmax, sigma};
     const int split = rdf_split(nbch);
-    // up to 64 bins in one pass over the pairs, more in blocks of 128
-    if (nbin <= 64)
-        k_rdf<false, 2><<<nbch * split, BEAD_TPB, 0, s>>>(sv, rep, bch, split, q, hist, nullptr, nullptr);
-    else
-        k_rdf<false, 4><<<dim3(nbch * split, (nbin + 127) / 128), BEAD_TPB, 0, s>>>(sv, rep, bch, split, q, hist,
-                                                                                    nullptr, nullptr);
+    // up to 256 bins (32 KB of sums a CTA) in one pass over the pairs, more in blocks of 256
+    const int nsum = std::min(nbin, 256);
+    k_rdf<false><<<dim3(nbch * split, (nbin + nsum - 1) / nsum), BEAD_TPB, 2 * RDF_WARPS * nsum * sizeof(double), s>>>(
+        sv, rep, bch, split, q, nsum, hist, nullptr, nullptr);
 }
 
 void launch_rdf_vjp(const StateView &sv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
                     float rmax, float sigma, const double *wgt, float2 *xadd, cudaStream_t s) {
     RdfConst q{ta, tb, nbin, rmax, sigma};
     const int split = rdf_split(nbch);
-    k_rdf<true, 1><<<nbch * split, BEAD_TPB, nbin * sizeof(float), s>>>(sv, rep, bch, split, q, nullptr, wgt, xadd);
+    k_rdf<true><<<nbch * split, BEAD_TPB, nbin * sizeof(float), s>>>(sv, rep, bch, split, q, 0, nullptr, wgt, xadd);
 }
 
 void launch_adj_state(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *X,
