@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(BEAD_TPB) k_gsum(const RepDev *__restrict__ re
 }
 
 #define VJP_TPB 256
-#define VJP_LIST 32         // hits a bead collects before they are evaluated
+#define VJP_LIST 32         // pairs a bead lists at a time
 #define VJP_TYPES 4         // types whose pairs have lane-private gradient sums
 #define VJP_COMBOS (VJP_TYPES * (VJP_TYPES + 1) / 2)
 
@@ -152,24 +152,29 @@ __device__ __forceinline__ void adj_update(const AdjUpdate &u, const RepDev &R, 
     u.F2[o] = make_float2(R.dt2 * x.x + R.dt * v0.x + R.cvt * vf.x, R.dt2 * x.y + R.dt * v0.y + R.cvt * vf.y);
 }
 
-// LPB lanes share a bead: they take its 3 x 3 cells' slots in turn (cells are
-// column-major: three contiguous ranges, and three more where the rows wrap),
-// list the ones inside the cutoff, then take the listed pairs in turn, so that
-// the noise and the derivative run on lanes that all have a pair.  Each pair is
-// evaluated by both of its beads: every bead's sums are made by its own lanes
-// in a fixed order, with no atomics on floats.  The sums of the parameters'
-// gradient are FP64: per lane and pair of types in shared memory for the first
-// four types (no two lanes on one word), through an atomic for the others.
+// LPB lanes share a bead: each takes its part of the bead's 3 x 3 cells' slots
+// (cells are column-major: three contiguous ranges, six where the rows wrap)
+// and marks the ones inside the cutoff in a word; the bead's hits are listed in
+// the order of its cells and slots and evaluated by its lanes in turn, so that
+// the noise and the derivative run on lanes that have a pair.  Each pair is
+// evaluated by both of its beads: no atomics on floats, and a bead's terms are
+// added in its list's order, as a thread per bead would add them (the same
+// bits).  The sums of the parameters' gradient are FP64: per lane and pair of
+// types in shared memory for the first four types (no two lanes on one word),
+// through an atomic for the others.
 // A CTA takes a run of consecutive tasks (256 / LPB beads of a chunk) and hands
 // its gradient sums over when the replica changes and at its end.  UPDATE: the
 // adjoint of the step's update is applied at once (adj_update); else the
 // products go to xbar and vbar.
-// What bounds it: instruction issue (175 warp instructions a bead at density 4,
-// 2.2 of 4 a cycle: half of them the 12.6 evaluations, 40 of whose 130
-// instructions are the noise) and the fullest list of a warp, 1.6 times the
-// mean.  24 boxes of 65,536 beads: 374 us, against 939 with a thread per bead
-// and an FP64 shared atomic per pair; one box: 32 against 68, of 16,384: 14
-// against 60, of 4,096: 11 against 61.
+// What bounds it: instruction issue (about 180 warp instructions a bead at
+// density 4, 2.2 of 4 a cycle: half of them the 12.6 evaluations, 40 of whose
+// 140 instructions are the noise) and the fullest list of a warp, 1.6 times the
+// mean.  24 boxes of 65,536 beads: 434 us, against 939 (and 82 for the update)
+// with a thread per bead and an FP64 shared atomic per pair; one box: 34
+// against 68, of 16,384: 14 against 60, of 4,096: 10 against 61.  Tried: one
+// queue of pairs per warp evaluated by full rounds, its terms summed through
+// shared memory, 504 us (more shared memory, 16 warps an SM); the order of the
+// sum left to the lanes, 397 us.
 template <int LPB, int MINB, bool UPDATE>
 __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long long step, const RepDev *__restrict__ reps,
                                                        const Chunk *__restrict__ ch, int ntask,
@@ -191,7 +196,7 @@ __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long 
     const int t0 = (int)((long long)ntask * blockIdx.x / gridDim.x);
     const int t1 = (int)((long long)ntask * (blockIdx.x + 1) / gridDim.x);
     int rep = -1;
-    float gam = 0.0f, s = 0.0f, sg = 0.0f;  // sg = s / (2 gamma): d s / d gamma
+    float gam = 0.0f, s = 0.0f;
     NoiseKey nk;
     // the CTA's gradient sums of replica `rep`, added to the global ones
     auto hand_over = [&]() {
@@ -228,7 +233,6 @@ __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long 
             if (tid < DPD_MAXT * DPD_MAXT) a_sh[tid] = R.a[tid];
             gam = R.gamma;
             s = sdt_at(R, step);
-            sg = gam > 0.0f ? s / (2.0f * gam) : 0.0f;
             nk = make_noise_key(R, step);
             __syncthreads();
         }
@@ -249,143 +253,208 @@ __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long 
         }
         const uint32_t gi = tgi & GID_MASK;
         const int ti = (int)(tgi >> TYPE_SHIFT);
-        // does some bead of the warp sit in an edge cell (its neighbours' images matter)
-        const bool wrap = __any_sync(0xffffffffu, act && (cx == 0 || cx == ncx - 1 || cy == 0 || cy == ncy - 1));
-        float xbx = 0.f, xby = 0.f, vbx = 0.f, vby = 0.f;
-        int n = 0;  // listed hits of the bead (the same in its lanes)
-        auto evaluate = [&]() {
-            __syncwarp();
-            for (int k = sub; k < n; k += LPB) {
-                const int j = list[bead][k];
-                const float2 pj = sv.pos[j], vj = sv.vt[j], gj = g[j];
-                const uint32_t tgj = sv.tg[j];
-                const int tj = (int)(tgj >> TYPE_SHIFT);
-                float dx = __fsub_rn(pi.x, pj.x), dy = __fsub_rn(pi.y, pj.y);
-                if (wrap) {
-                    dx = minimg(dx, L, h);
-                    dy = minimg(dy, L, h);
-                }
-                const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
-                float r, ir;
-                r_and_ir(r2, r, ir);
-                const float w = 1.0f - r;
-                const float dvx = vi.x - vj.x, dvy = vi.y - vj.y;
-                const float rv = (dx * dvx + dy * dvy) * ir;
-                const float th = pair_theta(nk, gi, tgj & GID_MASK);
-                const float a = a_sh[ti * DPD_MAXT + tj];
-                const float A = a - gam * w * rv + s * th;
-                const float fm = w * A * ir;
-                const float cxv = gi2.x - gj.x, cyv = gi2.y - gj.y;
-                const float cd = cxv * dx + cyv * dy;
-                const float dfr = (-A + w * gam * rv) * ir - w * A * ir * ir;
-                const float dfv = -gam * w * w * ir;
-                const float hx = dx * ir, hy = dy * ir;
-                xbx += cd * (dfr * hx + dfv * (dvx - rv * hx) * ir) + fm * cxv;
-                xby += cd * (dfr * hy + dfv * (dvy - rv * hy) * ir) + fm * cyv;
-                vbx += cd * dfv * hx;
-                vby += cd * dfv * hy;
-                if (gi < (tgj & GID_MASK)) {  // parameter gradients: each pair once
-                    const int lo = min(ti, tj), hi = max(ti, tj);
-                    const double da = (double)(cd * w * ir);
-                    if (hi < VJP_TYPES) acc[lo * (2 * VJP_TYPES - 1 - lo) / 2 + hi][tid] += da;
-                    else atomicAdd(&sgrad[lo * DPD_MAXT + hi], da);
-                    ggam += (double)(cd * w * (-w * rv + sg * th) * ir);
-                }
+        const bool low = act && cy == 0, high = act && cy == ncy - 1;  // ncy >= 3: the rows wrap at one end
+        // does some bead of the warp sit in an edge cell (its neighbours' images matter), or in one of an edge row
+        const bool rows = __any_sync(0xffffffffu, low || high);
+        const bool wrap = rows || __any_sync(0xffffffffu, act && (cx == 0 || cx == ncx - 1));
+        // the slots of the bead's columns in order: three ranges, or six; l: ends of the ranges counted together,
+        // b: what leads from that count to the slot
+        int l0 = 0, l1 = 0, l2 = 0, l3 = 0, l4 = 0, l5 = 0, b0 = 0, b1 = 0, b2 = 0, b3 = 0, b4 = 0, b5 = 0;
+        if (act) {
+            const int32_t *c0 = cs + (cx > 0 ? cx - 1 : ncx - 1) * ncy, *c1 = cs + cx * ncy;
+            const int32_t *c2 = cs + (cx + 1 < ncx ? cx + 1 : 0) * ncy;
+            if (!rows) {
+                b0 = c0[cy - 1];
+                b1 = c1[cy - 1];
+                b2 = c2[cy - 1];
+                l0 = c0[cy + 2] - b0;
+                l1 = l0 + (c1[cy + 2] - b1);
+                l2 = l1 + (c2[cy + 2] - b2);
+                b1 -= l0;
+                b2 -= l1;
+                l3 = l4 = l5 = l2;
+            } else {
+                // the rows before the wrap [ra, rb) and after it [rc, rd): row ncy - 1 then 0, 1; or ncy - 2, ncy - 1
+                // then 0; or cy - 1 .. cy + 1 and none
+                const int ra = low ? ncy - 1 : cy - 1, rb = low || high ? ncy : cy + 2;
+                const int rc = 0, rd = low ? 2 : (high ? 1 : 0);
+                b0 = c0[ra];
+                l0 = c0[rb] - b0;
+                b1 = c0[rc];
+                l1 = l0 + (c0[rd] - b1);
+                b2 = c1[ra];
+                l2 = l1 + (c1[rb] - b2);
+                b3 = c1[rc];
+                l3 = l2 + (c1[rd] - b3);
+                b4 = c2[ra];
+                l4 = l3 + (c2[rb] - b4);
+                b5 = c2[rc];
+                l5 = l4 + (c2[rd] - b5);
+                b1 -= l0;
+                b2 -= l1;
+                b3 -= l2;
+                b4 -= l3;
+                b5 -= l4;
             }
-            n = 0;
-            __syncwarp();
+        }
+        auto slot = [&](int k) {
+            if (!rows) return k + (k < l0 ? b0 : (k < l1 ? b1 : b2));
+            return k + (k < l0 ? b0 : (k < l1 ? b1 : (k < l2 ? b2 : (k < l3 ? b3 : (k < l4 ? b4 : b5)))));
         };
-        // the slots of rows [ra, rb] of the three columns, taken by the bead's lanes
-        // in turn, VJP_LIST a block: each lane marks its hits in a word, then lists them
-        auto sweep = [&](bool on, int ra, int rb) {
-            int s0 = 0, s1 = 0, s2 = 0, l0 = 0, l1 = 0, l2 = 0;
-            if (on) {
-                const int32_t *c0 = cs + (cx > 0 ? cx - 1 : ncx - 1) * ncy, *c1 = cs + cx * ncy;
-                const int32_t *c2 = cs + (cx + 1 < ncx ? cx + 1 : 0) * ncy;
-                s0 = c0[ra];
-                s1 = c1[ra];
-                s2 = c2[ra];
-                l0 = c0[rb + 1] - s0;
-                l1 = l0 + (c1[rb + 1] - s1);
-                l2 = l1 + (c2[rb + 1] - s2);
-                s1 -= l0;
-                s2 -= l1;
-            }
-            const int most = __reduce_max_sync(0xffffffffu, l2);
-            for (int kb = 0; kb < most; kb += VJP_LIST) {
-                uint32_t mark = 0;
-                const int rounds = min(VJP_LIST / LPB, (most - kb + LPB - 1) / LPB);
-#pragma unroll 4
-                for (int u = 0; u < rounds; u++) {
-                    const int k = kb + u * LPB + sub;
-                    const int j = k + (k < l0 ? s0 : (k < l1 ? s1 : s2));
-                    const float2 pj = sv.pos[k < l2 ? j : 0];
+        float xbx = 0.f, xby = 0.f, vbx = 0.f, vby = 0.f;  // x_bar in the bead's first lane, v_bar in its second
+        // the listed pairs [0, n) of every bead, in turn; their terms are added in the list's order
+        auto evaluate = [&](int n) {
+            __syncwarp();
+            const int rounds = (__reduce_max_sync(0xffffffffu, n) + LPB - 1) / LPB;
+            for (int q = 0; q < rounds; q++) {
+                const int k = q * LPB + sub;
+                float tx = 0.f, ty = 0.f, u = 0.f, hx = 0.f, hy = 0.f;
+                if (k < n) {
+                    const int j = list[bead][k];
+                    const float2 pj = sv.pos[j], vj = sv.vt[j], gj = g[j];
+                    const uint32_t tgj = sv.tg[j];
+                    const int tj = (int)(tgj >> TYPE_SHIFT);
                     float dx = __fsub_rn(pi.x, pj.x), dy = __fsub_rn(pi.y, pj.y);
                     if (wrap) {
                         dx = minimg(dx, L, h);
                         dy = minimg(dy, L, h);
                     }
                     const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
-                    mark |= (k < l2 && r2 < 1.0f && r2 > 1e-24f && j != d ? 1u : 0u) << u;
+                    float r, ir;
+                    r_and_ir(r2, r, ir);
+                    const float w = 1.0f - r;
+                    const float dvx = vi.x - vj.x, dvy = vi.y - vj.y;
+                    const float rv = (dx * dvx + dy * dvy) * ir;
+                    const float th = pair_theta(nk, gi, tgj & GID_MASK);
+                    const float a = a_sh[ti * DPD_MAXT + tj];
+                    const float A = a - gam * w * rv + s * th;
+                    const float fm = w * A * ir;
+                    const float cxv = gi2.x - gj.x, cyv = gi2.y - gj.y;
+                    const float cd = cxv * dx + cyv * dy;
+                    const float dfr = (-A + w * gam * rv) * ir - w * A * ir * ir;
+                    const float dfv = -gam * w * w * ir;
+                    hx = dx * ir;
+                    hy = dy * ir;
+                    tx = __fmaf_rn(fm, cxv, __fmul_rn(cd, dfr * hx + dfv * (dvx - rv * hx) * ir));
+                    ty = __fmaf_rn(fm, cyv, __fmul_rn(cd, dfr * hy + dfv * (dvy - rv * hy) * ir));
+                    u = cd * dfv;
+                    if (gi < (tgj & GID_MASK)) {  // parameter gradients: each pair once
+                        const int lo = min(ti, tj), hi = max(ti, tj);
+                        const double da = (double)(cd * w * ir);
+                        if (hi < VJP_TYPES) acc[lo * (2 * VJP_TYPES - 1 - lo) / 2 + hi][tid] += da;
+                        else atomicAdd(&sgrad[lo * DPD_MAXT + hi], da);
+                        ggam += (double)(cd * w * (-w * rv + (gam > 0.0f ? s * th / (2.0f * gam) : 0.0f)) * ir);
+                    }
                 }
-                int at = __popc(mark), all = at;  // this lane's place in its bead's list
+                if (LPB == 2) {  // each lane hands the other what it sums
+                    const float o1 = __shfl_xor_sync(0xffffffffu, sub ? tx : u, 1);
+                    const float o2 = __shfl_xor_sync(0xffffffffu, sub ? ty : hx, 1);
+                    const float o3 = __shfl_xor_sync(0xffffffffu, hy, 1);
+                    const int left = n - q * LPB;
+                    if (sub == 0) {
+                        if (left > 0) {
+                            xbx += tx;
+                            xby += ty;
+                        }
+                        if (left > 1) {
+                            xbx += o1;
+                            xby += o2;
+                        }
+                    } else {
+                        if (left > 0) {
+                            vbx = __fmaf_rn(o1, o2, vbx);
+                            vby = __fmaf_rn(o1, o3, vby);
+                        }
+                        if (left > 1) {
+                            vbx = __fmaf_rn(u, hx, vbx);
+                            vby = __fmaf_rn(u, hy, vby);
+                        }
+                    }
+                } else {
 #pragma unroll
-                for (int o = 1; o < LPB; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, at, o, LPB);
-                    if (sub >= o) at += t;
+                    for (int i = 0; i < LPB; i++) {
+                        const float ax = __shfl_sync(0xffffffffu, tx, i, LPB), ay = __shfl_sync(0xffffffffu, ty, i, LPB);
+                        const float au = __shfl_sync(0xffffffffu, u, i, LPB), ahx = __shfl_sync(0xffffffffu, hx, i, LPB);
+                        const float ahy = __shfl_sync(0xffffffffu, hy, i, LPB);
+                        if (q * LPB + i < n) {
+                            xbx += ax;
+                            xby += ay;
+                            vbx = __fmaf_rn(au, ahx, vbx);
+                            vby = __fmaf_rn(au, ahy, vby);
+                        }
+                    }
                 }
-                const int end = __shfl_sync(0xffffffffu, at, LPB - 1, LPB);
-                at -= all;
-                if (__any_sync(0xffffffffu, n + end > VJP_LIST)) evaluate();
-                at += n;
-                while (mark) {
-                    const int k = kb + (__ffs(mark) - 1) * LPB + sub;
-                    mark &= mark - 1;
-                    list[bead][at++] = k + (k < l0 ? s0 : (k < l1 ? s1 : s2));
-                }
-                n += end;
             }
+            __syncwarp();
         };
-        sweep(act, max(cy - 1, 0), min(cy + 1, ncy - 1));
-        const bool low = act && cy == 0, high = act && cy == ncy - 1;  // ncy >= 3
-        if (__any_sync(0xffffffffu, low || high)) sweep(low || high, low ? ncy - 1 : 0, low ? ncy - 1 : 0);
-        evaluate();
-        if (act) {
+        // each lane marks the hits of its part of the slots in a word; then the bead's hits are listed in order
+        const int per = (l5 + LPB - 1) / LPB, k0 = sub * per, k1 = min(k0 + per, l5);
+        const int most = __reduce_max_sync(0xffffffffu, per);
+        for (int kb = 0; kb < most; kb += 32) {
+            uint32_t mark = 0;
+            const int rounds = min(32, most - kb);
+#pragma unroll 4
+            for (int u = 0; u < rounds; u++) {
+                const int k = k0 + kb + u, j = slot(k);
+                const bool in = k < k1;
+                const float2 pj = sv.pos[in ? j : 0];
+                float dx = __fsub_rn(pi.x, pj.x), dy = __fsub_rn(pi.y, pj.y);
+                if (wrap) {
+                    dx = minimg(dx, L, h);
+                    dy = minimg(dy, L, h);
+                }
+                const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+                mark |= (in && r2 < 1.0f && r2 > 1e-24f && j != d ? 1u : 0u) << u;
+            }
+            int at = __popc(mark);  // the place of this lane's first hit among its bead's
+            const int own = at;
+#pragma unroll
+            for (int o = 1; o < LPB; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, at, o, LPB);
+                if (sub >= o) at += t;
+            }
+            const int n = __shfl_sync(0xffffffffu, at, LPB - 1, LPB);
+            at -= own;
+            for (int first = 0; __any_sync(0xffffffffu, first < n); first += VJP_LIST) {  // once, unless crowded
+                int to = at - first;
+                for (uint32_t m = mark; m; m &= m - 1, to++)
+                    if (to >= 0 && to < VJP_LIST) list[bead][to] = slot(k0 + kb + __ffs(m) - 1);
+                evaluate(max(0, min(n - first, VJP_LIST)));
+            }
+        }
+        if (LPB == 2) {
+            vbx = __shfl_down_sync(0xffffffffu, vbx, 1);
+            vby = __shfl_down_sync(0xffffffffu, vby, 1);
+        }
+        if (act && sub == 0) {
             // bonds: f_i = kb (1 - r0/r) d with d = x_p - x_i (linear chains; the
-            // branched shapes' bonds and angles are k_mol_vjp's), a lane per end
+            // branched shapes' bonds and angles are k_mol_vjp's)
             const int2 lk = R.arch == 0 ? sv.link[d] : make_int2(-1, -1);
 #pragma unroll
             for (int q = 0; q < 2; q++) {
                 const int p = q ? lk.y : lk.x;
-                if (p < 0 || sub != q % LPB) continue;
+                if (p < 0) continue;
                 const float2 pp = sv.pos[p], gp = g[p];
                 const float dx = minimg(pp.x - pi.x, L, h), dy = minimg(pp.y - pi.y, L, h);
                 const float r = sqrtf(dx * dx + dy * dy);
                 const float cxv = gi2.x - gp.x, cyv = gi2.y - gp.y;
                 const float cd = cxv * dx + cyv * dy;
                 const float u = 1.0f - R.r0 / r;
-                const float k0 = R.kb * R.r0 / (r * r) * cd / r;
-                xbx -= k0 * dx + R.kb * u * cxv;
-                xby -= k0 * dy + R.kb * u * cyv;
+                const float kr = R.kb * R.r0 / (r * r) * cd / r;
+                xbx -= kr * dx + R.kb * u * cxv;
+                xby -= kr * dy + R.kb * u * cyv;
                 if (q == 1) gkb += (double)(u * cd);  // each bond once, from its prev end
             }
-            if (R.ka != 0.0f && (lk.x >= 0 || lk.y >= 0) && sub == 2 % LPB) {
+            if (R.ka != 0.0f && (lk.x >= 0 || lk.y >= 0)) {
                 const float2 t = angle_vjp(sv, g, R, pi, gi2, lk);
                 xbx += t.x;
                 xby += t.y;
             }
-            if (R.stir_A != 0.0f && sub == 3 % LPB) {
+            if (R.stir_A != 0.0f) {
                 const double w2 = 2.0 * R.stir_k;
                 const double dfy = (double)R.stir_A * M_PI * w2 * cospi(w2 * (double)pi.y);
                 xby += (float)(dfy * ((double)gi2.x - gsum[c.rep] / (double)R.n));
             }
-        }
-#pragma unroll
-        for (int o = LPB / 2; o > 0; o >>= 1) {
-            xbx += __shfl_xor_sync(0xffffffffu, xbx, o);
-            xby += __shfl_xor_sync(0xffffffffu, xby, o);
-            vbx += __shfl_xor_sync(0xffffffffu, vbx, o);
-            vby += __shfl_xor_sync(0xffffffffu, vby, o);
         }
         if (act && sub == 0) {
             if (UPDATE) {
@@ -740,10 +809,10 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
         cudaMemsetAsync(gsum, 0, (size_t)nrep * sizeof(double), s);
         k_gsum<<<nbch, BEAD_TPB, 0, s>>>(rep, bch, g, gsum);
     }
-    // lanes per bead: eight or four while the tasks fit the GPU at once (a small box is latency: 4,096 beads take
+    // lanes per bead: eight or four while the tasks fit the GPU at once (a small box is latency: 4,096 beads took
     // 10.8 us with eight against 13.3 with four and 17.3 with two; 16,384 beads 14.1 with four, 17.4 with two), else two,
-    // whose lanes wait less for the fullest list (24 boxes of 65,536: 374 us, 455 with four, 585 with eight); then
-    // three CTAs an SM at 80 registers, two otherwise
+    // whose lanes wait less for the fullest list (24 boxes of 65,536: 374 us, 455 with four, 585 with eight, before the
+    // sums were ordered); then three CTAs an SM at 80 registers, two otherwise
     const bool update = up && !mol;  // the branched shapes add their share first
     const AdjUpdate none{};
     auto go = [&](auto kern, int lpb, int per_sm) {
