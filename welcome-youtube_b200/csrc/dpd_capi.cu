@@ -88,6 +88,7 @@ struct dpd_handle {
     int tile_w = 8, tile_h = 16;
     TileDesc *d_tiles = nullptr;
     int ntiles = 0;
+    std::vector<int32_t> tile0; // first tile of each replica, and the end
     bool any_chem = false;
     bool any_stir = false;      // some replica stirs: its term sums are cleared before each permute
     bool keys_valid = false;
@@ -366,19 +367,26 @@ static int build_tiles(dpd_handle *h) {
     if (h->tile_w < 1 || h->tile_h < 1 || (h->tile_w + 2) * (h->tile_h + 2) > maxc)
         return fail(DPD_E_ARG, "tile shape %dx%d: need (w+2)(h+2) <= %d", h->tile_w, h->tile_h, maxc);
     std::vector<TileDesc> t;
+    h->tile0.clear();
     for (int r = 0; r < h->nrep; r++) {
+        h->tile0.push_back((int32_t)t.size());
         const RepDev &R = h->rh[r];
         const int w = std::min(h->tile_w, R.ncx - 2), hh = std::min(h->tile_h, R.ncy - 2);
         for (int cx = 0; cx < R.ncx; cx += w)
             for (int cy = 0; cy < R.ncy; cy += hh)
                 t.push_back({r, cx, cy, std::min(w, R.ncx - cx), std::min(hh, R.ncy - cy), (int32_t)R.c0, R.ncx, R.ncy});
     }
-    if (h->d_tiles) {
-        cudaFree(h->d_tiles);
+    h->tile0.push_back((int32_t)t.size());
+    for (void *old : {(void *)h->d_tiles, (void *)h->b.rowpart}) {
+        if (!old) continue;
+        cudaFree(old);
         for (auto &p : h->allocs)
-            if (p == (void *)h->d_tiles) p = nullptr;
+            if (p == old) p = nullptr;
     }
+    h->d_tiles = nullptr;
+    h->b.rowpart = nullptr;
     TRY(dalloc(h, &h->d_tiles, t.size()));
+    TRY(dalloc(h, &h->b.rowpart, t.size() * ROW_WORDS));
     CK(cudaMemcpy(h->d_tiles, t.data(), t.size() * sizeof(TileDesc), cudaMemcpyHostToDevice));
     h->ntiles = (int)t.size();
     return DPD_OK;
@@ -431,17 +439,44 @@ static Bufs at_parity(const dpd_handle *h, Bufs b, int cur) {
     return b;
 }
 
-// the sort of buffer cur's counted keys into cell order (cell starts, src, dest); part: see dpd_profile_step
-static void enqueue_cell_sort(dpd_handle *h, const Bufs &b0, int cur, bool step_inc) {
+// the row the tile force kernel assembles for the stats ring, if one is registered
+static RowOut ring_row(const dpd_handle *h) {
+    RowOut row;
+    if (!h->ring || h->force_kernel != 0) return row;
+    row.rep = h->ring_rep;
+    row.slots = h->ring_slots;
+    row.host = h->ring;
+    row.tile0 = h->tile0[row.rep];
+    row.ntile = h->tile0[row.rep + 1] - row.tile0;
+    return row;
+}
+
+// the stirring sums are accumulated by the permute kernel and read by the forces
+static void clear_stir(dpd_handle *h, const Bufs &b) {
+    if (h->any_stir) cudaMemsetAsync(b.stir, 0, (size_t)h->nrep * sizeof(long long), h->s);
+}
+
+// The sort of buffer cur's counted keys into cell order (cell starts, src,
+// dest), with the stirring sums cleared for the permute that follows and row,
+// the stats row of the step before, collected.
+static void enqueue_cell_sort(dpd_handle *h, const Bufs &b0, int cur, bool step_inc, RowOut row = RowOut()) {
     const Bufs b = at_parity(h, b0, cur);
+    StepHead head;
+    head.row = row;
+    if (h->any_stir) {
+        head.stir = b.stir;
+        head.nstir = h->nrep;
+    }
     if (b.bins) {
-        launch_sort_bins(b, h->count2[cur ^ 1], h->C, step_inc, h->d_rep, h->d_cch, h->ncch, -1, h->s);
+        launch_sort_bins(b, h->count2[cur ^ 1], h->C, step_inc, h->d_rep, h->d_cch, h->ncch, -1, head, h->s);
         return;
     }
     if (h->sort_mode == 2 && sort_pfx_fits(h->C)) {
-        launch_sort_pfx(b, h->C, step_inc, h->d_bch, h->nbch, h->d_cch, h->ncch, -1, h->s);
+        launch_sort_pfx(b, h->C, step_inc, h->d_bch, h->nbch, h->d_cch, h->ncch, -1, head, h->s);
         return;
     }
+    if (row.rep >= 0) launch_row_collect(b, row, h->s);
+    clear_stir(h, b);
     enqueue_scan(h, b, step_inc);
     launch_place(b, h->d_bch, h->nbch, h->s);
     launch_cellfix(b, h->d_cch, h->ncch, h->s);
@@ -464,7 +499,7 @@ static void enqueue_keys(dpd_handle *h, const Bufs &b0, int cur, bool next) {
 // forces of buffer cur of b.  row: a stats row the tile kernel assembles on the
 // way (the other kernels leave it to the caller)
 static void enqueue_forces(dpd_handle *h, const Bufs &b0, int cur, bool next_keys,
-                           RowOut row = RowOut{-1, 0, nullptr}) {
+                           RowOut row = RowOut()) {
     const Bufs b = at_parity(h, b0, cur);
     if (h->any_mol) launch_mol_forces(b, cur, h->d_rep, h->d_bch, h->nbch, h->s);
     if (h->force_kernel == 0)
@@ -562,6 +597,7 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
     want(&b.obs, (size_t)nrep * OBS_N);
     want(&b.obs_out, (size_t)nrep * OBS_N);
     want(&b.obs_done, (size_t)nrep);
+    want(&b.row_pending, 1);
     want(&b.hist, 4096);
     want(&b.stir, (size_t)nrep);
     want(&b.rng, (size_t)4 * nrep);
@@ -812,16 +848,10 @@ extern "C" int dpd_set_dynamics(dpd_handle *h, int32_t r, const float *vhx, cons
 
 // ---------------------------------------------------------------- phases
 
-// the stirring sums are accumulated by the permute kernel and read by the forces
-static void clear_stir(dpd_handle *h, const Bufs &b) {
-    if (h->any_stir) cudaMemsetAsync(b.stir, 0, (size_t)h->nrep * sizeof(long long), h->s);
-}
-
 static void enqueue_sort(dpd_handle *h, PermuteMode mode) {
     // counts of the CURRENT positions
     enqueue_keys(h, h->b, h->cur, false);
     enqueue_cell_sort(h, h->b, h->cur, false);
-    clear_stir(h, h->b);
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, mode, h->s);
     h->cur ^= 1;
 }
@@ -977,12 +1007,14 @@ static bool cat_at(const dpd_handle *h, int64_t s) {
 // fuse the update into the sort whose counts the previous force kernel made.
 static void enqueue_step(dpd_handle *h, int64_t s) {
     const bool cat = cat_at(h, s);
+    const RowOut row = ring_row(h);
     if (!cat) {
-        enqueue_cell_sort(h, h->b, h->cur, true);
+        enqueue_cell_sort(h, h->b, h->cur, true, row);
     } else {
+        if (row.rep >= 0) launch_row_collect(h->b, row, h->s);
         launch_step_begin(h->b, h->nrep, h->s);
+        clear_stir(h, h->b);
     }
-    clear_stir(h, h->b);
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, cat ? PERM_KEEP : PERM_STEP, h->s);
     h->cur ^= 1;
     if (h->any_lipid) launch_chem_lists(h->b, h->cur, h->d_rep, -1, h->s);
@@ -993,8 +1025,8 @@ static void enqueue_step(dpd_handle *h, int64_t s) {
     }
     // the step's stats row into the ring: assembled by the tile force kernel's
     // epilogue from the beads it holds anyway, else by a pass of its own
-    if (h->ring && h->force_kernel == 0) {
-        enqueue_forces(h, h->b, h->cur, true, RowOut{h->ring_rep, h->ring_slots, h->ring});
+    if (row.rep >= 0) {
+        enqueue_forces(h, h->b, h->cur, true, row);
     } else {
         enqueue_forces(h, h->b, h->cur, true);
         if (h->ring)
@@ -1046,6 +1078,8 @@ static int enqueue_steps(dpd_handle *h, int64_t nsteps) {
             s++;
         }
     }
+    const RowOut row = ring_row(h);
+    if (row.rep >= 0) launch_row_collect(h->b, row, h->s);  // the last step's row
     CK(cudaGetLastError());
     h->step += nsteps;
     return DPD_OK;
@@ -1137,8 +1171,8 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
     uint32_t *other = h->count2[h->cur ^ 1];
     const bool pfx = h->sort_mode == 2 && sort_pfx_fits(h->C);
     if (!cat) {
-        if (sb.bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 0, h->s);
-        else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 0, h->s);
+        if (sb.bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 0, StepHead(), h->s);
+        else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 0, StepHead(), h->s);
         else if (h->sort_mode == 1) launch_scan_lb(sb, h->C, true, h->s);
         else launch_scan_part(sb, h->C, true, 1, h->s);
     } else {
@@ -1148,13 +1182,13 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
     if (!cat && h->sort_mode == 0) launch_scan_part(sb, h->C, true, 2, h->s);
     CK(cudaEventRecord(ev[k++], h->s));
     if (!cat && !sb.bins) {
-        if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 1, h->s);
+        if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 1, StepHead(), h->s);
         else launch_place(sb, h->d_bch, h->nbch, h->s);
     }
     CK(cudaEventRecord(ev[k++], h->s));
     if (!cat) {
-        if (sb.bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 1, h->s);
-        else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 2, h->s);
+        if (sb.bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 1, StepHead(), h->s);
+        else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 2, StepHead(), h->s);
         else launch_cellfix(sb, h->d_cch, h->ncch, h->s);
     }
     CK(cudaEventRecord(ev[k++], h->s));
@@ -1573,7 +1607,6 @@ static StateView view_cur(dpd_handle *h) {
 
 static void enqueue_plain_step(dpd_handle *h) {  // one step without chemistry (windows require chem off)
     enqueue_cell_sort(h, h->b, h->cur, true);
-    clear_stir(h, h->b);
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, PERM_STEP, h->s);
     h->cur ^= 1;
     enqueue_forces(h, h->b, h->cur, true);
@@ -1610,7 +1643,6 @@ static void enqueue_seg_step(dpd_handle *h, AdjBufs &A, int sg, int s, int par0)
     const Bufs b = seg_bufs(h, A, sg, s, par0);
     const int from = (par0 + s - 1) & 1;
     enqueue_cell_sort(h, b, from, true);
-    clear_stir(h, b);
     launch_permute(b, from, h->d_rep, h->d_bch, h->nbch, PERM_STEP, h->s);
     enqueue_forces(h, b, from ^ 1, true);
 }

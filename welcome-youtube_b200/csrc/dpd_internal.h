@@ -136,6 +136,24 @@ struct EventDev {
 //   4: max bond length (float bits)   5: chain heads   8..15: type counts
 #define OBS_FIX 16777216.0
 
+#define ROW_WORDS 12  // one tile's part of a stats row: momentum x, y, kinetic, 8 type counts, chain heads
+// A stats row that the tile force kernel assembles in its epilogue, in place of
+// a separate pass over the beads: replica rep's row of this step (rep < 0:
+// none) from its tiles [tile0, tile0 + ntile), for the ring host[step % slots]
+// (the step in word 6).
+struct RowOut {
+    int32_t rep = -1, slots = 0;
+    unsigned long long *host = nullptr;
+    int32_t tile0 = 0, ntile = 0;
+};
+// what the first kernel of a step does beside the sort: collect the row of the
+// step before, clear the stirring sums (nstir of them) for this step's
+struct StepHead {
+    RowOut row;
+    long long *stir = nullptr;
+    int32_t nstir = 0;
+};
+
 struct Bufs {
     float2 *pos[2], *vh[2], *vt[2], *f[2];
     uint32_t *tg[2];
@@ -160,6 +178,8 @@ struct Bufs {
     unsigned long long *obs;    // OBS_N per replica: the running sums (zero between stats rows)
     unsigned long long *obs_out;  // OBS_N per replica: the last stats row, handed over by k_observables
     unsigned int *obs_done;     // per replica: blocks of k_observables finished
+    long long *rowpart;         // per tile of the force kernel: ROW_WORDS sums of its part of the step's stats row
+    long long *row_pending;     // step + 1 of a row whose parts are not collected yet, else 0
     unsigned long long *hist;   // pair histogram scratch
     long long *stir;            // per replica: sum of the stirring terms (fixed point) of the current positions
     uint64_t *rng;              // per replica: the serial xoshiro256** state of the catalyst chemistry (4 words)
@@ -231,12 +251,13 @@ void launch_scan_lb(const Bufs &b, int64_t C, bool step_inc, cudaStream_t s);
 // adding the block prefixes themselves); part 0..2 or all with part < 0
 bool sort_pfx_fits(int64_t C);
 void launch_sort_pfx(const Bufs &b, int64_t C, bool step_inc, const Chunk *bch, int nbch, const Chunk *cch, int ncch,
-                     int part, cudaStream_t s);
+                     int part, const StepHead &head, cudaStream_t s);
+void launch_row_collect(const Bufs &b, const RowOut &row, cudaStream_t s);
 // the sort from the bins the force kernel filled: the scan of the counts (within the one kernel up to
 // BIN_SCAN_CELLS cells) and every cell's row in slot order; other: the counts of the other parity, cleared
 bool sort_bins_one(int64_t C);
 void launch_sort_bins(const Bufs &b, uint32_t *other, int64_t C, bool step_inc, const RepDev *rep, const Chunk *cch,
-                      int ncch, int part, cudaStream_t s);
+                      int ncch, int part, const StepHead &head, cudaStream_t s);
 void launch_place(const Bufs &b, const Chunk *bch, int nbch, cudaStream_t s);
 void launch_cellfix(const Bufs &b, const Chunk *cch, int ncch, cudaStream_t s);
 void launch_permute(const Bufs &b, int cur, const RepDev *rep, const Chunk *bch, int nbch, PermuteMode mode,
@@ -267,16 +288,8 @@ void launch_unpack(const Bufs &b, int cur, int b0, int n, float *x, float *y, fl
                    cudaStream_t s);
 void launch_set_dynamics(const Bufs &b, int cur, int b0, int n, const float *vhx, const float *vhy,
                          const float *fx, const float *fy, const float *vtx, const float *vty, cudaStream_t s);
-// A stats row that the tile force kernel assembles in its epilogue, in place
-// of a separate pass over the beads: replica rep's row of this step (rep < 0:
-// none), handed over to obs_out and, when host is set, into the ring
-// host[step % slots] (the step in word 6), as k_observables does.
-struct RowOut {
-    int32_t rep, slots;
-    unsigned long long *host;
-};
 void launch_forces_tile(const Bufs &b, int cur, const RepDev *rep, const TileDesc *tiles, int ntiles, int threads,
-                        bool next_keys, cudaStream_t s, RowOut row = RowOut{-1, 0, nullptr});
+                        bool next_keys, cudaStream_t s, RowOut row = RowOut());
 int tile_setup();
 size_t tile_smem_bytes();
 size_t bulk_smem_bytes();

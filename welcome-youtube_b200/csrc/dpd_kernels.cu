@@ -17,6 +17,7 @@
 #include <algorithm>
 
 #include "dpd_chem.cuh"
+#include "dpd_row.cuh"
 
 // ---------------------------------------------------------------- keys (prime / build_cells)
 
@@ -82,9 +83,16 @@ template <bool ZERO>
 __global__ void __launch_bounds__(SCAN_TPB) k_scan1(uint32_t *__restrict__ count, int32_t *__restrict__ cstart,
                                                     int32_t *__restrict__ bsum, long long C,
                                                     long long *__restrict__ step, int step_inc,
-                                                    DevStatus *__restrict__ status, const int32_t *__restrict__ gate) {
+                                                    DevStatus *__restrict__ status, const int32_t *__restrict__ gate,
+                                                    Bufs b, StepHead head) {
     pdl_begin();
     if (gate && !*gate) return;
+    if (head.row.rep >= 0 && blockIdx.x == gridDim.x - 1) {  // the extra CTA
+        row_collect(b, head.row);
+        return;
+    }
+    if (blockIdx.x == 0)
+        for (int k = (int)threadIdx.x; k < head.nstir; k += SCAN_TPB) head.stir[k] = 0;
     const long long base = (long long)blockIdx.x * SCAN_PER_BLOCK + (long long)threadIdx.x * SCAN_PER_THREAD;
     int v[SCAN_PER_THREAD];
     int s = 0;
@@ -435,9 +443,14 @@ __device__ __forceinline__ void cellfix_range(const Bufs &b, int s, int m) {
 
 template <bool PFX>
 __global__ void __launch_bounds__(CELL_TPB) k_cellfix(Bufs b, const Chunk *__restrict__ ch,
-                                                      const int32_t *__restrict__ gate, int nb, long long C) {
+                                                      const int32_t *__restrict__ gate, int nb, long long C,
+                                                      RowOut row) {
     pdl_begin();
     if (gate && !*gate) return;
+    if (PFX && row.rep >= 0 && blockIdx.x == gridDim.x - 1) {  // the extra CTA
+        row_collect(b, row);
+        return;
+    }
     __shared__ int pfx[PFX ? PFX_MAX : 1];
     if (PFX) block_prefixes(b.bsum, nb, pfx);
     const Chunk c = ch[blockIdx.x];
@@ -498,9 +511,16 @@ __device__ __forceinline__ void bin_cell(const Bufs &b, int cell, int s, int n) 
 template <bool ONE>
 __global__ void __launch_bounds__(CELL_TPB) k_binfix(Bufs b, uint32_t *__restrict__ other,
                                                      const RepDev *__restrict__ reps, const Chunk *__restrict__ ch,
-                                                     int nb, long long C, int step_inc) {
-    const Chunk c = ch[blockIdx.x];
+                                                     int nb, long long C, int step_inc, StepHead head) {
+    const bool extra = head.row.rep >= 0 && blockIdx.x == gridDim.x - 1;  // the CTA that collects the stats row
+    const Chunk c = ch[extra ? 0 : blockIdx.x];
     pdl_begin();
+    if (extra) {
+        row_collect(b, head.row);
+        return;
+    }
+    if (blockIdx.x == 0)
+        for (int k = (int)threadIdx.x; k < head.nstir; k += CELL_TPB) head.stir[k] = 0;
     __shared__ int pfx[ONE ? 1 : PFX_MAX];
     __shared__ int red[CELL_TPB / 32];
     __shared__ int ncrowd, cursor[CELL_TPB];
@@ -1248,7 +1268,7 @@ static void scan_part(const Bufs &b, int64_t C, bool step_inc, int part, const i
     const int nb = (int)((C + SCAN_PER_BLOCK - 1) / SCAN_PER_BLOCK);
     if (part == 1)
         launch_pdl(k_scan1<true>, nb, SCAN_TPB, 0, s, b.count, b.cstart, b.bsum, (long long)C, b.step,
-                   step_inc ? 1 : 0, b.status, gate);
+                   step_inc ? 1 : 0, b.status, gate, b, StepHead());
     else launch_pdl(k_scan2, nb, SCAN_TPB, 0, s, b.cstart, b.fill, b.bsum, (long long)C, nb, gate);
 }
 
@@ -1273,35 +1293,50 @@ void launch_place(const Bufs &b, const Chunk *bch, int nbch, cudaStream_t s) {
 }
 
 void launch_cellfix(const Bufs &b, const Chunk *cch, int ncch, cudaStream_t s) {
-    launch_pdl(k_cellfix<false>, ncch, CELL_TPB, 0, s, b, cch, (const int32_t *)nullptr, 0, 0ll);
+    launch_pdl(k_cellfix<false>, ncch, CELL_TPB, 0, s, b, cch, (const int32_t *)nullptr, 0, 0ll, RowOut());
 }
 
 bool sort_pfx_fits(int64_t C) { return (C + SCAN_PER_BLOCK - 1) / SCAN_PER_BLOCK <= PFX_MAX; }
 
 void launch_sort_pfx(const Bufs &b, int64_t C, bool step_inc, const Chunk *bch, int nbch, const Chunk *cch, int ncch,
-                     int part, cudaStream_t s) {
+                     int part, const StepHead &head, cudaStream_t s) {
     const int nb = (int)((C + SCAN_PER_BLOCK - 1) / SCAN_PER_BLOCK);
     const int32_t *no = nullptr;
+    StepHead clear = head;  // the row goes to the longer fix-up kernel
+    clear.row = RowOut();
     if (part < 0 || part == 0)
         launch_pdl(k_scan1<false>, nb, SCAN_TPB, 0, s, b.count, (int32_t *)b.fill, b.bsum, (long long)C, b.step,
-                   step_inc ? 1 : 0, b.status, no);
+                   step_inc ? 1 : 0, b.status, no, b, clear);
     if (part < 0 || part == 1)
         launch_pdl(k_place<true>, (nbch + PLACE_ITEMS - 1) / PLACE_ITEMS, BEAD_TPB, 0, s, b, bch, nbch, no, nb);
-    if (part < 0 || part == 2) launch_pdl(k_cellfix<true>, ncch, CELL_TPB, 0, s, b, cch, no, nb, (long long)C);
+    if (part < 0 || part == 2)
+        launch_pdl(k_cellfix<true>, ncch + (head.row.rep >= 0 ? 1 : 0), CELL_TPB, 0, s, b, cch, no, nb, (long long)C,
+                   head.row);
 }
 
 bool sort_bins_one(int64_t C) { return C <= BIN_SCAN_CELLS; }
 
+__global__ void __launch_bounds__(256) k_row_collect(Bufs b, RowOut row) {
+    pdl_begin();
+    row_collect(b, row);
+}
+
+void launch_row_collect(const Bufs &b, const RowOut &row, cudaStream_t s) {
+    launch_pdl(k_row_collect, 1, 256, 0, s, b, row);
+}
+
 void launch_sort_bins(const Bufs &b, uint32_t *other, int64_t C, bool step_inc, const RepDev *rep, const Chunk *cch,
-                      int ncch, int part, cudaStream_t s) {
-    const int nb = (int)((C + SCAN_PER_BLOCK - 1) / SCAN_PER_BLOCK);
+                      int ncch, int part, const StepHead &head, cudaStream_t s) {
+    const int nb = (int)((C + SCAN_PER_BLOCK - 1) / SCAN_PER_BLOCK), extra = head.row.rep >= 0 ? 1 : 0;
     const bool one = sort_bins_one(C);
     if (part != 1 && !one)
-        launch_pdl(k_scan1<true>, nb, SCAN_TPB, 0, s, b.count, (int32_t *)b.fill, b.bsum, (long long)C, b.step,
-                   step_inc ? 1 : 0, b.status, (const int32_t *)nullptr);
+        launch_pdl(k_scan1<true>, nb + extra, SCAN_TPB, 0, s, b.count, (int32_t *)b.fill, b.bsum, (long long)C, b.step,
+                   step_inc ? 1 : 0, b.status, (const int32_t *)nullptr, b, head);
     if (part == 0) return;
-    if (one) launch_pdl(k_binfix<true>, ncch, CELL_TPB, 0, s, b, other, rep, cch, nb, (long long)C, step_inc ? 1 : 0);
-    else launch_pdl(k_binfix<false>, ncch, CELL_TPB, 0, s, b, other, rep, cch, nb, (long long)C, 0);
+    if (one)
+        launch_pdl(k_binfix<true>, ncch + extra, CELL_TPB, 0, s, b, other, rep, cch, nb, (long long)C, step_inc ? 1 : 0,
+                   head);
+    else launch_pdl(k_binfix<false>, ncch, CELL_TPB, 0, s, b, other, rep, cch, nb, (long long)C, 0, StepHead());
 }
 
 void launch_permute(const Bufs &b, int cur, const RepDev *rep, const Chunk *bch, int nbch, PermuteMode mode,
@@ -1328,7 +1363,7 @@ void launch_resort(const Bufs &b, int cur, const RepDev *rep, const Chunk *bch, 
     scan_part(b, C, false, 1, gate, s);
     scan_part(b, C, false, 2, gate, s);
     launch_pdl(k_place<false>, (nbch + PLACE_ITEMS - 1) / PLACE_ITEMS, BEAD_TPB, 0, s, b, bch, nbch, gate, 0);
-    launch_pdl(k_cellfix<false>, ncch, CELL_TPB, 0, s, b, cch, gate, 0, 0ll);
+    launch_pdl(k_cellfix<false>, ncch, CELL_TPB, 0, s, b, cch, gate, 0, 0ll, RowOut());
     k_permute<PERM_SORT, 1><<<nbch, BEAD_TPB, 0, s>>>(b, cur, rep, bch, nbch, gate);
     k_copy_back<<<nbch, BEAD_TPB, 0, s>>>(b, cur, bch);
 }

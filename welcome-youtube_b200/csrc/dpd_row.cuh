@@ -40,47 +40,75 @@ struct RowAcc {
     }
 };
 
-// The end of a launch that assembles a stats row: the CTA's row sums go to
-// the replica's running sums (the slots of k_observables: 0, 1 momentum,
-// 2 kinetic, 5 heads, 8 + t type counts; 4, the max bond, is max_bond_out's),
-// and the last CTA of the grid hands the row over, to obs_out and into the
-// host ring, and clears the sums for the next row, as k_observables does.
-__device__ __forceinline__ void row_handover(const Bufs &b, const RowOut &row, const long long (*rs)[3],
-                                             const uint32_t (*rc)[DPD_MAXT / 2 + 1], bool mine, int32_t *last) {
+// The end of a force kernel that assembles a stats row: the CTA's sums of its
+// tile's owned beads into the tile's place of rowpart (plain stores; mine: the
+// tile belongs to the row's replica).  The first tile marks the row as pending.
+__device__ __forceinline__ void row_partial(const Bufs &b, const RowOut &row, const long long (*rs)[3],
+                                            const uint32_t (*rc)[DPD_MAXT / 2 + 1], bool mine) {
     __syncthreads();
-    unsigned long long *obs = b.obs + (size_t)row.rep * OBS_N;
     const int tid = (int)threadIdx.x, nw = (int)blockDim.x >> 5;
-    if (mine && tid < 3 + DPD_MAXT + 1) {  // the warps' sums: 3 fixed-point sums, the type counts, the heads
-        unsigned long long v = 0;
-        int slot;
-        if (tid < 3) {
-            for (int w = 0; w < nw; w++) v += (unsigned long long)rs[w][tid];
-            slot = tid;
-        } else if (tid < 3 + DPD_MAXT) {
-            const int t = tid - 3;
-            for (int w = 0; w < nw; w++) v += (rc[w][t >> 1] >> (16 * (t & 1))) & 0xFFFFu;
-            slot = 8 + t;
-        } else {
-            for (int w = 0; w < nw; w++) v += rc[w][DPD_MAXT / 2];
-            slot = 5;
+    if (!mine || tid > ROW_WORDS) return;
+    if (tid == ROW_WORDS) {
+        if ((int)blockIdx.x == row.tile0) *b.row_pending = *b.step + 1;
+        return;
+    }
+    // the warps' sums: 3 fixed-point sums, the type counts, the heads
+    long long v = 0;
+    if (tid < 3) {
+        for (int w = 0; w < nw; w++) v += rs[w][tid];
+    } else if (tid < 3 + DPD_MAXT) {
+        const int t = tid - 3;
+        for (int w = 0; w < nw; w++) v += (rc[w][t >> 1] >> (16 * (t & 1))) & 0xFFFFu;
+    } else {
+        for (int w = 0; w < nw; w++) v += rc[w][DPD_MAXT / 2];
+    }
+    b.rowpart[(size_t)((int)blockIdx.x - row.tile0) * ROW_WORDS + tid] = v;
+}
+
+// The pending row of the last force kernel, by one CTA of 256 threads: the
+// tiles' sums added up, the row in k_observables' slots (0, 1 momentum, 2
+// kinetic, 4 max bond, 5 heads, 8 + t type counts) into obs_out and the host
+// ring.  It rides along as an extra CTA of a kernel of the next step's sort
+// (launch_sort_bins, launch_sort_pfx), or runs alone at the end of a call.  As
+// a hand-over by the last CTA of the force kernel (a fence and a counter in
+// every CTA, then a dependent pass) a step of 4,096 beads took 17.1 us, now
+// 15.5; the 31,029-bead one, whose stirring sums are now cleared on the way
+// too, 28.5 and 20.9.
+__device__ __forceinline__ void row_collect(const Bufs &b, const RowOut &row) {
+    __shared__ long long part[8][ROW_WORDS];
+    const long long pending = *b.row_pending;
+    if (pending == 0) return;
+    const int tid = (int)threadIdx.x, w = tid >> 5;
+    // a thread takes whole tiles, 16 bytes a load, all of a tile's in flight
+    long long v[ROW_WORDS];
+#pragma unroll
+    for (int k = 0; k < ROW_WORDS; k++) v[k] = 0;
+    for (int t = tid; t < row.ntile; t += 256) {
+        const longlong2 *q = reinterpret_cast<const longlong2 *>(b.rowpart + (size_t)t * ROW_WORDS);
+#pragma unroll
+        for (int k = 0; k < ROW_WORDS / 2; k++) {
+            const longlong2 x = q[k];
+            v[2 * k] += x.x;
+            v[2 * k + 1] += x.y;
         }
-        if (v != 0) atomicAdd(obs + slot, v);
     }
-    __threadfence();
+#pragma unroll
+    for (int k = 0; k < ROW_WORDS; k++) {
+        const long long t = warp_sum_ll(v[k]);
+        if (lane_id() == 0) part[w][k] = t;
+    }
     __syncthreads();
-    if (tid == 0) *last = atomicAdd(b.obs_done + row.rep, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!*last) return;
-    __threadfence();
-    unsigned long long *out = row.host;
-    const long long step = *b.step;
-    if (out && row.slots > 0) out += (size_t)(step % row.slots) * OBS_N;
     if (tid < OBS_N) {
-        const unsigned long long v = atomicExch(obs + tid, 0ull);
+        const int k = tid < 3 ? tid : (tid >= 8 ? tid - 5 : (tid == 5 ? ROW_WORDS - 1 : -1));
+        unsigned long long v = 0;
+        if (k >= 0)
+            for (int q = 0; q < 8; q++) v += (unsigned long long)part[q][k];
+        if (tid == 4) v = atomicExch(b.obs + (size_t)row.rep * OBS_N + 4, 0ull);
         b.obs_out[(size_t)row.rep * OBS_N + tid] = v;
-        if (out) out[tid] = (row.slots > 0 && tid == 6) ? (unsigned long long)step : v;
+        const long long step = pending - 1;
+        if (row.host) row.host[(size_t)(step % row.slots) * OBS_N + tid] = tid == 6 ? (unsigned long long)step : v;
     }
-    if (tid == 0) b.obs_done[row.rep] = 0u;
+    if (tid == 0) *b.row_pending = 0;
 }
 
 // the running max bond of a tile's replica (one atomic per warp)

@@ -24,8 +24,8 @@
 // Epilogue per owned bead: harmonic bonds to prev/next, the force written to
 // HBM, and the cell of the next position with its count (the first half of
 // the next step's sort).  When the step's stats row is wanted (the stats ring),
-// the epilogue also sums the row's terms of the beads it holds, and the last
-// CTA hands the row over (RowAcc, row_handover).  A tile whose beads do not
+// the epilogue also sums the row's terms of the beads it holds and leaves the
+// tile's sums for the next kernel to collect (RowAcc, row_partial).  A tile whose beads do not
 // fit in shared memory computes its owned beads straight from HBM instead
 // (bead_pairs_direct).
 #include <algorithm>
@@ -71,7 +71,6 @@ struct TileSmemT {
     int32_t next_chunk;           // source chunks are handed to warps as they finish their last one
     long long rsum[TPB / 32][3];  // per warp, the stats-row sums of the tile's owned beads (RowAcc)
     uint32_t rcnt[TPB / 32][DPD_MAXT / 2 + 1];
-    int32_t rlast;                // this CTA hands the row over
 };
 
 #define TILE_PAD 0xFFFFu          // lxy of a slot that holds no bead of the tile (bulk-copy padding)
@@ -550,7 +549,7 @@ __global__ void __launch_bounds__(TPB, TILE_MINB * 256 / TPB) k_forces_tile(Bufs
         tile_epilogue<NEXTKEY>(b, cur, R, td, S, mb, rs, rc);
     }
     max_bond_out(b, td.rep, mb);
-    if (NEXTKEY && row.rep >= 0) row_handover(b, row, SS.rsum, SS.rcnt, want_row, &SS.rlast);
+    if (NEXTKEY && row.rep >= 0) row_partial(b, row, SS.rsum, SS.rcnt, want_row);
 }
 
 // ---------------------------------------------------------------- the bulk-staged kernel
