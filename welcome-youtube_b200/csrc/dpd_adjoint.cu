@@ -169,7 +169,7 @@ __device__ __forceinline__ void adj_update(const AdjUpdate &u, const RepDev &R, 
 // What bounds it: instruction issue (about 180 warp instructions a bead at
 // density 4, 2.2 of 4 a cycle: half of them the 12.6 evaluations, 40 of whose
 // 140 instructions are the noise) and the fullest list of a warp, 1.6 times the
-// mean.  24 boxes of 65,536 beads: 434 us, against 939 (and 82 for the update)
+// mean.  24 boxes of 65,536 beads: about 420 us, against 939 (and 82 for the update)
 // with a thread per bead and an FP64 shared atomic per pair; one box: 34
 // against 68, of 16,384: 14 against 60, of 4,096: 10 against 61.  Tried: one
 // queue of pairs per warp evaluated by full rounds, its terms summed through
@@ -809,10 +809,15 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
         cudaMemsetAsync(gsum, 0, (size_t)nrep * sizeof(double), s);
         k_gsum<<<nbch, BEAD_TPB, 0, s>>>(rep, bch, g, gsum);
     }
-    // lanes per bead: eight or four while the tasks fit the GPU at once (a small box is latency: 4,096 beads took
-    // 10.8 us with eight against 13.3 with four and 17.3 with two; 16,384 beads 14.1 with four, 17.4 with two), else two,
-    // whose lanes wait less for the fullest list (24 boxes of 65,536: 374 us, 455 with four, 585 with eight, before the
-    // sums were ordered); then three CTAs an SM at 80 registers, two otherwise
+    // Lanes per bead and CTAs an SM: as many lanes as keep all tasks on the GPU at once (a small box is latency), then
+    // few, whose lanes wait less for the fullest list.  us a launch with (lanes, CTAs an SM), density 4:
+    //   beads      (8, 2)  (4, 2)  (4, 3)  (2, 2)  (2, 4)
+    //   4,096         9.9    12.8    13.2    19.2    21.2
+    //   16,384       15.2    14.2    14.6    19.7    21.8
+    //   25,600       20.3    21.6    16.8    22.6    25.0
+    //   36,864       24.3    21.1    25.4    21.5    23.7
+    //   131,044      66.7    54.2    52.3    54.6    53.4
+    //   1,048,576   491     385     341     347     311
     const bool update = up && !mol;  // the branched shapes add their share first
     const AdjUpdate none{};
     auto go = [&](auto kern, int lpb, int per_sm) {
@@ -822,7 +827,9 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
     };
     if (nbch * 8 <= 2 * 148) go(update ? k_force_vjp<8, 2, true> : k_force_vjp<8, 2, false>, 8, 2);
     else if (nbch * 4 <= 2 * 148) go(update ? k_force_vjp<4, 2, true> : k_force_vjp<4, 2, false>, 4, 2);
-    else go(update ? k_force_vjp<2, 3, true> : k_force_vjp<2, 3, false>, 2, 3);
+    else if (nbch * 4 > 3 * 148 && nbch * 2 <= 2 * 148) go(update ? k_force_vjp<2, 2, true> : k_force_vjp<2, 2, false>, 2, 2);
+    else if (nbch <= 600) go(update ? k_force_vjp<4, 3, true> : k_force_vjp<4, 3, false>, 4, 3);
+    else go(update ? k_force_vjp<2, 4, true> : k_force_vjp<2, 4, false>, 2, 4);
     if (mol) {
         k_mol_vjp<<<nbch, BEAD_TPB, 0, s>>>(sv, rep, bch, mol, g, xbar, grad);
         if (up) k_adj_update<<<nbch, BEAD_TPB, 0, s>>>(rep, bch, xbar, vbar, *up);

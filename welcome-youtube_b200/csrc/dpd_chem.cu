@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(BEAD_TPB) k_chem_scan(Bufs b, int cur, const R
 __global__ void __launch_bounds__(BEAD_TPB) k_chem_grow(Bufs b, int cur, const RepDev *__restrict__ reps) {
     pdl_begin();
     const int n = (int)b.status->n_grow;
+    if (n == 0) return;  // (the same in every CTA: the counter of last_cta stays at rest)
     const int nw = (int)(gridDim.x * blockDim.x) >> 5;
     for (int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < n; k += nw)
         chem_grow_req_one(b, cur, reps, k, (int)lane_id());
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(BEAD_TPB) k_chem_grow(Bufs b, int cur, const R
 __global__ void __launch_bounds__(BEAD_TPB) k_chem_bond(Bufs b, int cur, const RepDev *__restrict__ reps) {
     pdl_begin();
     const int n = (int)b.status->n_bond;
+    if (n == 0) return;
     const int nw = (int)(gridDim.x * blockDim.x) >> 5;
     for (int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < n; k += nw)
         chem_bond_req_one(b, cur, reps, k, (int)lane_id());
