@@ -44,6 +44,91 @@ __device__ __forceinline__ void uf_union(int *parent, int a, int b, DevStatus *s
 
 __device__ __forceinline__ double min_image(double d, double L) { return d - L * rint(d / L); }
 
+__device__ __forceinline__ double exact_r2(float2 pi, float2 pj, double L) {
+    const double dx = min_image((double)pj.x - (double)pi.x, L), dy = min_image((double)pj.y - (double)pi.y, L);
+    return dx * dx + dy * dy;
+}
+
+// Contact searches.  One bead in five or fewer is of the type, so a CTA lists
+// its beads of the type in shared memory and NEAR_LANES lanes share each: they
+// take the slots of its 3 x 3 cells in turn (cells are column-major: three
+// contiguous ranges, two each where the rows wrap).  Squared distances are
+// FP32; one within NEAR_EPS of a threshold is taken again in FP64 with the
+// reference's minimum image (the FP32 error is below 1e-4: half an ulp of the
+// largest box on each coordinate, times two), so every comparison is the FP64
+// one.  786,432 beads: k_uf_link 115 us against 168, k_agg_link 105 against 128,
+// with a thread per bead and two FP64 divisions per candidate (what is left is the
+// union-find's own chains).
+constexpr int NEAR_LANES = 8;
+constexpr float NEAR_EPS = 4e-4f;
+
+// calls near(j, squared distance) for the slots j != d of bead d's cells within
+// the FP32 reach of lim, from this lane's share of them; same as exact_r2 where
+// it could matter for lim or lim2
+template <class F>
+__device__ __forceinline__ void each_near(const float2 *__restrict__ pos, const RepDev &R,
+                                          const int32_t *__restrict__ cs, int d, int sub, double lim, double lim2,
+                                          F near) {
+    const float2 pi = pos[d];
+    const float L = R.L, h = R.halfL, f1 = (float)lim, f2 = (float)lim2;
+    const int ncx = R.ncx, ncy = R.ncy;
+    int cx, cy;
+    cell_xy(R, pi.x, pi.y, cx, cy);
+    for (int ox = -1; ox <= 1; ox++) {
+        const int nx = cx + ox < 0 ? ncx - 1 : (cx + ox >= ncx ? 0 : cx + ox);
+        const int32_t *col = cs + nx * ncy;
+        for (int seg = -1; seg <= 1; seg++) {  // the rows below 0, inside, and past the top
+            const int r0 = max(cy - 1, seg * ncy), r1 = min(cy + 1, seg * ncy + ncy - 1);
+            if (r0 > r1) continue;
+            const int je = col[r1 - seg * ncy + 1];
+            for (int j = col[r0 - seg * ncy] + sub; j < je; j += NEAR_LANES) {
+                if (j == d) continue;
+                const float2 pj = pos[j];
+                const float dx = minimg(pj.x - pi.x, L, h), dy = minimg(pj.y - pi.y, L, h);
+                const float q = dx * dx + dy * dy;
+                if (q > f1 + NEAR_EPS) continue;
+                double r2 = (double)q;
+                if (fabsf(q - f1) <= NEAR_EPS || fabsf(q - f2) <= NEAR_EPS) r2 = exact_r2(pi, pj, (double)L);
+                if (r2 <= lim) near(j, r2);
+            }
+        }
+    }
+}
+
+// the CTA's beads d for which mine is true, listed in shared memory; returns their number
+__device__ __forceinline__ int list_beads(bool mine, int d, int *list, int *n) {
+    if (threadIdx.x == 0) *n = 0;
+    __syncthreads();
+    if (mine) list[atomicAdd(n, 1)] = d;
+    __syncthreads();
+    return *n;
+}
+
+// sums over the CTA of up to five values and a maximum, one atomic each
+__device__ __forceinline__ void cta_sums(const long long *v, int nv, unsigned mx, unsigned long long *const *dst,
+                                         unsigned long long *dst_max) {
+    __shared__ long long red[BEAD_TPB / 32][6];
+    const int w = (int)threadIdx.x >> 5;
+    for (int k = 0; k < nv; k++) {
+        const long long t = warp_sum_ll(v[k]);
+        if (lane_id() == 0) red[w][k] = t;
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane_id() == 0) red[w][5] = mx;
+    __syncthreads();
+    const int k = (int)threadIdx.x;
+    if (k < nv) {
+        long long t = 0;
+        for (int q = 0; q < BEAD_TPB / 32; q++) t += red[q][k];
+        if (t) atomicAdd(dst[k], (unsigned long long)t);
+    }
+    if (k == 5 && dst_max) {
+        long long t = 0;
+        for (int q = 0; q < BEAD_TPB / 32; q++) t = max(t, red[q][5]);
+        if (t) atomicMax(dst_max, (unsigned long long)t);
+    }
+}
+
 }  // namespace
 
 // parent[i] = i for the beads of type t of the replica, -1 for the others
@@ -65,41 +150,25 @@ __global__ void __launch_bounds__(BEAD_TPB) k_uf_link(Bufs b, int cur, const Rep
                                                       int *__restrict__ parent, unsigned long long *__restrict__ acc) {
     const Chunk c = ch[blockIdx.x];
     if (c.rep != rep_index) return;
+    __shared__ int list[BEAD_TPB], nlist;
     const RepDev &R = reps[c.rep];
-    const int d = c.begin + (int)threadIdx.x;
-    unsigned long long n_all = 0, n_same = 0;
-    if (d < c.end && parent[d] >= 0) {
-        const float2 *__restrict__ pos = b.pos[cur];
-        const float2 pi = pos[d];
-        const double L = (double)R.L, r2c = rcut * rcut;
-        const int32_t *cs = b.cstart + R.c0;
-        int cx, cy;
-        cell_xy(R, pi.x, pi.y, cx, cy);
-        const int rx = R.ncx >= 3 ? 1 : 0, ry = R.ncy >= 3 ? 1 : 0;
-        for (int ox = -rx; ox <= rx; ox++)
-            for (int oy = -ry; oy <= ry; oy++) {
-                const int nx = (cx + ox + R.ncx) % R.ncx, ny = (cy + oy + R.ncy) % R.ncy;
-                const int cc = nx * R.ncy + ny;
-                for (int j = cs[cc]; j < cs[cc + 1]; j++) {
-                    if (j == d) continue;
-                    const float2 pj = pos[j];
-                    const double dx = min_image((double)pj.x - (double)pi.x, L);
-                    const double dy = min_image((double)pj.y - (double)pi.y, L);
-                    const double r2 = dx * dx + dy * dy;
-                    if (r2 > 1.0) continue;
-                    const bool same = (int)(b.tg[cur][j] >> TYPE_SHIFT) == t;
-                    n_all++;
-                    n_same += same;
-                    if (same && j > d && r2 <= r2c) uf_union(parent, d, j, b.status);
-                }
-            }
+    const int d0 = c.begin + (int)threadIdx.x;
+    const int n = list_beads(d0 < c.end && parent[d0] >= 0, d0, list, &nlist);
+    const uint32_t *__restrict__ tg = b.tg[cur];
+    const int sub = (int)threadIdx.x % NEAR_LANES;
+    const double r2c = rcut * rcut;
+    long long cnt[2] = {0, 0};
+    for (int k = (int)threadIdx.x / NEAR_LANES; k < n; k += BEAD_TPB / NEAR_LANES) {
+        const int d = list[k];
+        each_near(b.pos[cur], R, b.cstart + R.c0, d, sub, 1.0, r2c, [&](int j, double r2) {
+            const bool same = (int)(tg[j] >> TYPE_SHIFT) == t;
+            cnt[0]++;
+            cnt[1] += same;
+            if (same && j > d && r2 <= r2c) uf_union(parent, d, j, b.status);
+        });
     }
-    n_all = warp_sum_ll((long long)n_all);
-    n_same = warp_sum_ll((long long)n_same);
-    if (lane_id() == 0 && n_all) {
-        atomicAdd(acc + 0, n_all);
-        atomicAdd(acc + 1, n_same);
-    }
+    unsigned long long *const dst[2] = {acc + 0, acc + 1};
+    cta_sums(cnt, 2, 0u, dst, nullptr);
 }
 
 // each bead's root, and the bead counted in its cluster's size
@@ -129,16 +198,9 @@ __global__ void __launch_bounds__(BEAD_TPB) k_uf_stats(const Chunk *__restrict__
         nb = s;
         mx = (unsigned)s;
     }
-    nc = warp_sum_ll(nc);
-    sq = warp_sum_ll(sq);
-    nb = warp_sum_ll(nb);
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (lane_id() == 0 && nc) {
-        atomicAdd(acc + 2, (unsigned long long)nc);
-        atomicAdd(acc + 3, (unsigned long long)sq);
-        atomicAdd(acc + 4, (unsigned long long)nb);
-        atomicMax(acc + 5, (unsigned long long)mx);
-    }
+    const long long v[3] = {nc, sq, nb};
+    unsigned long long *const dst[3] = {acc + 2, acc + 3, acc + 4};
+    cta_sums(v, 3, mx, dst, acc + 5);
 }
 
 // ---------------------------------------------------------------- membrane aggregates
@@ -168,30 +230,24 @@ __global__ void __launch_bounds__(BEAD_TPB) k_agg_link(Bufs b, int cur, const Re
                                                        int *__restrict__ parent) {
     const Chunk c = ch[blockIdx.x];
     if (c.rep != rep_index) return;
+    __shared__ int list[BEAD_TPB], nlist;
     const RepDev &R = reps[c.rep];
-    const int d = c.begin + (int)threadIdx.x;
-    if (d >= c.end || parent[d] < 0) return;
-    const int nx = b.link[cur][d].y;
-    if (nx >= 0 && parent[nx] >= 0) uf_union(parent, d, nx, b.status);
-    if ((int)(b.tg[cur][d] >> TYPE_SHIFT) != 2) return;
-    const float2 *__restrict__ pos = b.pos[cur];
-    const float2 pi = pos[d];
-    const double L = (double)R.L, r2c = r_tail * r_tail;
-    const int32_t *cs = b.cstart + R.c0;
-    int cx, cy;
-    cell_xy(R, pi.x, pi.y, cx, cy);
-    for (int ox = -1; ox <= 1; ox++)
-        for (int oy = -1; oy <= 1; oy++) {
-            const int gx = (cx + ox + R.ncx) % R.ncx, gy = (cy + oy + R.ncy) % R.ncy;
-            const int cc = gx * R.ncy + gy;
-            for (int j = cs[cc]; j < cs[cc + 1]; j++) {
-                if (j <= d || (int)(b.tg[cur][j] >> TYPE_SHIFT) != 2) continue;
-                const float2 pj = pos[j];
-                const double dx = min_image((double)pj.x - (double)pi.x, L);
-                const double dy = min_image((double)pj.y - (double)pi.y, L);
-                if (dx * dx + dy * dy <= r2c) uf_union(parent, d, j, b.status);
-            }
-        }
+    const uint32_t *__restrict__ tg = b.tg[cur];
+    const int d0 = c.begin + (int)threadIdx.x;
+    const bool lipid = d0 < c.end && parent[d0] >= 0;
+    if (lipid) {
+        const int nx = b.link[cur][d0].y;
+        if (nx >= 0 && parent[nx] >= 0) uf_union(parent, d0, nx, b.status);
+    }
+    const int n = list_beads(lipid && (int)(tg[d0] >> TYPE_SHIFT) == 2, d0, list, &nlist);
+    const int sub = (int)threadIdx.x % NEAR_LANES;
+    const double r2c = r_tail * r_tail;
+    for (int k = (int)threadIdx.x / NEAR_LANES; k < n; k += BEAD_TPB / NEAR_LANES) {
+        const int d = list[k];
+        each_near(b.pos[cur], R, b.cstart + R.c0, d, sub, r2c, r2c, [&](int j, double) {
+            if (j > d && (int)(tg[j] >> TYPE_SHIFT) == 2) uf_union(parent, d, j, b.status);
+        });
+    }
 }
 
 // per lipid bead: its root; molecules (beads without prev) counted per aggregate;
@@ -233,18 +289,9 @@ __global__ void __launch_bounds__(BEAD_TPB) k_agg_stats(Bufs b, int cur, const C
             mx = (unsigned)s;
         }
     }
-    na = warp_sum_ll(na);
-    nm = warp_sum_ll(nm);
-    nmol = warp_sum_ll(nmol);
-    small = warp_sum_ll(small);
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (lane_id() == 0 && na) {
-        atomicAdd(acc + 2, (unsigned long long)na);
-        atomicAdd(acc + 3, (unsigned long long)nm);
-        atomicAdd(acc + 4, (unsigned long long)nmol);
-        atomicMax(acc + 5, (unsigned long long)mx);
-        atomicAdd(acc + 6, (unsigned long long)small);
-    }
+    const long long v[4] = {na, nm, nmol, small};
+    unsigned long long *const dst[4] = {acc + 2, acc + 3, acc + 4, acc + 6};
+    cta_sums(v, 4, mx, dst, acc + 5);
 }
 
 void launch_aggregates(const Bufs &b, int cur, const RepDev *rep, const Chunk *bch, int nbch, int rep_index, int n,

@@ -1080,7 +1080,10 @@ __device__ __noinline__ int pair_hist_bin(float2 pi, float2 pj, double L, double
 // 30 bins to 3.0, all beads and the tails alone: 0.17 ms a call on average,
 // against 5.77 ms with FP64 hypot and division per pair and one global atomic
 // per pair.
-template <bool LANES>
+// GROUP lanes share a bead: one for all beads; for beads of two types, which the
+// CTA lists first, eight, so that lanes are not idle for the other types' beads
+// (the tails of the same configuration: 78 us against 172).
+template <bool LANES, int GROUP>
 __global__ void __launch_bounds__(BEAD_TPB) k_pair_hist(Bufs b, int cur, const RepDev *__restrict__ reps,
                                                         const Chunk *__restrict__ ch, int rep_index, int ta, int tb,
                                                         double rmax, int nbin) {
@@ -1089,7 +1092,7 @@ __global__ void __launch_bounds__(BEAD_TPB) k_pair_hist(Bufs b, int cur, const R
     for (int k = (int)threadIdx.x; k < nbin * ncopy; k += (int)blockDim.x) hsh[k] = 0u;
     __syncthreads();
     const RepDev &R = reps[rep_index];
-    unsigned int *mine = hsh + (LANES ? lane_id() : 0u);
+    unsigned int *mine_bins = hsh + (LANES ? lane_id() : 0u);
     const float2 *__restrict__ pos = b.pos[cur];
     const uint32_t *__restrict__ tg = b.tg[cur];
     const int ncx = R.ncx, ncy = R.ncy;
@@ -1099,12 +1102,10 @@ __global__ void __launch_bounds__(BEAD_TPB) k_pair_hist(Bufs b, int cur, const R
     const double L = (double)R.L;
     const float norm = (float)((double)nbin / rmax), tol = 1.5e-6f * (norm + (float)nbin);
     const float rm = (float)rmax + 4e-6f, r2max = rm * rm, far2 = 0.2499f * R.L * R.L;
-    for (int k = (int)blockIdx.x; k < R.nch; k += (int)gridDim.x) {
-        const Chunk c = ch[R.ch0 + k];
-        const int d = c.begin + (int)threadIdx.x;
-        if (d >= c.end) continue;
+    __shared__ int list[GROUP > 1 ? BEAD_TPB : 1], nlist;
+    const int sub = (int)threadIdx.x % GROUP;
+    auto count = [&](int d) {  // this lane's share of bead d's pairs
         const int ti = (int)(tg[d] >> TYPE_SHIFT);
-        if (ta >= 0 && ti != ta && ti != tb) continue;
         const int want = ti == ta ? tb : ta, also = ti == tb ? ta : want;  // partner types (ta < 0: any)
         const float2 pi = pos[d];
         int cx, cy;
@@ -1123,8 +1124,8 @@ __global__ void __launch_bounds__(BEAD_TPB) k_pair_hist(Bufs b, int cur, const R
                 const int js = max(col[r0], d + 1), je = col[r1 + 1];
                 const double py = (double)pi.y - seg * L;
                 const float pyh = (float)py, pyl = (float)(py - (double)pyh);
-                for (int j = js; j < je; j++) {
-                    if (ta >= 0) {
+                for (int j = js + sub; j < je; j += GROUP) {
+                    if (GROUP > 1) {
                         const int tj = (int)(tg[j] >> TYPE_SHIFT);
                         if (tj != want && tj != also) continue;
                     }
@@ -1136,10 +1137,25 @@ __global__ void __launch_bounds__(BEAD_TPB) k_pair_hist(Bufs b, int cur, const R
                     int bin = (int)q;
                     const float fr = q - (float)bin;
                     if (!(fr >= tol && fr <= 1.0f - tol && r2 < far2)) bin = pair_hist_bin(pi, pj, L, rmax, nbin);
-                    if (bin >= 0 && bin < nbin) atomicAdd(mine + bin * ncopy, 1u);
+                    if (bin >= 0 && bin < nbin) atomicAdd(mine_bins + bin * ncopy, 1u);
                 }
             }
         }
+    };
+    for (int k = (int)blockIdx.x; k < R.nch; k += (int)gridDim.x) {
+        const Chunk c = ch[R.ch0 + k];
+        const int d0 = c.begin + (int)threadIdx.x;
+        if (GROUP == 1) {
+            if (d0 < c.end) count(d0);
+            continue;
+        }
+        const int t = d0 < c.end ? (int)(tg[d0] >> TYPE_SHIFT) : -1;
+        __syncthreads();  // (the list of the chunk before is done with)
+        if (threadIdx.x == 0) nlist = 0;
+        __syncthreads();
+        if (t >= 0 && (t == ta || t == tb)) list[atomicAdd(&nlist, 1)] = d0;
+        __syncthreads();
+        for (int it = (int)threadIdx.x / GROUP; it < nlist; it += BEAD_TPB / GROUP) count(list[it]);
     }
     __syncthreads();
     for (int k = (int)threadIdx.x; k < nbin; k += (int)blockDim.x) {
@@ -1420,10 +1436,17 @@ void launch_pair_hist(const Bufs &b, int cur, const RepDev *rep, const Chunk *bc
                       int tb, double rmax, int nbin, cudaStream_t s) {
     // a column of counts per lane while the CTAs of an SM keep them in shared memory (256 bins: 32 KB a CTA)
     const int grid = std::max(1, std::min(nch, HIST_BLOCKS_PER_SM * 148));
-    if (nbin <= HIST_LANE_BINS)
-        k_pair_hist<true><<<grid, BEAD_TPB, (size_t)nbin * 32 * 4, s>>>(b, cur, rep, bch, rep_index, ta, tb, rmax, nbin);
-    else
-        k_pair_hist<false><<<grid, BEAD_TPB, (size_t)nbin * 4, s>>>(b, cur, rep, bch, rep_index, ta, tb, rmax, nbin);
+    const size_t lanes = (size_t)nbin * 32 * 4, one = (size_t)nbin * 4;
+    if (ta < 0) {
+        if (nbin <= HIST_LANE_BINS)
+            k_pair_hist<true, 1><<<grid, BEAD_TPB, lanes, s>>>(b, cur, rep, bch, rep_index, ta, tb, rmax, nbin);
+        else
+            k_pair_hist<false, 1><<<grid, BEAD_TPB, one, s>>>(b, cur, rep, bch, rep_index, ta, tb, rmax, nbin);
+    } else if (nbin <= HIST_LANE_BINS) {
+        k_pair_hist<true, 8><<<grid, BEAD_TPB, lanes, s>>>(b, cur, rep, bch, rep_index, ta, tb, rmax, nbin);
+    } else {
+        k_pair_hist<false, 8><<<grid, BEAD_TPB, one, s>>>(b, cur, rep, bch, rep_index, ta, tb, rmax, nbin);
+    }
 }
 
 void launch_pack(const Bufs &b, int cur, int b0, int n, float L, const float *x, const float *y, const float *vx,
