@@ -53,14 +53,16 @@ __device__ __forceinline__ double exact_r2(float2 pi, float2 pj, double L) {
 // its beads of the type in shared memory and NEAR_LANES lanes share each: they
 // take the slots of its 3 x 3 cells in turn (cells are column-major: three
 // contiguous ranges, two each where the rows wrap).  Squared distances are
-// FP32; one within NEAR_EPS of a threshold is taken again in FP64 with the
-// reference's minimum image (the FP32 error is below 1e-4: half an ulp of the
-// largest box on each coordinate, times two), so every comparison is the FP64
-// one.  786,432 beads: k_uf_link 115 us against 168, k_agg_link 105 against 128,
+// FP32; one within near_eps of a threshold is taken again in FP64 with the
+// reference's minimum image, so every comparison is the FP64 one.  786,432 beads: k_uf_link 115 us against 168, k_agg_link 105 against 128,
 // with a thread per bead and two FP64 divisions per candidate (what is left is the
 // union-find's own chains).
 constexpr int NEAR_LANES = 8;
-constexpr float NEAR_EPS = 4e-4f;
+
+// Bound of the FP32 error of a squared distance up to about 1: a coordinate
+// difference across the box edge is off by half an ulp of L at most (6e-8 L),
+// others are exact, so 2 sqrt(2) of that, and a few roundings near 1.
+__device__ __forceinline__ float near_eps(float L) { return 2e-6f + 2e-7f * L; }
 
 // calls near(j, squared distance) for the slots j != d of bead d's cells within
 // the FP32 reach of lim, from this lane's share of them; same as exact_r2 where
@@ -70,7 +72,7 @@ __device__ __forceinline__ void each_near(const float2 *__restrict__ pos, const 
                                           const int32_t *__restrict__ cs, int d, int sub, double lim, double lim2,
                                           F near) {
     const float2 pi = pos[d];
-    const float L = R.L, h = R.halfL, f1 = (float)lim, f2 = (float)lim2;
+    const float L = R.L, h = R.halfL, f1 = (float)lim, f2 = (float)lim2, eps = near_eps(L);
     const int ncx = R.ncx, ncy = R.ncy;
     int cx, cy;
     cell_xy(R, pi.x, pi.y, cx, cy);
@@ -86,9 +88,9 @@ __device__ __forceinline__ void each_near(const float2 *__restrict__ pos, const 
                 const float2 pj = pos[j];
                 const float dx = minimg(pj.x - pi.x, L, h), dy = minimg(pj.y - pi.y, L, h);
                 const float q = dx * dx + dy * dy;
-                if (q > f1 + NEAR_EPS) continue;
+                if (q > f1 + eps) continue;
                 double r2 = (double)q;
-                if (fabsf(q - f1) <= NEAR_EPS || fabsf(q - f2) <= NEAR_EPS) r2 = exact_r2(pi, pj, (double)L);
+                if (fabsf(q - f1) <= eps || fabsf(q - f2) <= eps) r2 = exact_r2(pi, pj, (double)L);
                 if (r2 <= lim) near(j, r2);
             }
         }
