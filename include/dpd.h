@@ -455,12 +455,21 @@ typedef struct {
  * amplitude following the temperature cycle. */
 DPD_API int dpd_window_loss(dpd_handle *h, int64_t nsteps, const dpd_rdf_spec *spec, const double *target,
                             double *loss, double *rdf_out);
-/* The same window, then its adjoint: the pair noise is replayed from its key,
- * the state is checkpointed every ckpt_every steps and each segment is
- * recomputed in reverse.  grad: nrep x DPD_NGRAD.  The handle ends at the end
- * of the window, as after dpd_window_loss. */
+/* The same window, then its adjoint: the pair noise is replayed from its key.
+ * The configurations of the last steps are kept, the ones before them stepped
+ * again from checkpoints: at most the memory of a checkpoint every ckpt_every
+ * steps and ckpt_every configurations (about 44 and 33 bytes a bead each), or,
+ * where that is more, a thirty-second of the device's (see
+ * dpd_set_window_memory); the results do not depend on it.  The storage stays
+ * with the handle.  grad: nrep x DPD_NGRAD.  The handle ends at the end of the
+ * window, as after dpd_window_loss. */
 DPD_API int dpd_window_adjoint(dpd_handle *h, int64_t nsteps, int32_t ckpt_every, const dpd_rdf_spec *spec,
                                const double *target, double *loss, double *grad, double *rdf_out);
+/* The memory the windows of this handle may take for checkpoints and
+ * configurations, in bytes, where that is more than ckpt_every asks for (0:
+ * never more than that; negative: the default, a thirty-second of the device's
+ * memory while four times that is free). */
+DPD_API int dpd_set_window_memory(dpd_handle *h, int64_t bytes);
 /* dpd_window_adjoint plus the cotangents of the window's start state: the
  * loss's gradient with respect to the positions (xbar), the stored half-step
  * velocities (vhbar) and the predicted velocities (vtbar) the window starts

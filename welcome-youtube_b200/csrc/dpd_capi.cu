@@ -1,6 +1,7 @@
 // dpd_capi.cu -- the C ABI of libdpd.so (include/dpd.h): handles, device
 // memory, CUDA graphs of the step, state in/out, error reporting.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -109,6 +110,7 @@ struct dpd_handle {
     // recomputed segment, adjoint arrays in gid order)
     std::vector<void *> adj_allocs;
     int adj_nck = 0, adj_nseg = 0, adj_nbin = 0;  // capacity of adj (0: none yet)
+    int64_t window_mem = -1;    // dpd_set_window_memory (-1: the default rule)
     AdjBufs adj;
     // staging for state in/out
     char *stage = nullptr;
@@ -1648,26 +1650,72 @@ static void enqueue_seg_step(dpd_handle *h, AdjBufs &A, int sg, int s, int par0)
 }
 
 // A differentiated window, enqueued: its steps with the loss's histogram, then
-// (after the loss's weights are on the device) its reverse pass.
+// (after the loss's weights are on the device) its reverse pass over the steps
+// after `stop`, in nseg segments of `len` steps (the first may be shorter).
 struct Window {
     int64_t nsteps;
-    int ckpt, nseg;
+    int len, nseg;     // nseg 0: no reverse pass
     const dpd_rdf_spec *spec;
     int64_t step0;     // the step the window starts from, or
     const FitDev *fd;  // where the device keeps it (a captured iteration), else null
-    bool backward;
     int64_t first_loss() const { return nsteps - spec->last_steps + 1; }  // window steps whose state enters the loss
+    // the step the horizon leaves: nothing before it is differentiated
+    int64_t stop() const { return spec->horizon > 0 ? std::max<int64_t>(0, first_loss() - 1 - spec->horizon) : 0; }
+    int64_t start(int sg) const { return std::max(stop(), nsteps - (int64_t)(nseg - sg) * len); }
 };
+
+// The segments of the reverse pass and the storage for them.  The forward pass
+// keeps the configurations of the last segment; the others are stepped again
+// from their checkpoints.  So the longest segments that fit are taken, all
+// steps in one where that fits, in the larger of
+//   what the caller's interval asks for: a checkpoint every ckpt steps of the
+//   window and the configurations of ckpt steps;
+//   a thirty-second of the device's memory, while four times that is free or
+//   held already (a failed allocation: the caller's interval), or what
+//   dpd_set_window_memory says.
+// A step made again costs a forward step: at 16,384 beads, a window of 200
+// steps with 70 differentiated, 60 of 260 steps were (the window and its gradient 8.2 ms,
+// 6.8 without); 24 boxes of 65,536, 70 of 250 differentiated, 50 of 300
+// (114.7 ms, 106.0 without, 3.8 GB of configurations).
+static int window_setup(dpd_handle *h, int ckpt, Window &w, AdjBufs &A) {
+    const size_t N = (size_t)h->N, C = (size_t)h->C;
+    const size_t ck_bytes = N * sizeof(float2) * 4 + N * sizeof(uint32_t) + N * sizeof(int2) + C * sizeof(int32_t);
+    const size_t seg_bytes = N * sizeof(float2) * 2 + N * sizeof(uint32_t) * 2 + N * sizeof(int2) + C * sizeof(int32_t);
+    const int64_t steps = w.nsteps - w.stop();
+    const size_t asked = (size_t)((w.nsteps + ckpt - 1) / ckpt) * ck_bytes + (size_t)ckpt * seg_bytes;
+    const size_t held = (size_t)h->adj_nck * ck_bytes + (size_t)h->adj_nseg * seg_bytes;
+    size_t may = asked, free_now = 0, total = 0;
+    if (h->window_mem >= 0) {
+        may = std::max(may, (size_t)h->window_mem);
+    } else {
+        may = std::max(may, held);
+        if (ck_bytes + (size_t)steps * seg_bytes > may) {
+            if (cudaMemGetInfo(&free_now, &total) != cudaSuccess) cudaGetLastError();
+            may = std::max(may, std::min(total / 32, (free_now + held) / 4));
+        }
+    }
+    for (;;) {
+        for (w.nseg = 1;; w.nseg++) {  // ends: segments of at most ckpt steps fit
+            const int64_t len = (steps + w.nseg - 1) / w.nseg;
+            w.len = (int)len;
+            if (len <= ckpt || (len <= INT_MAX && (size_t)w.nseg * ck_bytes + (size_t)len * seg_bytes <= may)) break;
+        }
+        const int rc = adj_setup(h, w.nseg, w.len, w.spec->nbin, A);
+        if (rc != DPD_E_NOMEM || may == asked) return rc;
+        cudaGetLastError();  // the failed allocation's
+        may = asked;
+    }
+}
 
 static void window_forward(dpd_handle *h, AdjBufs &A, const Window &w) {
     const float rmax = (float)w.spec->rmax, sig = (float)w.spec->sigma;
     const int cur0 = h->cur, nb = w.spec->nbin;
     cudaMemsetAsync(A.hist, 0, (size_t)h->nrep * nb * sizeof(double), h->s);
     int par0 = 0, last = 0;  // steps of the last segment, whose configurations stay stored for the reverse pass
+    int sg = -1;  // the segment of the step
     for (int64_t k = 1; k <= w.nsteps; k++) {
-        const int sg = (int)((k - 1) / w.ckpt);
-        if (w.backward && (k - 1) % w.ckpt == 0) ck_save(h, A.ck[sg]);
-        if (w.backward && sg == w.nseg - 1) enqueue_seg_step(h, A, sg, ++last, par0 = h->cur);
+        if (sg + 1 < w.nseg && k - 1 == w.start(sg + 1)) ck_save(h, A.ck[++sg]);
+        if (w.nseg > 0 && sg == w.nseg - 1) enqueue_seg_step(h, A, sg, ++last, par0 = h->cur);
         else enqueue_plain_step(h);
         if (k >= w.first_loss())
             launch_rdf(last ? seg_view(A, sg, last) : view_cur(h), h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb,
@@ -1697,8 +1745,7 @@ static void window_set_step(dpd_handle *h, const Window &w, int64_t k) {
 }
 
 // The reverse pass: segment by segment, the states of each (but the last,
-// stored by the forward pass) recomputed from its checkpoint, down to the
-// step the horizon leaves.  state[0..2] (may be null) receive the device
+// stored by the forward pass) recomputed from its checkpoint.  state[0..2] (may be null) receive the device
 // arrays of the start state's cotangents in gid order.
 static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const float2 **state) {
     const float rmax = (float)w.spec->rmax, sig = (float)w.spec->sigma;
@@ -1711,17 +1758,15 @@ static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const flo
     cudaMemsetAsync(A.F[0], 0, N * sizeof(float2), h->s);
     cudaMemsetAsync(A.grad, 0, (size_t)h->nrep * DPD_NGRAD * sizeof(double), h->s);
     const int64_t first_loss = w.first_loss();
-    const int64_t k_stop = w.spec->horizon > 0 ? std::max<int64_t>(0, first_loss - 1 - w.spec->horizon) : 0;
-    const int sg_stop = (int)(k_stop / w.ckpt), s_stop = (int)(k_stop - (int64_t)sg_stop * w.ckpt);
-    for (int sg = w.nseg - 1; sg >= sg_stop; sg--) {
-        const int64_t k0 = (int64_t)sg * w.ckpt;
-        const int len = (int)std::min<int64_t>(w.ckpt, w.nsteps - k0);
+    for (int sg = w.nseg - 1; sg >= 0; sg--) {
+        const int64_t k0 = w.start(sg);
+        const int len = (int)(w.start(sg + 1) - k0);
         if (sg < w.nseg - 1) {
             window_set_step(h, w, k0);
             enqueue_keys(h, seg_bufs(h, A, sg, 1, 0), 0, true);
             for (int s = 1; s <= len; s++) enqueue_seg_step(h, A, sg, s, 0);
         }
-        for (int s = len; s > (sg == sg_stop ? s_stop : 0); s--) {
+        for (int s = len; s > 0; s--) {
             const int64_t k = k0 + s;
             const StateView v = seg_view(A, sg, s);
             if (k >= first_loss)
@@ -1733,9 +1778,9 @@ static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const flo
             p ^= 1;
         }
     }
-    // the forces stored at step k_stop (the window start without a horizon) depend on the parameters too
-    const StateView v0 = seg_view(A, sg_stop, s_stop);
-    launch_force_vjp(v0, w.step0 + k_stop, h->d_rep, h->d_bch, h->nbch, A.F[p], A.xb, A.vb, A.grad, A.gsum, h->nrep,
+    // the forces stored at the first differentiated step (the window start without a horizon) depend on the parameters too
+    const StateView v0 = seg_view(A, 0, 0);
+    launch_force_vjp(v0, w.step0 + w.stop(), h->d_rep, h->d_bch, h->nbch, A.F[p], A.xb, A.vb, A.grad, A.gsum, h->nrep,
                      h->any_stir, mol, h->s, base);
     if (state) {
         launch_adj_state(v0.tg, h->d_rep, h->d_bch, h->nbch, A.X[p], A.V[p], A.xb, A.vb, A.X[p ^ 1], A.V[p ^ 1],
@@ -1811,14 +1856,13 @@ static int window_impl(dpd_handle *h, int64_t nsteps, int32_t ckpt, const dpd_rd
     if (state_out && spec->horizon > 0)
         return fail(DPD_E_ARG, "start-state cotangents need the full reverse pass (horizon 0)");
     if (ckpt < 1 || ckpt > nsteps) ckpt = (int32_t)nsteps;
-    const int nseg = (int)((nsteps + ckpt - 1) / ckpt);
     const int nb = spec->nbin;
     std::vector<long long> npairs;
     TRY(count_pairs(h, spec, npairs));
     AdjBufs A;
-    TRY(adj_setup(h, backward ? nseg : 0, backward ? ckpt : 0, nb, A));
+    Window w{nsteps, 0, 0, spec, h->step, nullptr};
+    TRY(backward ? window_setup(h, ckpt, w, A) : adj_setup(h, 0, 0, nb, A));
     if (!h->keys_valid) enqueue_next_keys(h);
-    const Window w{nsteps, ckpt, nseg, spec, h->step, nullptr, backward};
     window_forward(h, A, w);
     CK(cudaGetLastError());
     h->step = w.step0 + nsteps;
@@ -1841,6 +1885,12 @@ static int window_impl(dpd_handle *h, int64_t nsteps, int32_t ckpt, const dpd_rd
     }
     CK(cudaStreamSynchronize(h->s));
     return check_status(h);
+}
+
+extern "C" int dpd_set_window_memory(dpd_handle *h, int64_t bytes) {
+    if (!h) return fail(DPD_E_ARG, "null handle");
+    h->window_mem = bytes < 0 ? -1 : bytes;
+    return DPD_OK;
 }
 
 extern "C" int dpd_window_loss(dpd_handle *h, int64_t nsteps, const dpd_rdf_spec *spec, const double *target,
@@ -1919,11 +1969,12 @@ extern "C" int dpd_fit_graph(dpd_handle *h, int64_t nsteps, int32_t ckpt, const 
                 return fail(DPD_E_ARG, "fit: a shared slot (%d) must start equal in every replica", s);
     }
     if (ckpt < 1 || ckpt > nsteps) ckpt = (int32_t)nsteps;
-    const int nseg = (int)((nsteps + ckpt - 1) / ckpt), nb = spec->nbin, nrep = h->nrep;
+    const int nb = spec->nbin, nrep = h->nrep;
     std::vector<long long> npairs;
     TRY(count_pairs(h, spec, npairs));
     AdjBufs A;
-    TRY(adj_setup(h, nseg, ckpt, nb, A));
+    Window w{nsteps, 0, 0, spec, 0, nullptr};
+    TRY(window_setup(h, ckpt, w, A));
     // the fit's own device memory, freed before returning
     char *mem = nullptr;
     const size_t o_np = ((sizeof(FitDev) + 255) / 256) * 256, o_tg = o_np + (((size_t)nrep * 8 + 255) / 256) * 256;
@@ -1933,8 +1984,8 @@ extern "C" int dpd_fit_graph(dpd_handle *h, int64_t nsteps, int32_t ckpt, const 
     const size_t total = o_val + (((size_t)iters * fit->n * 8 + 255) / 256) * 256;
     if (cudaMalloc(&mem, total) != cudaSuccess) return fail(DPD_E_NOMEM, "cudaMalloc(%zu) for the fit", total);
     FitArgs a;
-    a.w = Window{nsteps, ckpt, nseg, spec, 0, (FitDev *)mem, true};
-    a.fd = (FitDev *)mem;
+    a.w = w;
+    a.w.fd = a.fd = (FitDev *)mem;
     a.npairs = (const long long *)(mem + o_np);
     a.target = (const double *)(mem + o_tg);
     a.loss = (double *)(mem + o_loss);

@@ -103,6 +103,7 @@ EXPORTS = [
     "dpd_pair_forces", "dpd_bond_forces", "dpd_integrate", "dpd_chemistry", "dpd_get_events", "dpd_events_async",
     "dpd_observables", "dpd_pair_hist", "dpd_get_stream", "dpd_kernels_per_step", "dpd_step_async",
     "dpd_sync", "dpd_set_graph_steps", "dpd_profile_step", "dpd_stats", "dpd_set_tuning", "dpd_get_tuning",
+    "dpd_set_window_memory",
     "dpd_sort_cells_noalloc", "dpd_set_params", "dpd_window_loss", "dpd_window_adjoint", "dpd_window_adjoint_state",
     "dpd_fit_graph",
     "dpd_force_vjp",
@@ -178,6 +179,7 @@ def load(path: str | None = None):
         "dpd_stats": ([vp, i32, fp], C.c_int),
         "dpd_set_tuning": ([vp, C.POINTER(DpdTuning)], C.c_int),
         "dpd_get_tuning": ([vp, C.POINTER(DpdTuning)], C.c_int),
+        "dpd_set_window_memory": ([vp, C.c_int64], C.c_int),
         "dpd_sort_cells_noalloc": ([fp, fp, i32, dbl, fp, fp, vp], C.c_int),
         "dpd_set_params": ([vp, i32, C.POINTER(DpdParams)], C.c_int),
         "dpd_window_loss": ([vp, i64, C.POINTER(DpdRdfSpec), fp, fp, fp], C.c_int),

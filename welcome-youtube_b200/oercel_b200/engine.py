@@ -343,6 +343,11 @@ class Engine:
         check(self.lib.dpd_window_loss(self.h, int(nsteps), C.byref(spec), ptr(tgt), ptr(loss), ptr(rdf)))
         return loss, rdf
 
+    def set_window_memory(self, nbytes):
+        """bytes the differentiated windows may take for their configurations where that is more than ckpt_every
+        asks for (0: never more, None: the default rule; see dpd_set_window_memory)"""
+        check(self.lib.dpd_set_window_memory(self.h, -1 if nbytes is None else int(nbytes)))
+
     def window_adjoint(self, nsteps, ckpt_every, spec, target):
         """window loss and its gradient (nrep x 66: a_ij upper triangle, gamma, k_bond)"""
         tgt = np.ascontiguousarray(np.broadcast_to(target, (self.nrep, spec.nbin)), np.float64)
