@@ -33,6 +33,7 @@ def run(memory, nsteps, ckpt, last, horizon, replicas, stir):
     (12, 1, 4, 3),    # a checkpoint a step, loss steps in more than one segment
     (17, 4, 2, 6),    # the horizon inside an interval
     (17, 17, 9, 20),  # a horizon past the start
+    (40, 7, 36, 2),   # more loss steps than one launch of their kernels takes
 ])
 def test_segments_agree(cuda_ok, replicas, stir, nsteps, ckpt, last, horizon):
     bead = 4 * 9.0 ** 2 * 33

@@ -142,9 +142,15 @@ __global__ void __launch_bounds__(BEAD_TPB) k_gsum(const RepDev *__restrict__ re
 //   x_bar(n)  = x_bar(n+1) + J_x^T F_bar
 //   vh_bar(n) = dt x_bar(n) + vh_bar(n+1) + J_v^T F_bar
 //   F_bar(n)  = dt^2 x_bar(n) + dt vh_bar(n+1) + cvt J_v^T F_bar
-// of bead d of the configuration n+1; xf = J_x^T F_bar, vf = J_v^T F_bar
-__device__ __forceinline__ void adj_update(const AdjUpdate &u, const RepDev &R, int d, float2 xf, float2 vf) {
-    const float2 x0 = u.X[d], v0 = u.V[d];
+// of bead d (type t) of the configuration n+1; xf = J_x^T F_bar, vf = J_v^T F_bar
+__device__ __forceinline__ void adj_update(const AdjUpdate &u, const RepDev &R, int d, int t, float2 xf, float2 vf) {
+    float2 x0 = u.X[d];
+    const float2 v0 = u.V[d];
+    if (u.G && (t == u.ta || t == u.tb)) {
+        const float2 g = u.G[d];
+        x0.x += g.x;
+        x0.y += g.y;
+    }
     const int o = u.src[d];
     const float2 x = make_float2(x0.x + xf.x, x0.y + xf.y);
     u.X2[o] = x;
@@ -458,7 +464,7 @@ __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long 
         }
         if (act && sub == 0) {
             if (UPDATE) {
-                adj_update(up, R, d, make_float2(xbx, xby), make_float2(vbx, vby));
+                adj_update(up, R, d, ti, make_float2(xbx, xby), make_float2(vbx, vby));
             } else {
                 xbar[d] = make_float2(xbx, xby);
                 vbar[d] = make_float2(vbx, vby);
@@ -503,16 +509,19 @@ struct RdfPair {
 //   VJP == true   lane = pair: the derivative of its bins' Gaussians against
 //                 the bin weights; the bead's sum is taken in the order of the
 //                 window's cells and slots
+// blockIdx.z: the configuration.
 // What bounds it: the issue of the scan (about 200 slots around each bead of
 // the types, most of another type) and of 13 Gaussians per pair and side.
 // 24 boxes of 65,536 beads: 186 us (VJP: 272) against 766 (783) with a thread
 // per bead and an FP64 shared atomic per pair and bin; one box of 16,384: 10
-// (13) against 100 (87).
+// (13) against 100 (87), or 1.7 (2.2) in a launch with 31 others (rdf_batch).
 template <bool VJP>
-__global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__restrict__ reps,
-                                                  const Chunk *__restrict__ ch, int split, RdfConst q, int nsum,
-                                                  double *__restrict__ hist, const double *__restrict__ wgt,
-                                                  float2 *__restrict__ xadd) {
+__global__ void __launch_bounds__(BEAD_TPB) k_rdf(const __grid_constant__ RdfViews views,
+                                                  const RepDev *__restrict__ reps, const Chunk *__restrict__ ch,
+                                                  int split, RdfConst q, int nsum, double *__restrict__ hist,
+                                                  const double *__restrict__ wgt, float2 *__restrict__ G, size_t N) {
+    const StateView sv = views.v[blockIdx.z];
+    if (VJP) G += blockIdx.z * N;
     __shared__ int list[BEAD_TPB];
     __shared__ int nlist, next;
     __shared__ RdfPair queue[RDF_WARPS][RDF_QCAP];
@@ -682,10 +691,7 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
             evaluate(waiting);
             waiting = 0;
             const float gy = __shfl_sync(0xffffffffu, gx, 1);
-            if (lane == 0) {
-                const float2 x = xadd[d];
-                xadd[d] = make_float2(x.x + gx, x.y + gy);
-            }
+            if (lane == 0) G[d] = make_float2(gx, gy);
             gx = 0.0f;
         }
         int nxt = 0;
@@ -704,12 +710,13 @@ __global__ void __launch_bounds__(BEAD_TPB) k_rdf(StateView sv, const RepDev *__
 }
 
 // the adjoint of the update alone, after the branched shapes' k_mol_vjp has added its share to xb
-__global__ void __launch_bounds__(BEAD_TPB) k_adj_update(const RepDev *__restrict__ reps, const Chunk *__restrict__ ch,
+__global__ void __launch_bounds__(BEAD_TPB) k_adj_update(const uint32_t *__restrict__ tg,
+                                                         const RepDev *__restrict__ reps, const Chunk *__restrict__ ch,
                                                          const float2 *__restrict__ xb, const float2 *__restrict__ vb,
                                                          AdjUpdate up) {
     const Chunk c = ch[blockIdx.x];
     const int d = c.begin + (int)threadIdx.x;
-    if (d < c.end) adj_update(up, reps[c.rep], d, xb[d], vb[d]);
+    if (d < c.end) adj_update(up, reps[c.rep], d, (int)(tg[d] >> TYPE_SHIFT), xb[d], vb[d]);
 }
 
 // cotangents of the window's start state into gid order: x_bar(0) gains the part
@@ -832,7 +839,7 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
     else go(update ? k_force_vjp<2, 4, true> : k_force_vjp<2, 4, false>, 2, 4);
     if (mol) {
         k_mol_vjp<<<nbch, BEAD_TPB, 0, s>>>(sv, rep, bch, mol, g, xbar, grad);
-        if (up) k_adj_update<<<nbch, BEAD_TPB, 0, s>>>(rep, bch, xbar, vbar, *up);
+        if (up) k_adj_update<<<nbch, BEAD_TPB, 0, s>>>(sv.tg, rep, bch, xbar, vbar, *up);
     }
 }
 
@@ -844,21 +851,28 @@ static int rdf_split(int nbch) {
     return split;
 }
 
-void launch_rdf(const StateView &sv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
+// A configuration of a small box is a fraction of a wave, its time that of the
+// slowest warp: one of 16,384 beads alone takes 10 us (VJP: 13), 32 together 1.7
+// (2.2) each.  So as many are taken together as make two waves of whole chunks;
+// a box with that many chunks alone gains nothing by it.
+int rdf_batch(int nbch) { return std::max(1, std::min(RDF_VIEWS, 2 * 8 * 148 / nbch)); }
+
+void launch_rdf(const RdfViews &views, int nv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
                 float rmax, float sigma, double *hist, cudaStream_t s) {
     RdfConst q{ta, tb, nbin, rmax, sigma};
-    const int split = rdf_split(nbch);
+    const int split = rdf_split(nbch * nv);
     // up to 256 bins (32 KB of sums a CTA) in one pass over the pairs, more in blocks of 256
     const int nsum = std::min(nbin, 256);
-    k_rdf<false><<<dim3(nbch * split, (nbin + nsum - 1) / nsum), BEAD_TPB, 2 * RDF_WARPS * nsum * sizeof(double), s>>>(
-        sv, rep, bch, split, q, nsum, hist, nullptr, nullptr);
+    k_rdf<false><<<dim3(nbch * split, (nbin + nsum - 1) / nsum, nv), BEAD_TPB, 2 * RDF_WARPS * nsum * sizeof(double),
+                   s>>>(views, rep, bch, split, q, nsum, hist, nullptr, nullptr, 0);
 }
 
-void launch_rdf_vjp(const StateView &sv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
-                    float rmax, float sigma, const double *wgt, float2 *xadd, cudaStream_t s) {
+void launch_rdf_vjp(const RdfViews &views, int nv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb,
+                    int nbin, float rmax, float sigma, const double *wgt, float2 *G, size_t N, cudaStream_t s) {
     RdfConst q{ta, tb, nbin, rmax, sigma};
-    const int split = rdf_split(nbch);
-    k_rdf<true><<<nbch * split, BEAD_TPB, nbin * sizeof(float), s>>>(sv, rep, bch, split, q, 0, nullptr, wgt, xadd);
+    const int split = rdf_split(nbch * nv);
+    k_rdf<true><<<dim3(nbch * split, 1, nv), BEAD_TPB, nbin * sizeof(float), s>>>(views, rep, bch, split, q, 0, nullptr,
+                                                                                wgt, G, N);
 }
 
 void launch_adj_state(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *X,

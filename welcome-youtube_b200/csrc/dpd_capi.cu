@@ -62,6 +62,7 @@ struct AdjBufs {
     float2 *vh[2], *f[2];       // the half-step velocities and forces of a segment's steps, in turn
     float2 *X[2], *V[2], *F[2]; // the adjoint state of one configuration and of the one before, in turn
     float2 *xb, *vb;
+    float2 *G;                  // the loss's own x_bar of rdf_batch() configurations
     double *hist, *wgt, *grad;
     double *gsum;            // per replica: the sum of the x cotangents (stirring)
     long long *stir;         // per replica: the stirring sums of a segment's steps
@@ -1556,6 +1557,7 @@ static int adj_setup(dpd_handle *h, int nck, int nseg, int nbin, AdjBufs &A) {
         want(&A.V[k], N);
         want(&A.F[k], N);
     }
+    want(&A.G, N * std::min(nseg, rdf_batch(h->nbch)));
     want(&A.xb, N);
     want(&A.vb, N);
     want(&A.hist, (size_t)h->nrep * nbin);
@@ -1713,13 +1715,19 @@ static void window_forward(dpd_handle *h, AdjBufs &A, const Window &w) {
     cudaMemsetAsync(A.hist, 0, (size_t)h->nrep * nb * sizeof(double), h->s);
     int par0 = 0, last = 0;  // steps of the last segment, whose configurations stay stored for the reverse pass
     int sg = -1;  // the segment of the step
+    const int batch = rdf_batch(h->nbch);
+    RdfViews views;
+    int nv = 0;
     for (int64_t k = 1; k <= w.nsteps; k++) {
         if (sg + 1 < w.nseg && k - 1 == w.start(sg + 1)) ck_save(h, A.ck[++sg]);
         if (w.nseg > 0 && sg == w.nseg - 1) enqueue_seg_step(h, A, sg, ++last, par0 = h->cur);
         else enqueue_plain_step(h);
-        if (k >= w.first_loss())
-            launch_rdf(last ? seg_view(A, sg, last) : view_cur(h), h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb,
-                       nb, rmax, sig, A.hist, h->s);
+        if (k < w.first_loss()) continue;
+        views.v[nv++] = last ? seg_view(A, sg, last) : view_cur(h);
+        if (!last || nv == batch || k == w.nsteps) {  // kept configurations wait for a launch's worth of them
+            launch_rdf(views, nv, h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb, nb, rmax, sig, A.hist, h->s);
+            nv = 0;
+        }
     }
     if (!last) return;
     // the end of the window into the handle's buffers, those it started from (a captured iteration is replayed there)
@@ -1752,6 +1760,7 @@ static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const flo
     const size_t N = (size_t)h->N;
     const dpd_template *mol = h->any_mol ? h->b.mol : nullptr;
     const long long *base = w.fd ? &w.fd->base : nullptr;
+    const int batch = rdf_batch(h->nbch);
     int p = 0;  // which of X, V, F hold the adjoint state
     cudaMemsetAsync(A.X[0], 0, N * sizeof(float2), h->s);
     cudaMemsetAsync(A.V[0], 0, N * sizeof(float2), h->s);
@@ -1766,14 +1775,21 @@ static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const flo
             enqueue_keys(h, seg_bufs(h, A, sg, 1, 0), 0, true);
             for (int s = 1; s <= len; s++) enqueue_seg_step(h, A, sg, s, 0);
         }
+        int g0 = 0, ng = 0;  // A.G holds the loss's x_bar of the segment's steps g0, g0 - 1, ... (ng of them)
         for (int s = len; s > 0; s--) {
             const int64_t k = k0 + s;
-            const StateView v = seg_view(A, sg, s);
-            if (k >= first_loss)
-                launch_rdf_vjp(v, h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb, w.spec->nbin, rmax, sig, A.wgt,
-                               A.X[p], h->s);
-            const AdjUpdate up{A.X[p], A.V[p], A.F[p], A.X[p ^ 1], A.V[p ^ 1], A.F[p ^ 1], A.seg[s - 1].src};
-            launch_force_vjp(v, w.step0 + k, h->d_rep, h->d_bch, h->nbch, A.F[p], A.xb, A.vb, A.grad, A.gsum, h->nrep,
+            const bool in_loss = k >= first_loss;
+            if (in_loss && (g0 < s || g0 - s >= ng)) {
+                g0 = s;
+                ng = (int)std::min<int64_t>(std::min(s, batch), k - first_loss + 1);
+                RdfViews views;
+                for (int u = 0; u < ng; u++) views.v[u] = seg_view(A, sg, s - u);
+                launch_rdf_vjp(views, ng, h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb, w.spec->nbin, rmax, sig,
+                               A.wgt, A.G, N, h->s);
+            }
+            const AdjUpdate up{A.X[p], A.V[p], A.F[p], A.X[p ^ 1], A.V[p ^ 1], A.F[p ^ 1], A.seg[s - 1].src,
+                               in_loss ? A.G + (size_t)(g0 - s) * N : nullptr, w.spec->ta, w.spec->tb};
+            launch_force_vjp(seg_view(A, sg, s), w.step0 + k, h->d_rep, h->d_bch, h->nbch, A.F[p], A.xb, A.vb, A.grad, A.gsum, h->nrep,
                              h->any_stir, mol, h->s, base, &up);
             p ^= 1;
         }

@@ -298,11 +298,14 @@ void launch_forces_bulk(const Bufs &b, int cur, const RepDev *rep, const TileDes
 // The adjoint of the Groot-Warren update that made a configuration from the
 // one before: (X, V, F) hold x_bar, vh_bar and F_bar in its slots, (X2, V2, F2)
 // take them in the slots of the configuration before (old slot = src[slot],
-// the step's sort).
+// the step's sort).  G (or null): the loss's own x_bar of this configuration,
+// set for the beads of types ta and tb.
 struct AdjUpdate {
     const float2 *X, *V, *F;
     float2 *X2, *V2, *F2;
     const int32_t *src;
+    const float2 *G;
+    int ta, tb;
 };
 // gsum: nrep doubles of scratch (the mean x cotangent of the stirring term), used when stir;
 // mol: the replicas' lipid templates when some replica has branched lipids, else null;
@@ -327,10 +330,18 @@ void launch_rdf_loss(const RepDev *rep, int nrep, const double *hist, const long
                      cudaStream_t s);
 void launch_fit_update(RepDev *rep, int nrep, const double *grad, FitDev *fd, double *grad_out, double *value_out,
                        cudaStream_t s);
-void launch_rdf(const StateView &sv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
+#define RDF_VIEWS 32  // configurations a launch of the loss's kernels takes
+struct RdfViews {
+    StateView v[RDF_VIEWS];
+};
+// how many configurations of nbch chunks a launch should take where that many are stored
+int rdf_batch(int nbch);
+// the histogram of the configurations v[0, nv) added to hist
+void launch_rdf(const RdfViews &views, int nv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
                 float rmax, float sigma, double *hist, cudaStream_t s);
-void launch_rdf_vjp(const StateView &sv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb, int nbin,
-                    float rmax, float sigma, const double *wgt, float2 *xadd, cudaStream_t s);
+// the loss's x_bar of the beads of types ta and tb in configuration v[k] to G + k N
+void launch_rdf_vjp(const RdfViews &views, int nv, const RepDev *rep, const Chunk *bch, int nbch, int ta, int tb,
+                    int nbin, float rmax, float sigma, const double *wgt, float2 *G, size_t N, cudaStream_t s);
 // the start-state cotangents of slot-order X, V, xb, vb into gid-order arrays: positions, half-step velocities,
 // predicted velocities
 void launch_adj_state(const uint32_t *tg, const RepDev *rep, const Chunk *bch, int nbch, const float2 *X,
