@@ -257,10 +257,11 @@ DPD_API int dpd_get_tuning(const dpd_handle *h, dpd_tuning *t);
 DPD_API int dpd_set_graph_steps(dpd_handle *h, int32_t steps);
 /* One real step launched kernel by kernel with CUDA events around each launch
  * on the handle's stream: ms[k] = device time of kernel k in launch order
- * (scan1, scan2, place, cellfix, permute, [2 chemistry kernels], [catalyst
+ * (scan1, scan2, place, cellfix, permute, [2 chemistry entries], [catalyst
  * check with its sort], forces); *n_out = number of kernels.  On a step with a
  * catalyst check the first entry is a one-thread step-counter kernel and the
- * next three are not launched (0 ms). */
+ * next three are not launched (0 ms).  An entry whose kernel the handle's sort
+ * does not launch (sort_mode) and the second chemistry entry are 0 ms too. */
 DPD_API int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *n_out);
 
 /* The reference's random soup (init_soup + set_velocities,

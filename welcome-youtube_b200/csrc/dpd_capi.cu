@@ -984,7 +984,7 @@ extern "C" int dpd_chemistry(dpd_handle *h, int64_t step) {
     TRY(set_device_step(h, step));
     CK(cudaMemsetAsync(&h->b.status->n_grow, 0, 2 * sizeof(unsigned), h->s));
     launch_chem_scan(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->s);
-    launch_chem_lists(h->b, h->cur, h->d_rep, -1, h->s);
+    launch_chem_lists(h->b, h->cur, h->d_rep, h->s);
     // the catalyst chemistry as the reference's chemistry(): no sort afterwards
     if (h->any_cat) launch_catalyst(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->nrep, h->C, h->nmax, h->stream_grid, h->s);
     CK(cudaGetLastError());
@@ -1020,7 +1020,7 @@ static void enqueue_step(dpd_handle *h, int64_t s) {
     }
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, cat ? PERM_KEEP : PERM_STEP, h->s);
     h->cur ^= 1;
-    if (h->any_lipid) launch_chem_lists(h->b, h->cur, h->d_rep, -1, h->s);
+    if (h->any_lipid) launch_chem_lists(h->b, h->cur, h->d_rep, h->s);
     if (cat) {
         launch_resort(plain_counts(h), h->cur, h->d_rep, h->d_bch, h->nbch, h->d_cch, h->ncch, h->C, h->s);
         launch_catalyst(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->nrep, h->C, h->nmax, h->stream_grid, h->s);
@@ -1164,7 +1164,7 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
     if (!h || !ms || !n_out) return fail(DPD_E_ARG, "null argument");
     if (!h->keys_valid) enqueue_next_keys(h);
     const bool cat = cat_at(h, h->step + 1);
-    const int nk = 6 + (h->any_lipid ? chem_kernel_count() : 0) + (cat ? 1 : 0);
+    const int nk = 6 + (h->any_lipid ? 2 : 0) + (cat ? 1 : 0);
     if (cap < nk) return fail(DPD_E_ARG, "need room for %d kernel times", nk);
     std::vector<cudaEvent_t> ev(nk + 1);
     for (auto &e : ev) CK(cudaEventCreate(&e));
@@ -1199,11 +1199,10 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
     launch_permute(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, cat ? PERM_KEEP : PERM_STEP, h->s);
     CK(cudaEventRecord(ev[k++], h->s));
     h->cur ^= 1;
-    if (h->any_lipid)
-        for (int c = 0; c < chem_kernel_count(); c++) {
-            launch_chem_lists(h->b, h->cur, h->d_rep, c, h->s);
-            CK(cudaEventRecord(ev[k++], h->s));
-        }
+    if (h->any_lipid) {  // one kernel; the second chemistry entry is 0
+        launch_chem_lists(h->b, h->cur, h->d_rep, h->s);
+        for (int c = 0; c < 2; c++) CK(cudaEventRecord(ev[k++], h->s));
+    }
     if (cat) {
         launch_resort(plain_counts(h), h->cur, h->d_rep, h->d_bch, h->nbch, h->d_cch, h->ncch, h->C, h->s);
         launch_catalyst(h->b, h->cur, h->d_rep, h->d_bch, h->nbch, h->nrep, h->C, h->nmax, h->stream_grid, h->s);

@@ -128,10 +128,12 @@ __device__ __forceinline__ bool growable_end(const uint32_t *tg, const int2 *lin
 }
 
 // the 3x3 cells around position pi as contiguous slot ranges: per column the
-// rows cy-1..cy+1 are one range, or two where the rows wrap
+// rows cy-1..cy+1 are one range, or two where the rows wrap.  The f-th bead of
+// them is slot f + off[k] of the first range with f < end[k] (ends counted
+// together; all indexes known, so the six stay in registers).
 struct NbrRanges {
-    int s[6], e[6];
-    int n, total;
+    int off[6], end[6];
+    int total;
 };
 
 __device__ __forceinline__ NbrRanges nbr_ranges(const Bufs &b, const RepDev &R, float2 pi) {
@@ -140,38 +142,32 @@ __device__ __forceinline__ NbrRanges nbr_ranges(const Bufs &b, const RepDev &R, 
     const int32_t *cs = b.cstart + R.c0;
     int cx, cy;
     cell_xy(R, pi.x, pi.y, cx, cy);
-    q.n = 0;
+    const int left = cx > 0 ? cx - 1 : ncx - 1, right = cx + 1 < ncx ? cx + 1 : 0;
+    // rows [r0, r1), then [0, r2) where they wrap
+    const int r0 = cy > 0 ? cy - 1 : ncy - 1, r1 = cy > 0 ? min(cy + 2, ncy) : ncy;
+    const int r2 = cy == 0 ? 2 : (cy + 1 == ncy ? 1 : 0);
     q.total = 0;
 #pragma unroll
-    for (int ox = -1; ox <= 1; ox++) {
-        const int col = ((cx + ox + ncx) % ncx) * ncy;
-        if (cy >= 1 && cy + 1 < ncy) {
-            q.s[q.n] = cs[col + cy - 1];
-            q.e[q.n++] = cs[col + cy + 2];
-        } else if (cy == 0) {
-            q.s[q.n] = cs[col + ncy - 1];
-            q.e[q.n++] = cs[col + ncy];
-            q.s[q.n] = cs[col];
-            q.e[q.n++] = cs[col + 2];
-        } else {
-            q.s[q.n] = cs[col + cy - 1];
-            q.e[q.n++] = cs[col + ncy];
-            q.s[q.n] = cs[col];
-            q.e[q.n++] = cs[col + 1];
-        }
+    for (int c = 0; c < 3; c++) {
+        const int32_t *col = cs + (c == 0 ? left : (c == 1 ? cx : right)) * ncy;
+        const int s0 = col[r0], e0 = col[r1], s1 = col[0], e1 = col[r2];
+        q.off[2 * c] = s0 - q.total;
+        q.total += e0 - s0;
+        q.end[2 * c] = q.total;
+        q.off[2 * c + 1] = s1 - q.total;
+        q.total += e1 - s1;
+        q.end[2 * c + 1] = q.total;
     }
-    for (int k = 0; k < q.n; k++) q.total += q.e[k] - q.s[k];
     return q;
 }
 
 // slot of the f-th bead of the ranges
 __device__ __forceinline__ int nbr_slot(const NbrRanges &q, int f) {
-    int k = 0;
-    while (f >= q.e[k] - q.s[k]) {
-        f -= q.e[k] - q.s[k];
-        k++;
-    }
-    return q.s[k] + f;
+    int off = q.off[5];
+#pragma unroll
+    for (int k = 4; k >= 0; k--)
+        if (f < q.end[k]) off = q.off[k];
+    return f + off;
 }
 
 // warp minimum of a 64-bit key (distance bits, gid): the lexicographic nearest
@@ -197,7 +193,7 @@ __device__ __forceinline__ bool maybe_end(uint32_t tj, int2 lj) {
 
 #define GROW_KEEP 4  // candidate ends a lane keeps in registers (32 x 4 = 128 beads in the 3x3 cells)
 
-// stage 2 request of list entry k, by one whole warp: the listed P needs
+// stage 2 request of entry k of the growth list, by one whole warp: the listed P needs
 // >= n_t_min T beads within r_grow and claims its nearest growable end within
 // r_grow (req[k] = end or -1).  Each lane keeps the possible ends among its
 // candidates; the warp then takes them in increasing (distance, gid) order and
@@ -229,13 +225,13 @@ __device__ __forceinline__ void chem_grow_req_one(const Bufs &b, int cur, const 
         const int f = lane + 32 * m;
         if (f >= q.total) break;
         const int j = nbr_slot(q, f);
-        if (j == d) continue;
-        const float2 pj = pos[j];
-        const float dd = dist2(pi.x, pi.y, pj.x, pj.y, L, h);
-        if (!(dd < r2)) continue;
+        const float2 pj = pos[j];  // all three at once: the kernel is a chain of dependent loads
         const uint32_t tj = tg[j];
+        const int2 lj = link[j];
+        const float dd = dist2(pi.x, pi.y, pj.x, pj.y, L, h);
+        if (j == d || !(dd < r2)) continue;
         nt += type_of(tj) == T_T;
-        if (maybe_end(tj, link[j])) {
+        if (maybe_end(tj, lj)) {
             key[m] = ((unsigned long long)__float_as_uint(dd) << 32) | (tj & GID_MASK);
             slot[m] = j;
         }
@@ -324,57 +320,45 @@ __device__ __forceinline__ void chem_grow_apply_one(const Bufs &b, int cur, int 
     push_event(b, step, 0, g, tg[e] & GID_MASK, p.x, p.y, it.y);
 }
 
-// stage 3 request of list entry k, by one whole warp: a T that is still free
-// claims its nearest free H within r_bond
-__device__ __forceinline__ void chem_bond_req_one(const Bufs &b, int cur, const RepDev *__restrict__ reps, int k,
-                                                  int lane) {
+// the nearest free H within r_bond of a T that is still free, entry it of the
+// bonding list, found by one whole warp (-1: none)
+__device__ __forceinline__ int chem_bond_find(const Bufs &b, int cur, const RepDev *__restrict__ reps, int2 it,
+                                              int lane) {
     const uint32_t *tg = b.tg[cur];
     const float2 *pos = b.pos[cur];
     const int2 *link = b.link[cur];
-    const int2 it = b.bond_list[k];
     const int d = it.x;
     const int2 lk = link[d];
-    int e = -1;
-    if (type_of(tg[d]) == T_T && lk.x < 0 && lk.y < 0) {
-        const RepDev &R = reps[it.y];
-        const float2 pi = pos[d];
-        const float L = R.L, h = R.halfL, r2 = R.r2_bond;
-        const NbrRanges q = nbr_ranges(b, R, pi);
-        unsigned long long best = NONE_LIST_KEY;
-        int bj = -1;
-        for (int f = lane; f < q.total; f += 32) {
-            const int j = nbr_slot(q, f);
-            if (j == d) continue;
-            const uint32_t tj = tg[j];
-            if (type_of(tj) != T_H) continue;
-            const int2 lj = link[j];
-            if (lj.x >= 0 || lj.y >= 0) continue;
-            const float2 pj = pos[j];
-            const float dd = dist2(pi.x, pi.y, pj.x, pj.y, L, h);
-            if (!(dd < r2)) continue;
-            const unsigned long long key = ((unsigned long long)__float_as_uint(dd) << 32) | (tj & GID_MASK);
-            if (key < best) {
-                best = key;
-                bj = j;
-            }
+    const uint32_t td = tg[d];
+    const float2 pi = pos[d];
+    if (type_of(td) != T_T || lk.x >= 0 || lk.y >= 0) return -1;
+    const RepDev &R = reps[it.y];
+    const float L = R.L, h = R.halfL, r2 = R.r2_bond;
+    const NbrRanges q = nbr_ranges(b, R, pi);
+    unsigned long long best = NONE_LIST_KEY;
+    int bj = -1;
+    for (int f = lane; f < q.total; f += 32) {
+        const int j = nbr_slot(q, f);
+        const float2 pj = pos[j];
+        const uint32_t tj = tg[j];
+        const int2 lj = link[j];
+        const float dd = dist2(pi.x, pi.y, pj.x, pj.y, L, h);
+        if (j == d || type_of(tj) != T_H || lj.x >= 0 || lj.y >= 0 || !(dd < r2)) continue;
+        const unsigned long long key = ((unsigned long long)__float_as_uint(dd) << 32) | (tj & GID_MASK);
+        if (key < best) {
+            best = key;
+            bj = j;
         }
-        const unsigned long long wbest = warp_min_u64(best);
-        const int mine = (best == wbest && wbest != NONE_LIST_KEY) ? bj : -1;
-        e = (int)__reduce_max_sync(0xffffffffu, (unsigned)(mine + 1)) - 1;
     }
-    if (lane == 0) {
-        b.req[k] = e;
-        if (e >= 0) atomicMin(b.claim + e, tg[d] & GID_MASK);
-    }
+    const unsigned long long wbest = warp_min_u64(best);
+    const int mine = (best == wbest && wbest != NONE_LIST_KEY) ? bj : -1;
+    return (int)__reduce_max_sync(0xffffffffu, (unsigned)(mine + 1)) - 1;
 }
 
-// stage 3 application of list entry k
-__device__ __forceinline__ void chem_bond_apply_one(const Bufs &b, int cur, int k, long long step) {
-    const int h = __ldcg(b.req + k);
-    if (h < 0) return;
+// stage 3 application of a bonding list entry that claimed the free H bead h
+__device__ __forceinline__ void chem_bond_apply_one(const Bufs &b, int cur, int2 it, int h, long long step) {
     const uint32_t *tg = b.tg[cur];
     int2 *link = b.link[cur];
-    const int2 it = b.bond_list[k];
     const int d = it.x;
     const uint32_t g = tg[d] & GID_MASK;
     if (__ldcg(b.claim + h) != g) return;

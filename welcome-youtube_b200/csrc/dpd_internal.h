@@ -352,5 +352,5 @@ int chem_kernel_count();
 int lib_error(int code, const char *msg);  // sets dpd_last_error() and returns code
 // the break stage and the candidate draws on the current sorted state (phase entry point)
 void launch_chem_scan(const Bufs &b, int cur, const RepDev *rep, const Chunk *bch, int nbch, cudaStream_t s);
-// the growth and bonding stages over the candidate lists (part 0..3, or all with part < 0)
-void launch_chem_lists(const Bufs &b, int cur, const RepDev *rep, int part, cudaStream_t s);
+// the growth and bonding stages over the candidate lists
+void launch_chem_lists(const Bufs &b, int cur, const RepDev *rep, cudaStream_t s);
