@@ -172,12 +172,14 @@ __device__ __forceinline__ void adj_update(const AdjUpdate &u, const RepDev &R, 
 // its gradient sums over when the replica changes and at its end.  UPDATE: the
 // adjoint of the step's update is applied at once (adj_update); else the
 // products go to xbar and vbar.
-// What bounds it: instruction issue (about 180 warp instructions a bead at
-// density 4, 2.2 of 4 a cycle: half of them the 12.6 evaluations, 40 of whose
-// 140 instructions are the noise) and the fullest list of a warp, 1.6 times the
-// mean.  24 boxes of 65,536 beads: about 420 us, against 939 (and 82 for the update)
-// with a thread per bead and an FP64 shared atomic per pair; one box: 34
-// against 68, of 16,384: 14 against 60, of 4,096: 10 against 61.  Tried: one
+// What bounds it: about 180 warp instructions a bead at density 4, half of them
+// the 12.6 evaluations (40 of whose 140 instructions are the noise), issued at
+// 2.2 of 4 a cycle: the chains of loads and arithmetic of a few warps.  So a
+// lane evaluates two pairs at a time: 24 boxes of 65,536 beads 403 us, 429 with
+// one.  And the fullest list of a warp is 1.6 times the mean.  The same boxes
+// took 939 us (and 82 for the update) with a thread per bead and an FP64 shared
+// atomic per pair; one box 31 against 68, of 16,384: 14 against 60, of 4,096: 10
+// against 61.  Tried: one
 // queue of pairs per warp evaluated by full rounds, its terms summed through
 // shared memory, 504 us (more shared memory, 16 warps an SM); the order of the
 // sum left to the lanes, 397 us.
@@ -257,6 +259,7 @@ __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long 
             tgi = sv.tg[d];
             cell_xy(R, pi.x, pi.y, cx, cy);
         }
+        const int d0 = act ? d : c.begin;  // (a slot to read for lanes without a pair)
         const uint32_t gi = tgi & GID_MASK;
         const int ti = (int)(tgi >> TYPE_SHIFT);
         const bool low = act && cy == 0, high = act && cy == ncy - 1;  // ncy >= 3: the rows wrap at one end
@@ -308,89 +311,102 @@ __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long 
             return k + (k < l0 ? b0 : (k < l1 ? b1 : (k < l2 ? b2 : (k < l3 ? b3 : (k < l4 ? b4 : b5)))));
         };
         float xbx = 0.f, xby = 0.f, vbx = 0.f, vby = 0.f;  // x_bar in the bead's first lane, v_bar in its second
-        // the listed pairs [0, n) of every bead, in turn; their terms are added in the list's order
-        auto evaluate = [&](int n) {
-            __syncwarp();
-            const int rounds = (__reduce_max_sync(0xffffffffu, n) + LPB - 1) / LPB;
-            for (int q = 0; q < rounds; q++) {
-                const int k = q * LPB + sub;
-                float tx = 0.f, ty = 0.f, u = 0.f, hx = 0.f, hy = 0.f;
-                if (k < n) {
-                    const int j = list[bead][k];
-                    const float2 pj = sv.pos[j], vj = sv.vt[j], gj = g[j];
-                    const uint32_t tgj = sv.tg[j];
-                    const int tj = (int)(tgj >> TYPE_SHIFT);
-                    float dx = __fsub_rn(pi.x, pj.x), dy = __fsub_rn(pi.y, pj.y);
-                    if (wrap) {
-                        dx = minimg(dx, L, h);
-                        dy = minimg(dy, L, h);
+        // The pair of the lane's bead with entry k of its list (some entry if there are only n: then nothing counts);
+        // its terms, and the parameter gradients.
+        struct Terms {
+            float tx, ty, u, hx, hy;
+        };
+        auto pair = [&](int k, int n) {
+            Terms t;
+            const int j = n > 0 ? list[bead][min(k, n - 1)] : d0;
+            const float2 pj = sv.pos[j], vj = sv.vt[j], gj = g[j];
+            const uint32_t tgj = sv.tg[j];
+            const int tj = (int)(tgj >> TYPE_SHIFT);
+            float dx = __fsub_rn(pi.x, pj.x), dy = __fsub_rn(pi.y, pj.y);
+            if (wrap) {
+                dx = minimg(dx, L, h);
+                dy = minimg(dy, L, h);
+            }
+            const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+            float r, ir;
+            r_and_ir(r2, r, ir);
+            const float w = 1.0f - r;
+            const float dvx = vi.x - vj.x, dvy = vi.y - vj.y;
+            const float rv = (dx * dvx + dy * dvy) * ir;
+            const float th = pair_theta(nk, gi, tgj & GID_MASK);
+            const float a = a_sh[ti * DPD_MAXT + tj];
+            const float A = a - gam * w * rv + s * th;
+            const float fm = w * A * ir;
+            const float cxv = gi2.x - gj.x, cyv = gi2.y - gj.y;
+            const float cd = cxv * dx + cyv * dy;
+            const float dfr = (-A + w * gam * rv) * ir - w * A * ir * ir;
+            const float dfv = -gam * w * w * ir;
+            t.hx = dx * ir;
+            t.hy = dy * ir;
+            t.tx = __fmaf_rn(fm, cxv, __fmul_rn(cd, dfr * t.hx + dfv * (dvx - rv * t.hx) * ir));
+            t.ty = __fmaf_rn(fm, cyv, __fmul_rn(cd, dfr * t.hy + dfv * (dvy - rv * t.hy) * ir));
+            t.u = cd * dfv;
+            if (k < n && gi < (tgj & GID_MASK)) {  // parameter gradients: each pair once
+                const int lo = min(ti, tj), hi = max(ti, tj);
+                const double da = (double)(cd * w * ir);
+                if (hi < VJP_TYPES) acc[lo * (2 * VJP_TYPES - 1 - lo) / 2 + hi][tid] += da;
+                else atomicAdd(&sgrad[lo * DPD_MAXT + hi], da);
+                ggam += (double)(cd * w * (-w * rv + (gam > 0.0f ? s * th / (2.0f * gam) : 0.0f)) * ir);
+            }
+            return t;
+        };
+        // the terms of round q's pairs added in the list's order
+        auto add = [&](const Terms &t, int q, int n) {
+            if (LPB == 2) {  // each lane hands the other what it sums
+                const float o1 = __shfl_xor_sync(0xffffffffu, sub ? t.tx : t.u, 1);
+                const float o2 = __shfl_xor_sync(0xffffffffu, sub ? t.ty : t.hx, 1);
+                const float o3 = __shfl_xor_sync(0xffffffffu, t.hy, 1);
+                const int left = n - q * LPB;
+                if (sub == 0) {
+                    if (left > 0) {
+                        xbx += t.tx;
+                        xby += t.ty;
                     }
-                    const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
-                    float r, ir;
-                    r_and_ir(r2, r, ir);
-                    const float w = 1.0f - r;
-                    const float dvx = vi.x - vj.x, dvy = vi.y - vj.y;
-                    const float rv = (dx * dvx + dy * dvy) * ir;
-                    const float th = pair_theta(nk, gi, tgj & GID_MASK);
-                    const float a = a_sh[ti * DPD_MAXT + tj];
-                    const float A = a - gam * w * rv + s * th;
-                    const float fm = w * A * ir;
-                    const float cxv = gi2.x - gj.x, cyv = gi2.y - gj.y;
-                    const float cd = cxv * dx + cyv * dy;
-                    const float dfr = (-A + w * gam * rv) * ir - w * A * ir * ir;
-                    const float dfv = -gam * w * w * ir;
-                    hx = dx * ir;
-                    hy = dy * ir;
-                    tx = __fmaf_rn(fm, cxv, __fmul_rn(cd, dfr * hx + dfv * (dvx - rv * hx) * ir));
-                    ty = __fmaf_rn(fm, cyv, __fmul_rn(cd, dfr * hy + dfv * (dvy - rv * hy) * ir));
-                    u = cd * dfv;
-                    if (gi < (tgj & GID_MASK)) {  // parameter gradients: each pair once
-                        const int lo = min(ti, tj), hi = max(ti, tj);
-                        const double da = (double)(cd * w * ir);
-                        if (hi < VJP_TYPES) acc[lo * (2 * VJP_TYPES - 1 - lo) / 2 + hi][tid] += da;
-                        else atomicAdd(&sgrad[lo * DPD_MAXT + hi], da);
-                        ggam += (double)(cd * w * (-w * rv + (gam > 0.0f ? s * th / (2.0f * gam) : 0.0f)) * ir);
-                    }
-                }
-                if (LPB == 2) {  // each lane hands the other what it sums
-                    const float o1 = __shfl_xor_sync(0xffffffffu, sub ? tx : u, 1);
-                    const float o2 = __shfl_xor_sync(0xffffffffu, sub ? ty : hx, 1);
-                    const float o3 = __shfl_xor_sync(0xffffffffu, hy, 1);
-                    const int left = n - q * LPB;
-                    if (sub == 0) {
-                        if (left > 0) {
-                            xbx += tx;
-                            xby += ty;
-                        }
-                        if (left > 1) {
-                            xbx += o1;
-                            xby += o2;
-                        }
-                    } else {
-                        if (left > 0) {
-                            vbx = __fmaf_rn(o1, o2, vbx);
-                            vby = __fmaf_rn(o1, o3, vby);
-                        }
-                        if (left > 1) {
-                            vbx = __fmaf_rn(u, hx, vbx);
-                            vby = __fmaf_rn(u, hy, vby);
-                        }
+                    if (left > 1) {
+                        xbx += o1;
+                        xby += o2;
                     }
                 } else {
+                    if (left > 0) {
+                        vbx = __fmaf_rn(o1, o2, vbx);
+                        vby = __fmaf_rn(o1, o3, vby);
+                    }
+                    if (left > 1) {
+                        vbx = __fmaf_rn(t.u, t.hx, vbx);
+                        vby = __fmaf_rn(t.u, t.hy, vby);
+                    }
+                }
+            } else {
 #pragma unroll
-                    for (int i = 0; i < LPB; i++) {
-                        const float ax = __shfl_sync(0xffffffffu, tx, i, LPB), ay = __shfl_sync(0xffffffffu, ty, i, LPB);
-                        const float au = __shfl_sync(0xffffffffu, u, i, LPB), ahx = __shfl_sync(0xffffffffu, hx, i, LPB);
-                        const float ahy = __shfl_sync(0xffffffffu, hy, i, LPB);
-                        if (q * LPB + i < n) {
-                            xbx += ax;
-                            xby += ay;
-                            vbx = __fmaf_rn(au, ahx, vbx);
-                            vby = __fmaf_rn(au, ahy, vby);
-                        }
+                for (int i = 0; i < LPB; i++) {
+                    const float ax = __shfl_sync(0xffffffffu, t.tx, i, LPB), ay = __shfl_sync(0xffffffffu, t.ty, i, LPB);
+                    const float au = __shfl_sync(0xffffffffu, t.u, i, LPB), ahx = __shfl_sync(0xffffffffu, t.hx, i, LPB);
+                    const float ahy = __shfl_sync(0xffffffffu, t.hy, i, LPB);
+                    if (q * LPB + i < n) {
+                        xbx += ax;
+                        xby += ay;
+                        vbx = __fmaf_rn(au, ahx, vbx);
+                        vby = __fmaf_rn(au, ahy, vby);
                     }
                 }
             }
+        };
+        // the listed pairs [0, n) of every bead, two rounds of its lanes at a time (two independent chains a lane)
+        auto evaluate = [&](int n) {
+            __syncwarp();
+            const int rounds = (__reduce_max_sync(0xffffffffu, n) + LPB - 1) / LPB;
+            int q = 0;
+            for (; q + 1 < rounds; q += 2) {
+                const Terms t0 = pair(q * LPB + sub, n), t1 = pair((q + 1) * LPB + sub, n);
+                add(t0, q, n);
+                add(t1, q + 1, n);
+            }
+            if (q < rounds) add(pair(q * LPB + sub, n), q, n);
             __syncwarp();
         };
         // each lane marks the hits of its part of the slots in a word; then the bead's hits are listed in order
@@ -819,12 +835,12 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
     // Lanes per bead and CTAs an SM: as many lanes as keep all tasks on the GPU at once (a small box is latency), then
     // few, whose lanes wait less for the fullest list.  us a launch with (lanes, CTAs an SM), density 4:
     //   beads      (8, 2)  (4, 2)  (4, 3)  (2, 2)  (2, 4)
-    //   4,096         9.9    12.8    13.2    19.2    21.2
-    //   16,384       15.2    14.2    14.6    19.7    21.8
-    //   25,600       20.3    21.6    16.8    22.6    25.0
-    //   36,864       24.3    21.1    25.4    21.5    23.7
-    //   131,044      66.7    54.2    52.3    54.6    53.4
-    //   1,048,576   491     385     341     347     311
+    //   4,096         9.6    12.3    12.7    18.8    20.0
+    //   16,384       15.3    13.8    14.2    18.8    20.2
+    //   25,600       20.0    20.7    16.3    20.7    22.1
+    //   36,864       24.4    20.8    24.6    21.0    22.3
+    //   131,044      67.4    52.4    50.5    52.2    48.8
+    //   1,048,576   492     378     342     331     290
     const bool update = up && !mol;  // the branched shapes add their share first
     const AdjUpdate none{};
     auto go = [&](auto kern, int lpb, int per_sm) {
