@@ -116,7 +116,8 @@ struct dpd_handle {
     // staging for state in/out
     char *stage = nullptr;
     int dev = 0;                // the device the handle was made on
-    // pinned host memory the device writes its status and stats rows into (no staging on the way back)
+    // where copies of the device's status and of a stats row arrive (pageable: pinned memory saves a call 1-2 us and
+    // costs the handle 2.5 ms to make)
     struct HostSide {
         DevStatus st;
         unsigned long long row[OBS_N];
@@ -358,7 +359,7 @@ static void free_all(dpd_handle *h) {
     free_adj(h);
     for (void *p : h->allocs) cudaFree(p);
     h->allocs.clear();
-    if (h->host) cudaFreeHost(h->host);
+    delete h->host;
     h->host = nullptr;
     if (h->s) cudaStreamDestroy(h->s);
 }
@@ -555,7 +556,7 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
 
     choose_tile(h);
     CK(cudaGetDevice(&h->dev));
-    CK(cudaHostAlloc((void **)&h->host, sizeof *h->host, cudaHostAllocDefault));
+    h->host = new dpd_handle::HostSide();
     // the handle's arrays, carved from one allocation that is cleared as a whole
     std::vector<std::pair<void **, size_t>> plan;
     auto want = [&](auto **q, size_t count) { plan.push_back({(void **)q, count * sizeof(**q)}); };
