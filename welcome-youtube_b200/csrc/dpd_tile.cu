@@ -254,7 +254,7 @@ __device__ void tile_pairs(TB &S, uint32_t *q, int *next_chunk, int first, const
             len = src_ranges(S, s, v, LH, tw, th, r1s, len1, s2m);
         }
         const int maxlen = __reduce_max_sync(0xffffffffu, len);
-        // this round's first candidate in either range as a byte offset, and how many are left in the first and in all
+        // the first candidates of these four in either range as a byte offset, and how many are left in the first and in all
         int o1 = 8 * r1s, o2 = 8 * s2m, left1 = len1, left = len;
         const uint32_t s8 = (uint32_t)s << 19;
         for (int k = 0; k < maxlen; k += 4) {
@@ -382,7 +382,7 @@ __device__ void tile_direct(const Bufs &b, int cur, const RepDev &R, const TileD
     for (int c = 1; c <= td.w; c++) {
         const int gx = td.cx0 + c - 1, g0 = cs[gx * ncy + td.cy0], g1 = cs[gx * ncy + td.cy0 + td.h];
         for (int base = g0; base < g1; base += blockDim.x) {
-            RowAcc acc;  // this round's row terms
+            RowAcc acc;  // the row terms of these beads
             const int g = base + tid;
             const bool act = g < g1;
             uint32_t key = 0;
@@ -450,7 +450,7 @@ __device__ __forceinline__ void tile_epilogue(const Bufs &b, int cur, const RepD
     const int e0 = S.lcs[LH + 1], e1 = S.lcs[td.w * LH + td.h + 1];
     const float2 *__restrict__ gpos = b.pos[cur];
     for (int base = e0; base < e1; base += EPI_ITEMS * blockDim.x) {
-        RowAcc acc;  // this round's row terms
+        RowAcc acc;  // the row terms of these beads
         int gg[EPI_ITEMS];
         bool own[EPI_ITEMS];
 #pragma unroll

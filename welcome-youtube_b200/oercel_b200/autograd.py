@@ -11,8 +11,8 @@ of the repulsions a_ij, the friction gamma, the bond constant k_bond and,
 optionally, the start state, for every replica r of an Engine.  Its value is
 the smoothed pair-distribution loss of dpd_window_loss; its gradient is the
 window adjoint (dpd_window_adjoint / dpd_window_adjoint_state: the pair noise
-replayed from its key, checkpoints every `ckpt` steps, each segment recomputed
-in reverse).  Because the adjoint needs the forward pass anyway, the forward
+replayed from its key; configurations that do not fit in memory are stepped
+again from checkpoints, see Engine.set_window_memory).  Because the adjoint needs the forward pass anyway, the forward
 of this Function runs the adjoint at once when any input requires a gradient
 and keeps the result for backward; with no gradient wanted it runs the plain
 window.  Inputs:
