@@ -469,7 +469,7 @@ DPD_API int dpd_window_adjoint(dpd_handle *h, int64_t nsteps, int32_t ckpt_every
 /* The memory the windows of this handle may take for checkpoints and
  * configurations, in bytes, where that is more than ckpt_every asks for (0:
  * never more than that; negative: the default, a thirty-second of the device's
- * memory while four times that is free). */
+ * memory while four times that is free).  Releases the storage held. */
 DPD_API int dpd_set_window_memory(dpd_handle *h, int64_t bytes);
 /* dpd_window_adjoint plus the cotangents of the window's start state: the
  * loss's gradient with respect to the positions (xbar), the stored half-step

@@ -1905,6 +1905,8 @@ static int window_impl(dpd_handle *h, int64_t nsteps, int32_t ckpt, const dpd_rd
 
 extern "C" int dpd_set_window_memory(dpd_handle *h, int64_t bytes) {
     if (!h) return fail(DPD_E_ARG, "null handle");
+    CK(cudaStreamSynchronize(h->s));
+    free_adj(h);  // what an earlier limit allowed
     h->window_mem = bytes < 0 ? -1 : bytes;
     return DPD_OK;
 }
