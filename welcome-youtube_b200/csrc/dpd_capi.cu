@@ -429,17 +429,22 @@ static void choose_tile(dpd_handle *h) {
         }
 }
 
-// the exclusive scan of the cell counts, in the form the handle's tuning picked
-static void enqueue_scan(dpd_handle *h, const Bufs &b, bool step_inc) {
-    if (h->sort_mode == 1) launch_scan_lb(b, h->C, step_inc, h->s);
-    else launch_scan(b, h->C, step_inc, h->s);
+// The kernels of the cell sort, from the handle's sort_mode and what its boxes
+// allow: scan of the counts in two passes or in one, placement and fix-up; a
+// block-local scan whose prefixes placement and fix-up add; or the bins.
+enum class SortForm { TWO_PASS, LOOK_BACK, PREFIXES, BINS };
+
+static SortForm sort_form(const dpd_handle *h) {
+    if (h->sort_mode == 1) return SortForm::LOOK_BACK;
+    if (h->sort_mode == 0) return SortForm::TWO_PASS;
+    if (h->bins) return SortForm::BINS;
+    return sort_pfx_fits(h->C) ? SortForm::PREFIXES : SortForm::TWO_PASS;
 }
 
-// the sort of the counted keys into cell order (cell starts, src, dest)
-// b with the counts of buffer parity cur and, in sort_mode 2, the bins
+// b with the counts of buffer parity cur and, for the sort from bins, the bins
 static Bufs at_parity(const dpd_handle *h, Bufs b, int cur) {
     b.count = h->count2[cur];
-    b.bins = h->sort_mode == 2 ? h->bins : nullptr;
+    b.bins = sort_form(h) == SortForm::BINS ? h->bins : nullptr;
     return b;
 }
 
@@ -471,17 +476,19 @@ static void enqueue_cell_sort(dpd_handle *h, const Bufs &b0, int cur, bool step_
         head.stir = b.stir;
         head.nstir = h->nrep;
     }
-    if (b.bins) {
+    const SortForm form = sort_form(h);
+    if (form == SortForm::BINS) {
         launch_sort_bins(b, h->count2[cur ^ 1], h->C, step_inc, h->d_rep, h->d_cch, h->ncch, -1, head, h->s);
         return;
     }
-    if (h->sort_mode == 2 && sort_pfx_fits(h->C)) {
+    if (form == SortForm::PREFIXES) {
         launch_sort_pfx(b, h->C, step_inc, h->d_bch, h->nbch, h->d_cch, h->ncch, -1, head, h->s);
         return;
     }
     if (row.rep >= 0) launch_row_collect(b, row, h->s);
     clear_stir(h, b);
-    enqueue_scan(h, b, step_inc);
+    if (form == SortForm::LOOK_BACK) launch_scan_lb(b, h->C, step_inc, h->s);
+    else launch_scan(b, h->C, step_inc, h->s);
     launch_place(b, h->d_bch, h->nbch, h->s);
     launch_cellfix(b, h->d_cch, h->ncch, h->s);
 }
@@ -1156,9 +1163,10 @@ extern "C" int dpd_set_graph_steps(dpd_handle *h, int32_t steps) {
 
 // One step launched kernel by kernel with CUDA events between the launches on
 // the handle's stream; ms[k] = device time of kernel k (scan1 (the whole scan
-// with sort_mode 1, the block-local scan with 2; 0 ms where the sort is one
-// kernel), scan2 (0 ms with sort_mode 1 and 2), place (0 ms with bins), cellfix, permute, [2 chemistry], [catalyst check + its sort], forces).  The
-// step is a real step; on a step with a catalyst check the first entry is the
+// in one pass, or the block-local one; 0 ms where the sort is one kernel),
+// scan2 (0 ms but for the scan in two passes), place (0 ms with bins), cellfix,
+// permute, [2 chemistry], [catalyst check + its sort], forces).  The step is a
+// real step; on a step with a catalyst check the first entry is the
 // step counter's kernel, the next three are not launched (0 ms) and the
 // permute keeps the slot order.
 extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *n_out) {
@@ -1173,25 +1181,26 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
     CK(cudaEventRecord(ev[k++], h->s));
     const Bufs sb = at_parity(h, h->b, h->cur);
     uint32_t *other = h->count2[h->cur ^ 1];
-    const bool pfx = h->sort_mode == 2 && sort_pfx_fits(h->C);
+    const SortForm form = sort_form(h);
+    const bool bins = form == SortForm::BINS, pfx = form == SortForm::PREFIXES;
     if (!cat) {
-        if (sb.bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 0, StepHead(), h->s);
+        if (bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 0, StepHead(), h->s);
         else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 0, StepHead(), h->s);
-        else if (h->sort_mode == 1) launch_scan_lb(sb, h->C, true, h->s);
+        else if (form == SortForm::LOOK_BACK) launch_scan_lb(sb, h->C, true, h->s);
         else launch_scan_part(sb, h->C, true, 1, h->s);
     } else {
         launch_step_begin(h->b, h->nrep, h->s);
     }
     CK(cudaEventRecord(ev[k++], h->s));
-    if (!cat && h->sort_mode == 0) launch_scan_part(sb, h->C, true, 2, h->s);
+    if (!cat && form == SortForm::TWO_PASS) launch_scan_part(sb, h->C, true, 2, h->s);
     CK(cudaEventRecord(ev[k++], h->s));
-    if (!cat && !sb.bins) {
+    if (!cat && !bins) {
         if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 1, StepHead(), h->s);
         else launch_place(sb, h->d_bch, h->nbch, h->s);
     }
     CK(cudaEventRecord(ev[k++], h->s));
     if (!cat) {
-        if (sb.bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 1, StepHead(), h->s);
+        if (bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 1, StepHead(), h->s);
         else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 2, StepHead(), h->s);
         else launch_cellfix(sb, h->d_cch, h->ncch, h->s);
     }
@@ -1434,9 +1443,9 @@ extern "C" int dpd_get_rng(dpd_handle *h, int32_t r, uint64_t *state) {
 
 extern "C" int dpd_kernels_per_step(const dpd_handle *h, int32_t *n_plain, int32_t *n_chem) {
     if (!h) return fail(DPD_E_ARG, "null handle");
-    // the scan, placement and fix-up of the sort mode, permute, forces (+ the chemistry kernels)
-    const int sort = h->sort_mode == 0 || (h->sort_mode == 2 && !sort_pfx_fits(h->C)) ? 4
-                     : h->sort_mode == 2 && h->bins ? (sort_bins_one(h->C) ? 1 : 2) : 3;
+    // the scan, placement and fix-up of the sort, permute, forces (+ the chemistry kernels)
+    const SortForm form = sort_form(h);
+    const int sort = form == SortForm::TWO_PASS ? 4 : form == SortForm::BINS ? (sort_bins_one(h->C) ? 1 : 2) : 3;
     if (n_plain) *n_plain = sort + 2 + (h->any_lipid ? chem_kernel_count() : 0);
     if (n_chem) *n_chem = chem_kernel_count();
     return DPD_OK;
