@@ -1,0 +1,32 @@
+"""The autotuner's choices on an engine whose kernel times are given."""
+import pytest
+
+from oercel_b200.autotune import autotune
+
+
+class Timed:
+    """kernel times of a step: the sort's four, permute, forces"""
+    n_beads = [4096]
+
+    def __init__(self, sort, forces):
+        self.sort, self.forces, self.t = sort, forces, dict(sort_mode=2, tile_w=8)
+
+    def set_tuning(self, **kv):
+        self.t.update(kv)
+
+    def tuning(self):
+        return dict(self.t)
+
+    def profile_step(self):
+        m = self.t["sort_mode"]
+        return [*self.sort[m], 5.0, self.forces[m] * (1.0 if self.t["tile_w"] == 4 else 2.0)]
+
+
+@pytest.mark.parametrize("forces,want", [([20.0, 20.0, 24.0], 1), ([20.0, 20.0, 20.5], 2), ([20.0, 25.0, 25.0], 0)])
+def test_sort_is_judged_with_the_forces_it_bins_in(forces, want):
+    """mode 2 moves a part of the sort into the force kernel: its own kernels alone are always the fewest here"""
+    sort = [[3.0, 2.0, 2.0, 2.0], [3.0, 0.0, 2.0, 2.0], [0.0, 0.0, 0.0, 4.5]]
+    e = Timed(sort, forces)
+    out = autotune(e, candidates=[dict(tile_w=2), dict(tile_w=4)], use_cache=False)
+    assert out["tuning"] == dict(sort_mode=want, tile_w=4)
+    assert out["sort_ms"] == sum(sort[want])
