@@ -30,3 +30,21 @@ def test_sort_is_judged_with_the_forces_it_bins_in(forces, want):
     out = autotune(e, candidates=[dict(tile_w=2), dict(tile_w=4)], use_cache=False)
     assert out["tuning"] == dict(sort_mode=want, tile_w=4)
     assert out["sort_ms"] == sum(sort[want])
+
+
+class Shaped(Timed):
+    """the force kernel's time by tile shape"""
+
+    def __init__(self, best):
+        super().__init__([[1.0] * 4] * 3, None)
+        self.best = best
+        self.t = dict(force_kernel=0, tile_w=7, tile_h=12, tile_threads=256, sort_mode=2)
+
+    def profile_step(self):
+        return [1.0, 1.0, 1.0, 1.0, 5.0, 20.0 if (self.t["tile_w"], self.t["tile_h"]) == self.best else 25.0]
+
+
+@pytest.mark.parametrize("best", [(7, 12), (10, 18)])
+def test_the_engines_own_shape_is_a_candidate(best):
+    out = autotune(Shaped(best), use_cache=False)
+    assert (out["tuning"]["tile_w"], out["tuning"]["tile_h"]) == best

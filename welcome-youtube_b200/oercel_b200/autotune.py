@@ -67,7 +67,10 @@ def autotune(engine, repeats=3, candidates=None, cache_path=None, use_cache=True
         engine.set_tuning(**cache[key]["tuning"])
         return cache[key]
     best, timings = None, []
-    for cand in candidates or FORCE_CANDIDATES:
+    # the engine's own choice first: its tile shape follows the boxes' sizes and is often none of the list's
+    now = engine.tuning()
+    own = {k: now[k] for k in ("force_kernel", "tile_w", "tile_h", "tile_threads")}
+    for cand in candidates or [own, *FORCE_CANDIDATES]:
         try:
             engine.set_tuning(**cand)
         except Exception:
