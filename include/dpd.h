@@ -461,8 +461,9 @@ DPD_API int dpd_window_loss(dpd_handle *h, int64_t nsteps, const dpd_rdf_spec *s
  * again from checkpoints: at most the memory of a checkpoint every ckpt_every
  * steps and ckpt_every configurations (about 44 and 33 bytes a bead each), or,
  * where that is more, a thirty-second of the device's (see
- * dpd_set_window_memory); the results do not depend on it.  The storage stays
- * with the handle.  grad: nrep x DPD_NGRAD.  The handle ends at the end of the
+ * dpd_set_window_memory), and about 104 bytes a bead of scratch; the results do
+ * not depend on it.  The storage stays with the handle: as much as the largest
+ * of its windows took.  grad: nrep x DPD_NGRAD.  The handle ends at the end of the
  * window, as after dpd_window_loss. */
 DPD_API int dpd_window_adjoint(dpd_handle *h, int64_t nsteps, int32_t ckpt_every, const dpd_rdf_spec *spec,
                                const double *target, double *loss, double *grad, double *rdf_out);

@@ -10,6 +10,7 @@
 #include <initializer_list>
 #include <string>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/dpd.h"
@@ -62,7 +63,8 @@ struct AdjBufs {
     float2 *vh[2], *f[2];       // the half-step velocities and forces of a segment's steps, in turn
     float2 *X[2], *V[2], *F[2]; // the adjoint state of one configuration and of the one before, in turn
     float2 *xb, *vb;
-    float2 *G;                  // the loss's own x_bar of rdf_batch() configurations
+    float2 *G;                  // the loss's own x_bar of ng configurations
+    int ng = 0;
     double *hist, *wgt, *grad;
     double *gsum;            // per replica: the sum of the x cotangents (stirring)
     long long *stir;         // per replica: the stirring sums of a segment's steps
@@ -107,12 +109,10 @@ struct dpd_handle {
     bool any_mol = false;       // some replica has branched lipids (k_mol_forces)
     int stream_grid = 1;        // blocks per replica of the catalyst stream kernel
     int64_t cat_period = 0;
-    // reverse-mode storage, grown on demand (full checkpoints, the states of one
-    // recomputed segment, adjoint arrays in gid order)
-    std::vector<void *> adj_allocs;
-    int adj_nck = 0, adj_nseg = 0, adj_nbin = 0;  // capacity of adj (0: none yet)
+    // reverse-mode storage (adj_layout)
+    char *adj_mem = nullptr;    // one allocation, laid out anew by each call that uses it
+    size_t adj_bytes = 0;
     int64_t window_mem = -1;    // dpd_set_window_memory (-1: the default rule)
-    AdjBufs adj;
     // staging for state in/out
     char *stage = nullptr;
     int dev = 0;                // the device the handle was made on
@@ -348,10 +348,9 @@ static void drop_graphs(dpd_handle *h) {
 }
 
 static void free_adj(dpd_handle *h) {
-    for (void *p : h->adj_allocs) cudaFree(p);
-    h->adj_allocs.clear();
-    h->adj_nck = h->adj_nseg = h->adj_nbin = 0;
-    h->adj = AdjBufs();
+    if (h->adj_mem) cudaFree(h->adj_mem);
+    h->adj_mem = nullptr;
+    h->adj_bytes = 0;
 }
 
 static void free_all(dpd_handle *h) {
@@ -1509,37 +1508,20 @@ extern "C" int dpd_set_params(dpd_handle *h, int32_t r, const dpd_params *p) {
 
 // ---------------------------------------------------------------- reverse mode
 
+// an array's place in the storage of the reverse mode
+static size_t adj_place(size_t bytes) { return (bytes + 64 + 255) & ~(size_t)255; }
 
-template <typename T>
-static int adj_alloc(dpd_handle *h, T **p, size_t count) {
-    void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, count * sizeof(T) + 64);
-    if (e != cudaSuccess) return fail(DPD_E_NOMEM, "cudaMalloc for the adjoint: %s", cudaGetErrorString(e));
-    h->adj_allocs.push_back(q);
-    *p = (T *)q;
-    return DPD_OK;
-}
-
-static int adj_setup(dpd_handle *h, int nck, int nseg, int nbin, AdjBufs &A) {
-    // storage kept on the handle and grown on demand: a window that fits reuses
-    // the buffers of the last one (freeing and allocating them every call costs a
-    // device synchronisation per buffer)
-    const int want_ck = nck, want_seg = nseg;
-    if (h->adj_nbin > 0 && nck <= h->adj_nck && nseg <= h->adj_nseg && nbin <= h->adj_nbin) {
-        A = h->adj;
-        A.ck.resize(want_ck);
-        A.seg.resize(want_seg);
-        return DPD_OK;
-    }
-    nck = std::max(nck, h->adj_nck);
-    nseg = std::max(nseg, h->adj_nseg);
-    nbin = std::max(nbin, h->adj_nbin);
-    free_adj(h);
+// the arrays of a reverse pass over nseg stored configurations after nck
+// checkpoints, with the loss's x_bar of ng configurations, laid out from base
+// on (or, base null, only measured); returns the bytes they take
+static size_t adj_layout(const dpd_handle *h, char *base, int nck, int nseg, int ng, int nbin, AdjBufs &A) {
     const size_t N = (size_t)h->N, C = (size_t)h->C;
+    size_t at = 0;
+    auto want = [&](auto **p, size_t count) {
+        *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base ? base + at : nullptr);
+        at += adj_place(count * sizeof(**p));
+    };
     A = AdjBufs();
-    // every buffer carved from one allocation (one cudaMalloc instead of a few hundred)
-    std::vector<std::pair<void **, size_t>> plan;
-    auto want = [&](auto **p, size_t count) { plan.push_back({(void **)p, count * sizeof(**p)}); };
     A.ck.resize(nck);
     for (auto &c : A.ck) {
         want(&c.pos, N);
@@ -1566,7 +1548,8 @@ static int adj_setup(dpd_handle *h, int nck, int nseg, int nbin, AdjBufs &A) {
         want(&A.V[k], N);
         want(&A.F[k], N);
     }
-    want(&A.G, N * std::min(nseg, rdf_batch(h->nbch)));
+    A.ng = ng;
+    want(&A.G, N * ng);
     want(&A.xb, N);
     want(&A.vb, N);
     want(&A.hist, (size_t)h->nrep * nbin);
@@ -1574,20 +1557,25 @@ static int adj_setup(dpd_handle *h, int nck, int nseg, int nbin, AdjBufs &A) {
     want(&A.grad, (size_t)h->nrep * DPD_NGRAD);
     want(&A.gsum, (size_t)h->nrep);
     want(&A.stir, (size_t)h->nrep);
-    size_t total = 0;
-    for (auto &q : plan) total += (q.second + 64 + 255) & ~(size_t)255;
-    char *base = nullptr;
-    TRY(adj_alloc(h, &base, total));
-    for (auto &q : plan) {
-        *q.first = base;
-        base += (q.second + 64 + 255) & ~(size_t)255;
+    return at;
+}
+
+// The storage stays with the handle: one allocation of the most that a call
+// needed, laid out anew by each call (an allocation per call would cost a
+// device synchronisation, and each call's arrays beside the last one's more
+// than either asked for).
+static int adj_setup(dpd_handle *h, int nck, int nseg, int ng, int nbin, AdjBufs &A) {
+    const size_t bytes = adj_layout(h, nullptr, nck, nseg, ng, nbin, A);
+    if (bytes > h->adj_bytes) {
+        free_adj(h);
+        const cudaError_t e = cudaMalloc(&h->adj_mem, bytes);
+        if (e != cudaSuccess) {
+            h->adj_mem = nullptr;
+            return fail(DPD_E_NOMEM, "cudaMalloc for the adjoint: %s", cudaGetErrorString(e));
+        }
+        h->adj_bytes = bytes;
     }
-    h->adj = A;
-    h->adj_nck = nck;
-    h->adj_nseg = nseg;
-    h->adj_nbin = nbin;
-    A.ck.resize(want_ck);
-    A.seg.resize(want_seg);
+    adj_layout(h, h->adj_mem, nck, nseg, ng, nbin, A);
     return DPD_OK;
 }
 
@@ -1684,23 +1672,31 @@ struct Window {
 //   a thirty-second of the device's memory, while four times that is free or
 //   held already (a failed allocation: the caller's interval), or what
 //   dpd_set_window_memory says.
+// The loss's x_bar of the configurations that its kernels take together counts
+// too; where it does not fit they take fewer, at least one (that one is scratch,
+// as the arrays of one configuration are).
 // A step made again costs a forward step: at 16,384 beads, a window of 200
 // steps with 70 differentiated, 60 of 260 steps were (the window and its gradient 8.2 ms,
 // 6.8 without); 24 boxes of 65,536, 70 of 250 differentiated, 50 of 300
 // (114.7 ms, 106.0 without, 3.8 GB of configurations).
 static int window_setup(dpd_handle *h, int ckpt, Window &w, AdjBufs &A) {
-    const size_t N = (size_t)h->N, C = (size_t)h->C;
-    const size_t ck_bytes = N * sizeof(float2) * 4 + N * sizeof(uint32_t) + N * sizeof(int2) + C * sizeof(int32_t);
-    const size_t seg_bytes = N * sizeof(float2) * 2 + N * sizeof(uint32_t) * 2 + N * sizeof(int2) + C * sizeof(int32_t);
-    const int64_t steps = w.nsteps - w.stop();
+    const size_t N = (size_t)h->N, cells = adj_place((size_t)(h->C + 1) * sizeof(int32_t));
+    const size_t vec = adj_place(N * sizeof(float2)), word = adj_place(N * sizeof(uint32_t));
+    const size_t ck_bytes = 5 * vec + word + cells, seg_bytes = 3 * vec + 2 * word + cells;
+    const size_t g_bytes = N * sizeof(float2);
+    const int64_t steps = w.nsteps - w.stop(), batch = std::min(rdf_batch(h->nbch), w.spec->last_steps);
     const size_t asked = (size_t)((w.nsteps + ckpt - 1) / ckpt) * ck_bytes + (size_t)ckpt * seg_bytes;
-    const size_t held = (size_t)h->adj_nck * ck_bytes + (size_t)h->adj_nseg * seg_bytes;
+    auto takes = [&](int nseg, int64_t len) {
+        return (size_t)nseg * ck_bytes + (size_t)len * seg_bytes + (size_t)std::min(len, batch) * g_bytes;
+    };
     size_t may = asked, free_now = 0, total = 0;
     if (h->window_mem >= 0) {
         may = std::max(may, (size_t)h->window_mem);
     } else {
+        const size_t scratch = adj_layout(h, nullptr, 0, 0, 0, w.spec->nbin, A);
+        const size_t held = h->adj_bytes > scratch ? h->adj_bytes - scratch : 0;
         may = std::max(may, held);
-        if (ck_bytes + (size_t)steps * seg_bytes > may) {
+        if (takes(1, steps) > may) {
             if (cudaMemGetInfo(&free_now, &total) != cudaSuccess) cudaGetLastError();
             may = std::max(may, std::min(total / 32, (free_now + held) / 4));
         }
@@ -1709,9 +1705,12 @@ static int window_setup(dpd_handle *h, int ckpt, Window &w, AdjBufs &A) {
         for (w.nseg = 1;; w.nseg++) {  // ends: segments of at most ckpt steps fit
             const int64_t len = (steps + w.nseg - 1) / w.nseg;
             w.len = (int)len;
-            if (len <= ckpt || (len <= INT_MAX && (size_t)w.nseg * ck_bytes + (size_t)len * seg_bytes <= may)) break;
+            if (len <= ckpt || (len <= INT_MAX && takes(w.nseg, len) <= may)) break;
         }
-        const int rc = adj_setup(h, w.nseg, w.len, w.spec->nbin, A);
+        const size_t states = (size_t)w.nseg * ck_bytes + (size_t)w.len * seg_bytes;
+        const size_t room = may > states ? (may - states) / g_bytes : 0;
+        const int ng = (int)std::max<size_t>(1, std::min(room, (size_t)std::min<int64_t>(w.len, batch)));
+        const int rc = adj_setup(h, w.nseg, w.len, ng, w.spec->nbin, A);
         if (rc != DPD_E_NOMEM || may == asked) return rc;
         cudaGetLastError();  // the failed allocation's
         may = asked;
@@ -1769,7 +1768,6 @@ static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const flo
     const size_t N = (size_t)h->N;
     const dpd_template *mol = h->any_mol ? h->b.mol : nullptr;
     const long long *base = w.fd ? &w.fd->base : nullptr;
-    const int batch = rdf_batch(h->nbch);
     int p = 0;  // which of X, V, F hold the adjoint state
     cudaMemsetAsync(A.X[0], 0, N * sizeof(float2), h->s);
     cudaMemsetAsync(A.V[0], 0, N * sizeof(float2), h->s);
@@ -1790,7 +1788,7 @@ static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const flo
             const bool in_loss = k >= first_loss;
             if (in_loss && (g0 < s || g0 - s >= ng)) {
                 g0 = s;
-                ng = (int)std::min<int64_t>(std::min(s, batch), k - first_loss + 1);
+                ng = (int)std::min<int64_t>(std::min(s, A.ng), k - first_loss + 1);
                 RdfViews views;
                 for (int u = 0; u < ng; u++) views.v[u] = seg_view(A, sg, s - u);
                 launch_rdf_vjp(views, ng, h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb, w.spec->nbin, rmax, sig,
@@ -1886,7 +1884,7 @@ static int window_impl(dpd_handle *h, int64_t nsteps, int32_t ckpt, const dpd_rd
     TRY(count_pairs(h, spec, npairs));
     AdjBufs A;
     Window w{nsteps, 0, 0, spec, h->step, nullptr};
-    TRY(backward ? window_setup(h, ckpt, w, A) : adj_setup(h, 0, 0, nb, A));
+    TRY(backward ? window_setup(h, ckpt, w, A) : adj_setup(h, 0, 0, 0, nb, A));
     if (!h->keys_valid) enqueue_next_keys(h);
     window_forward(h, A, w);
     CK(cudaGetLastError());
@@ -2084,7 +2082,7 @@ extern "C" int dpd_force_vjp(dpd_handle *h, int32_t r, int64_t step, const float
     const RepDev &R = h->rh[r];
     const size_t n = (size_t)R.n, N = (size_t)h->N, a = ((n * 4 + 255) / 256) * 256;
     AdjBufs A;
-    TRY(adj_setup(h, 0, 0, 1, A));
+    TRY(adj_setup(h, 0, 0, 0, 1, A));
     CK(cudaMemsetAsync(A.grad, 0, (size_t)h->nrep * DPD_NGRAD * sizeof(double), h->s));
     if (h->nrep > 1) CK(cudaMemsetAsync(A.F[0], 0, N * sizeof(float2), h->s));  // the other replicas' cotangents
     const float *sx = gx, *sy = gy;
