@@ -13,6 +13,8 @@
 #include <type_traits>
 #include <vector>
 
+#include <cuda.h>
+
 #include "../../include/dpd.h"
 #include "dpd_internal.h"
 
@@ -39,8 +41,10 @@ int lib_error(int code, const char *msg) {
 #define CK(call)                                                                                        \
     do {                                                                                                \
         cudaError_t e_ = (call);                                                                        \
-        if (e_ != cudaSuccess) return fail(DPD_E_CUDA, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), \
-                                           __FILE__, __LINE__);                                         \
+        if (e_ != cudaSuccess) {                                                                        \
+            cudaGetLastError(); /* a refused call's error is this call's, not the next one's */         \
+            return fail(DPD_E_CUDA, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+        }                                                                                               \
     } while (0)
 
 // reverse-mode storage (defined here: the handle keeps it between windows)
@@ -749,19 +753,44 @@ static int ensure_replica(const dpd_handle *h, int r) {
 
 // ---------------------------------------------------------------- state in/out
 
-// are all of these (null ones aside) memory of the handle's device, aligned for
-// its kernels?  They can then be read or written in place; anything else goes
-// through the staging arrays and copies that take any pointer.
-static bool on_device(const dpd_handle *h, std::initializer_list<const void *> ps, size_t align) {
-    bool ok = true;
-    for (const void *p : ps) {
-        if (!p || !ok) continue;
-        cudaPointerAttributes pa;
-        ok = (uintptr_t)p % align == 0 && cudaPointerGetAttributes(&pa, p) == cudaSuccess &&
-             pa.type == cudaMemoryTypeDevice && pa.device == h->dev;
+struct ArrayArg {
+    const void *p;
+    size_t bytes;
+};
+
+// Are all of these (null ones aside) arrays in one allocation each on the
+// handle's device, aligned for its kernels?  They can then be read or written
+// in place; anything else goes through the staging arrays and copies that take
+// any pointer, and that refuse an array which is shorter than the replica.
+static bool on_device(const dpd_handle *h, std::initializer_list<ArrayArg> args, size_t align) {
+    static const auto attributes = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &found) != cudaSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return (decltype(&cuPointerGetAttributes))f;
+    }();
+    if (!attributes) return false;
+    for (const ArrayArg &a : args) {
+        if (!a.p) continue;
+        unsigned type = 0, managed = 0;
+        int dev = -1;
+        CUdeviceptr start = 0;
+        size_t size = 0;
+        CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                      CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                      CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+        void *got[] = {&type, &managed, &dev, &start, &size};
+        if ((uintptr_t)a.p % align != 0 ||
+            attributes(sizeof(what) / sizeof(what[0]), what, got, (CUdeviceptr)a.p) != CUDA_SUCCESS ||
+            type != CU_MEMORYTYPE_DEVICE || managed || dev != h->dev)
+            return false;
+        const size_t at = (size_t)((CUdeviceptr)a.p - start);
+        if (at > size || size - at < a.bytes) return false;
     }
-    cudaGetLastError();
-    return ok;
+    return true;
 }
 
 extern "C" int dpd_set_state(dpd_handle *h, int32_t r, const float *x, const float *y, const float *vx,
@@ -776,7 +805,9 @@ extern "C" int dpd_set_state(dpd_handle *h, int32_t r, const float *x, const flo
     uint32_t *sg = (uint32_t *)(p + 4 * a);
     int32_t *sp = (int32_t *)(p + 5 * a), *sn = (int32_t *)(p + 6 * a);
     uint8_t *st = (uint8_t *)(p + 7 * a);
-    if (on_device(h, {x, y, vx, vy, gid, prev, next}, 4) && on_device(h, {type}, 1)) {
+    const size_t w = n * 4;
+    if (on_device(h, {{x, w}, {y, w}, {vx, w}, {vy, w}, {gid, w}, {prev, w}, {next, w}}, 4) &&
+        on_device(h, {{type, n}}, 1)) {
         launch_pack(h->b, h->cur, R.b0, (int)n, R.L, x, y, vx, vy, type, gid, prev, next, h->s);
     } else {
         CK(cudaMemcpyAsync(sx, x, n * 4, cudaMemcpyDefault, h->s));
@@ -810,7 +841,10 @@ extern "C" int dpd_get_state(dpd_handle *h, int32_t r, float *x, float *y, float
     TRY(ensure_replica(h, r));
     const RepDev &R = h->rh[r];
     const size_t n = (size_t)R.n, a = ((n * 4 + 255) / 256) * 256;
-    if (on_device(h, {x, y, vhx, vhy, vtx, vty, fx, fy, gid, prev, next}, 4) && on_device(h, {type}, 1)) {
+    const size_t w = n * 4;
+    if (on_device(h, {{x, w}, {y, w}, {vhx, w}, {vhy, w}, {vtx, w}, {vty, w}, {fx, w}, {fy, w}, {gid, w}, {prev, w},
+                      {next, w}}, 4) &&
+        on_device(h, {{type, n}}, 1)) {
         launch_unpack(h->b, h->cur, R.b0, (int)n, x, y, vhx, vhy, vtx, vty, fx, fy, type, gid, prev, next, h->s);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(h->s));
@@ -2086,7 +2120,7 @@ extern "C" int dpd_force_vjp(dpd_handle *h, int32_t r, int64_t step, const float
     CK(cudaMemsetAsync(A.grad, 0, (size_t)h->nrep * DPD_NGRAD * sizeof(double), h->s));
     if (h->nrep > 1) CK(cudaMemsetAsync(A.F[0], 0, N * sizeof(float2), h->s));  // the other replicas' cotangents
     const float *sx = gx, *sy = gy;
-    if (!on_device(h, {gx, gy}, 4)) {
+    if (!on_device(h, {{gx, n * 4}, {gy, n * 4}}, 4)) {
         sx = (float *)h->stage;
         sy = (float *)(h->stage + a);
         CK(cudaMemcpyAsync(h->stage, gx, n * 4, cudaMemcpyDefault, h->s));
@@ -2101,7 +2135,7 @@ extern "C" int dpd_force_vjp(dpd_handle *h, int32_t r, int64_t step, const float
     CK(cudaGetLastError());
     float *outs[4] = {xbar_x, xbar_y, vbar_x, vbar_y};
     float *st[4];
-    const bool direct = on_device(h, {xbar_x, xbar_y, vbar_x, vbar_y}, 4);
+    const bool direct = on_device(h, {{outs[0], n * 4}, {outs[1], n * 4}, {outs[2], n * 4}, {outs[3], n * 4}}, 4);
     for (int k = 0; k < 4; k++) st[k] = direct ? outs[k] : (float *)(h->stage + k * a);
     Bufs w = h->b;
     w.f[h->cur] = A.xb;
