@@ -481,7 +481,7 @@ static void enqueue_cell_sort(dpd_handle *h, const Bufs &b0, int cur, bool step_
     }
     const SortForm form = sort_form(h);
     if (form == SortForm::BINS) {
-        launch_sort_bins(b, h->count2[cur ^ 1], h->C, step_inc, h->d_rep, h->d_cch, h->ncch, -1, head, h->s);
+        launch_sort_bins(b, h->count2[cur ^ 1], h->C, step_inc, h->d_cch, h->ncch, -1, head, h->s);
         return;
     }
     if (form == SortForm::PREFIXES) {
@@ -504,9 +504,9 @@ static Bufs plain_counts(const dpd_handle *h) {
     return b;
 }
 
-// clear the counts (both parities) and count the current (or the next) positions of buffer cur of b
+// clear the counts (both parities, and the crowded cells' lists) and count the current (or the next) positions of buffer cur of b
 static void enqueue_keys(dpd_handle *h, const Bufs &b0, int cur, bool next) {
-    cudaMemsetAsync(h->count2[0], 0, 2 * (size_t)(h->C + 64) * sizeof(uint32_t), h->s);
+    cudaMemsetAsync(h->count2[0], 0, (h->bins ? 3 : 2) * (size_t)(h->C + 64) * sizeof(uint32_t), h->s);
     launch_keys(at_parity(h, b0, cur), cur, h->d_rep, h->d_bch, h->nbch, next, h->s);
 }
 
@@ -587,15 +587,19 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
     want(&b.fill, C + 4);
     want(&b.src, N);
     want(&b.dest, N);
-    // (both parities in one array, cleared together; each begins on a 16-byte boundary)
-    want(&h->count2[0], 2 * (C + 64));
     // Bins up to ten beads a cell: a row of 32 is then too short for about one cell in 10^8 of a random soup (denser
     // boxes keep the placement kernel); and up to 196,608 cells, where the kernel saved is worth more than the force
     // kernel's wait for the counts: 13.3 against 18.3 us a step at 1,024 cells, 21.4 (26.1) at 16,384, 44.0 (47.0) at
     // 65,536, 88.9 (91.0) at 176,400, but 126.2 (120.7) at 262,144.
     double dense = 0.0;
     for (int r = 0; r < nrep; r++) dense = std::max(dense, (double)h->rh[r].n / h->rh[r].ncell);
-    if (dense <= 10.0 && C <= 196608) want(&h->bins, C * BIN_CAP);
+    const bool bins = dense <= 10.0 && C <= 196608;
+    if (bins) {
+        want(&h->bins, C * BIN_CAP);
+        want(&b.crowd_next, N);
+    }
+    // (both parities and the crowded cells in one array, cleared together; each begins on a 16-byte boundary)
+    want(&h->count2[0], (bins ? 3 : 2) * (C + 64));
     want(&b.cstart, C + 4);
     want(&b.bsum, C / SCAN_PER_BLOCK + 2);
     want(&b.scan_state, C / SCAN_PER_BLOCK + 2);
@@ -660,6 +664,7 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
         base += (q.second + 64 + 255) & ~(size_t)255;
     }
     h->count2[1] = h->count2[0] + (C + 64) / 4 * 4;
+    if (bins) b.crowd = (int32_t *)(h->count2[1] + (C + 64) / 4 * 4);
     b.jump = dj;
     b.mol = dm;
     CK(cudaMemcpy(h->d_rep, h->rh.data(), nrep * sizeof(RepDev), cudaMemcpyHostToDevice));
@@ -1217,7 +1222,7 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
     const SortForm form = sort_form(h);
     const bool bins = form == SortForm::BINS, pfx = form == SortForm::PREFIXES;
     if (!cat) {
-        if (bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 0, StepHead(), h->s);
+        if (bins) launch_sort_bins(sb, other, h->C, true, h->d_cch, h->ncch, 0, StepHead(), h->s);
         else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 0, StepHead(), h->s);
         else if (form == SortForm::LOOK_BACK) launch_scan_lb(sb, h->C, true, h->s);
         else launch_scan_part(sb, h->C, true, 1, h->s);
@@ -1233,7 +1238,7 @@ extern "C" int dpd_profile_step(dpd_handle *h, float *ms, int32_t cap, int32_t *
     }
     CK(cudaEventRecord(ev[k++], h->s));
     if (!cat) {
-        if (bins) launch_sort_bins(sb, other, h->C, true, h->d_rep, h->d_cch, h->ncch, 1, StepHead(), h->s);
+        if (bins) launch_sort_bins(sb, other, h->C, true, h->d_cch, h->ncch, 1, StepHead(), h->s);
         else if (pfx) launch_sort_pfx(sb, h->C, true, h->d_bch, h->nbch, h->d_cch, h->ncch, 2, StepHead(), h->s);
         else launch_cellfix(sb, h->d_cch, h->ncch, h->s);
     }

@@ -343,13 +343,14 @@ __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 // Count a bead (slot) into its next cell and, with bins, put it into the
 // cell's row at the place the count gives (in arrival order; k_binfix puts the
-// row in slot order).  Without bins no value is returned: the add is
-// fire-and-forget.
+// row in slot order), or, past the row's end, into the cell's list.  Without
+// bins no value is returned: the add is fire-and-forget.
 __device__ __forceinline__ void count_key(const Bufs &b, uint32_t key, int slot, bool active) {
     if (!active) return;
     if (b.bins) {
         const uint32_t r = atomicAdd(b.count + key, 1u);
         if (r < BIN_CAP) b.bins[(size_t)key * BIN_CAP + r] = slot;
+        else b.crowd_next[slot] = atomicExch(b.crowd + key, slot + 1);
     } else {
         atomicAdd(b.count + key, 1u);
     }

@@ -163,6 +163,7 @@ struct Bufs {
     int32_t *src, *dest;
     uint32_t *count;            // the counts the next force kernel makes or the next sort reads (one array per parity)
     int32_t *bins;              // per cell BIN_CAP slots: the beads counted into it, or null (see k_binfix)
+    int32_t *crowd, *crowd_next;  // per cell: slot + 1 of the last bead past its row (0: none); per slot: the one before
     int32_t *cstart;            // C + 1
     int32_t *bsum;              // scan block totals
     unsigned long long *scan_state;   // single-pass scan: per block (epoch | flag | value), see k_scan_lb
@@ -256,8 +257,8 @@ void launch_row_collect(const Bufs &b, const RowOut &row, cudaStream_t s);
 // the sort from the bins the force kernel filled: the scan of the counts (within the one kernel up to
 // BIN_SCAN_CELLS cells) and every cell's row in slot order; other: the counts of the other parity, cleared
 bool sort_bins_one(int64_t C);
-void launch_sort_bins(const Bufs &b, uint32_t *other, int64_t C, bool step_inc, const RepDev *rep, const Chunk *cch,
-                      int ncch, int part, const StepHead &head, cudaStream_t s);
+void launch_sort_bins(const Bufs &b, uint32_t *other, int64_t C, bool step_inc, const Chunk *cch, int ncch, int part,
+                      const StepHead &head, cudaStream_t s);
 void launch_place(const Bufs &b, const Chunk *bch, int nbch, cudaStream_t s);
 void launch_cellfix(const Bufs &b, const Chunk *cch, int ncch, cudaStream_t s);
 void launch_permute(const Bufs &b, int cur, const RepDev *rep, const Chunk *bch, int nbch, PermuteMode mode,

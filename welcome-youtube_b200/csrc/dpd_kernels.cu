@@ -411,6 +411,21 @@ __device__ __forceinline__ void fix_cell(int32_t *__restrict__ src, int32_t *__r
         }
 }
 
+// a crowded cell: in-place insertion sort in global memory
+__device__ __forceinline__ void fix_crowded(int32_t *src, int32_t *dest, int s, int m, DevStatus *status) {
+    atomicMax(&status->bigcell, (unsigned)m);
+    for (int k = 1; k < m; k++) {
+        const int t = src[s + k];
+        int q = k - 1;
+        while (q >= 0 && src[s + q] > t) {
+            src[s + q + 1] = src[s + q];
+            q--;
+        }
+        src[s + q + 1] = t;
+    }
+    for (int k = 0; k < m; k++) dest[src[s + k]] = s + k;
+}
+
 // Beads that land in one cell keep their old slot order (the reference's
 // stable counting sort, oercel.c:832-933): the atomics gave each bead some
 // place in its cell; here every cell orders its beads by old slot.
@@ -426,18 +441,7 @@ __device__ __forceinline__ void cellfix_range(const Bufs &b, int s, int m) {
     } else if (m <= 16) {
         fix_cell<16>(b.src, b.dest, s, m);
     } else {
-        // crowded cell: in-place insertion sort in global memory
-        atomicMax(&b.status->bigcell, (unsigned)m);
-        for (int k = 1; k < m; k++) {
-            const int t = b.src[s + k];
-            int q = k - 1;
-            while (q >= 0 && b.src[s + q] > t) {
-                b.src[s + q + 1] = b.src[s + q];
-                q--;
-            }
-            b.src[s + q + 1] = t;
-        }
-        for (int k = 0; k < m; k++) b.dest[b.src[s + k]] = s + k;
+        fix_crowded(b.src, b.dest, s, m, b.status);
     }
 }
 
@@ -478,9 +482,9 @@ __global__ void __launch_bounds__(CELL_TPB) k_cellfix(Bufs b, const Chunk *__res
 // also adds up the counts before its own (up to BIN_SCAN_CELLS cells, at most
 // 128 KB read per CTA, from L2), so that the sort of a small handle is one
 // kernel; else k_scan1<true> left the cells' starts within its blocks and the
-// block totals.  A cell with more beads than its row holds (at the densities
-// that use bins, none in 10^8 cells) is gathered from the keys of its replica
-// by the whole CTA, once for all such cells it has.
+// block totals.  A cell with more beads than its row holds (none in 10^8 cells
+// of a soup at the densities that use bins, but any state can be set) finds the
+// others in its list.
 // What bounds it: latency (a small box: starts, row, stores), else HBM and L2
 // sectors: a row is read 32 bytes at a time, one or two sectors a cell.
 #define BIN_SCAN_CELLS 32768
@@ -508,10 +512,23 @@ __device__ __forceinline__ void bin_cell(const Bufs &b, int cell, int s, int n) 
         }
 }
 
+// a cell of n > BIN_CAP beads: its row, then its list (the last bead to arrive first), which is left empty
+__device__ __noinline__ void crowded_cell(int32_t *src, int32_t *dest, const int32_t *row, int32_t *last,
+                                          const int32_t *next, int s, int n, DevStatus *status) {
+    for (int k = 0; k < BIN_CAP; k++) src[s + k] = row[k];
+    int q = *last;
+    *last = 0;
+    for (int k = n - 1; k >= BIN_CAP; k--) {
+        src[s + k] = q - 1;
+        q = next[q - 1];
+    }
+    fix_crowded(src, dest, s, n, status);
+}
+
 template <bool ONE>
 __global__ void __launch_bounds__(CELL_TPB) k_binfix(Bufs b, uint32_t *__restrict__ other,
-                                                     const RepDev *__restrict__ reps, const Chunk *__restrict__ ch,
-                                                     int nb, long long C, int step_inc, StepHead head) {
+                                                     const Chunk *__restrict__ ch, int nb, long long C, int step_inc,
+                                                     StepHead head) {
     const bool extra = head.row.rep >= 0 && blockIdx.x == gridDim.x - 1;  // the CTA that collects the stats row
     const Chunk c = ch[extra ? 0 : blockIdx.x];
     pdl_begin();
@@ -523,10 +540,8 @@ __global__ void __launch_bounds__(CELL_TPB) k_binfix(Bufs b, uint32_t *__restric
         for (int k = (int)threadIdx.x; k < head.nstir; k += CELL_TPB) head.stir[k] = 0;
     __shared__ int pfx[ONE ? 1 : PFX_MAX];
     __shared__ int red[CELL_TPB / 32];
-    __shared__ int ncrowd, cursor[CELL_TPB];
     const int tid = (int)threadIdx.x, cell = c.begin + tid;
     const bool act = cell < c.end;
-    if (tid == 0) ncrowd = 0;
     int s = 0, n = 0;
     if (ONE) {
         int part = 0;
@@ -561,9 +576,10 @@ __global__ void __launch_bounds__(CELL_TPB) k_binfix(Bufs b, uint32_t *__restric
     if (act) {
         b.cstart[cell] = s;
         if (cell + 1 == C) b.cstart[C] = s + n;
-        if (n > 16) {
-            if (n <= BIN_CAP) bin_cell<32>(b, cell, s, n);
-            else atomicAdd(&ncrowd, 1);
+        if (n > BIN_CAP) {
+            crowded_cell(b.src, b.dest, b.bins + (size_t)cell * BIN_CAP, b.crowd + cell, b.crowd_next, s, n, b.status);
+        } else if (n > 16) {
+            bin_cell<32>(b, cell, s, n);
         } else if (n > 8) {
             bin_cell<16>(b, cell, s, n);
         } else if (n > 4) {
@@ -572,17 +588,6 @@ __global__ void __launch_bounds__(CELL_TPB) k_binfix(Bufs b, uint32_t *__restric
             bin_cell<4>(b, cell, s, n);
         }
     }
-    __syncthreads();
-    if (ncrowd == 0) return;
-    cursor[tid] = n > BIN_CAP ? s : -1;
-    __syncthreads();
-    const RepDev &R = reps[c.rep];
-    for (int i = R.b0 + tid; i < R.b0 + R.n; i += CELL_TPB) {
-        const int k = (int)b.key[i] - c.begin;
-        if (k >= 0 && k < c.end - c.begin && cursor[k] >= 0) b.src[atomicAdd(&cursor[k], 1)] = i;
-    }
-    __syncthreads();
-    if (n > BIN_CAP) cellfix_range(b, s, n);
 }
 
 // ---------------------------------------------------------------- permute (+ integrate)
@@ -1341,8 +1346,8 @@ void launch_row_collect(const Bufs &b, const RowOut &row, cudaStream_t s) {
     launch_pdl(k_row_collect, 1, 256, 0, s, b, row);
 }
 
-void launch_sort_bins(const Bufs &b, uint32_t *other, int64_t C, bool step_inc, const RepDev *rep, const Chunk *cch,
-                      int ncch, int part, const StepHead &head, cudaStream_t s) {
+void launch_sort_bins(const Bufs &b, uint32_t *other, int64_t C, bool step_inc, const Chunk *cch, int ncch, int part,
+                      const StepHead &head, cudaStream_t s) {
     const int nb = (int)((C + SCAN_PER_BLOCK - 1) / SCAN_PER_BLOCK), extra = head.row.rep >= 0 ? 1 : 0;
     const bool one = sort_bins_one(C);
     if (part != 1 && !one)
@@ -1350,9 +1355,8 @@ void launch_sort_bins(const Bufs &b, uint32_t *other, int64_t C, bool step_inc, 
                    step_inc ? 1 : 0, b.status, (const int32_t *)nullptr, b, head);
     if (part == 0) return;
     if (one)
-        launch_pdl(k_binfix<true>, ncch + extra, CELL_TPB, 0, s, b, other, rep, cch, nb, (long long)C, step_inc ? 1 : 0,
-                   head);
-    else launch_pdl(k_binfix<false>, ncch, CELL_TPB, 0, s, b, other, rep, cch, nb, (long long)C, 0, StepHead());
+        launch_pdl(k_binfix<true>, ncch + extra, CELL_TPB, 0, s, b, other, cch, nb, (long long)C, step_inc ? 1 : 0, head);
+    else launch_pdl(k_binfix<false>, ncch, CELL_TPB, 0, s, b, other, cch, nb, (long long)C, 0, StepHead());
 }
 
 void launch_permute(const Bufs &b, int cur, const RepDev *rep, const Chunk *bch, int nbch, PermuteMode mode,
