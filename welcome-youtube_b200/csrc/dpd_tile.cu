@@ -26,8 +26,7 @@
 // the next step's sort).  When the step's stats row is wanted (the stats ring),
 // the epilogue also sums the row's terms of the beads it holds and leaves the
 // tile's sums for the next kernel to collect (RowAcc, row_partial).  A tile whose beads do not
-// fit in shared memory computes its owned beads straight from HBM instead
-// (bead_pairs_direct).
+// fit in shared memory is done in parts that do (tile_parts).
 #include <algorithm>
 
 #include "dpd_row.cuh"
@@ -370,8 +369,8 @@ __device__ __forceinline__ float2 finish_bead(const Bufs &b, int cur, const RepD
 #define TILE_MINB 4
 
 // The owned beads of tile td straight from HBM (full-shell sums, bonds, force,
-// next key): the path for a tile too crowded for shared memory (rare; the
-// same bits).  arow: the tile's a_ij table in shared memory.
+// next key): for a row of cells, or with bulk staging a tile, too crowded for
+// shared memory (the same bits).  a: the tile's a_ij table in shared memory.
 template <bool NEXTKEY>
 __device__ void tile_direct(const Bufs &b, int cur, const RepDev &R, const TileDesc &td, const float *a, long long step,
                             float &mb, long long (*rs)[3], uint32_t (*rc)[DPD_MAXT / 2 + 1]) {
@@ -495,32 +494,18 @@ __device__ __forceinline__ void tile_epilogue(const Bufs &b, int cur, const RepD
     }
 }
 
+// The staged tile td: phases 0 to 2 and the epilogue.  False, and nothing done
+// but phase 0, if its beads do not fit in shared memory.  S.a is set.
 template <bool NEXTKEY, int TPB>
-__global__ void __launch_bounds__(TPB, TILE_MINB * 256 / TPB) k_forces_tile(Bufs b, int cur, const RepDev *__restrict__ reps,
-                                                          const TileDesc *__restrict__ tiles, RowOut row) {
-    // The successor may be scheduled only once this grid's CTAs reach their
-    // epilogue: scheduled earlier, its waiting CTAs would hold SM slots that
-    // later tiles need (1 % of the step at 1M beads).
-    pdl_wait();
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    TileSmemT<TPB> &SS = *reinterpret_cast<TileSmemT<TPB> *>(smem_raw);
+__device__ __forceinline__ bool tile_staged(const Bufs &b, int cur, const RepDev &R, const TileDesc td,
+                                            TileSmemT<TPB> &SS, long long step, float &mb, long long (*rs)[3],
+                                            uint32_t (*rc)[DPD_MAXT / 2 + 1]) {
     auto &S = SS.t;
     constexpr int MAXB = TILE_MAXB * (TPB / 256);
-    const TileDesc td = tiles[blockIdx.x];
-    const RepDev &R = reps[td.rep];
     const int ncx = td.ncx, ncy = td.ncy;  // from the tile: the cell starts need no load of R first
     const int LH = td.h + 2, nl = (td.w + 2) * LH;
     const int32_t *__restrict__ cs = b.cstart + td.c0;
     const int tid = (int)threadIdx.x, lane = (int)lane_id(), wq = tid >> 5;
-    const long long step = *b.step;
-    if (tid < DPD_MAXT * DPD_MAXT) S.a[tid] = a_at(R, tid, step);
-    const bool want_row = NEXTKEY && row.rep == td.rep;  // this tile's beads enter the step's stats row
-    long long(*rs)[3] = want_row ? SS.rsum : nullptr;
-    uint32_t(*rc)[DPD_MAXT / 2 + 1] = want_row ? SS.rcnt : nullptr;
-    if (want_row && lane == 0) {  // each warp's slot of the row sums (only that warp's lane 0 writes it)
-        SS.rsum[wq][0] = SS.rsum[wq][1] = SS.rsum[wq][2] = 0;
-        for (int k = 0; k < DPD_MAXT / 2 + 1; k++) SS.rcnt[wq][k] = 0;
-    }
     // ---- phase 0: local cells, their bead counts, exclusive scan
     int cnt = 0, lx = 0, ly = 0, code = 0;
     if (tid < nl) {
@@ -556,35 +541,106 @@ __global__ void __launch_bounds__(TPB, TILE_MINB * 256 / TPB) k_forces_tile(Bufs
         __syncthreads();
     }
     const int n = S.n;
-    float mb = 0.0f;
-    if (n > MAXB) {
-        tile_direct<NEXTKEY>(b, cur, R, td, S.a, step, mb, rs, rc);
-    } else {
-        // per local cell: its beads' cell and image code
-        if (tid < nl)
-            for (int k = before; k < before + cnt; k++) {
-                S.lxy[k] = (uint16_t)((lx << 8) | ly);
-                S.img[k] = (uint8_t)code;
-            }
-        __syncthreads();
-        // copy in: consecutive beads of a column are consecutive in HBM
-        // (coalesced); every copy of a thread is issued before it waits
-        for (int k = tid; k < n; k += TPB) {
-            const int v = S.lxy[k], l = (v >> 8) * LH + (v & 255);
-            const int g = S.gst[l] + (k - S.lcs[l]);
-            cp_async8(&S.pos[k], b.pos[cur] + g);
-            cp_async8(&S.vt[k], b.vt[cur] + g);
-            cp_async4(&S.tg[k], b.tg[cur] + g);
-            S.accx[k] = 0;
-            S.accy[k] = 0;
+    if (n > MAXB) return false;
+    // per local cell: its beads' cell and image code
+    if (tid < nl)
+        for (int k = before; k < before + cnt; k++) {
+            S.lxy[k] = (uint16_t)((lx << 8) | ly);
+            S.img[k] = (uint8_t)code;
         }
-        if (tid == 0) SS.next_chunk = TPB / 32;  // chunk w goes to warp w first
-        cp_async_wait_all();
-        __syncthreads();
-        tile_pairs_any(S, SS.q[wq], &SS.next_chunk, wq, R, td, step, b.status);
-        __syncthreads();
-        pdl_trigger();
-        tile_epilogue<NEXTKEY>(b, cur, R, td, S, mb, rs, rc);
+    __syncthreads();
+    // copy in: consecutive beads of a column are consecutive in HBM
+    // (coalesced); every copy of a thread is issued before it waits
+    for (int k = tid; k < n; k += TPB) {
+        const int v = S.lxy[k], l = (v >> 8) * LH + (v & 255);
+        const int g = S.gst[l] + (k - S.lcs[l]);
+        cp_async8(&S.pos[k], b.pos[cur] + g);
+        cp_async8(&S.vt[k], b.vt[cur] + g);
+        cp_async4(&S.tg[k], b.tg[cur] + g);
+        S.accx[k] = 0;
+        S.accy[k] = 0;
+    }
+    if (tid == 0) SS.next_chunk = TPB / 32;  // chunk w goes to warp w first
+    cp_async_wait_all();
+    __syncthreads();
+    tile_pairs_any(S, SS.q[wq], &SS.next_chunk, wq, R, td, step, b.status);
+    __syncthreads();
+    pdl_trigger();
+    tile_epilogue<NEXTKEY>(b, cur, R, td, S, mb, rs, rc);
+    return true;
+}
+
+// A tile whose beads do not fit in shared memory, in parts that do, one after
+// the other: strips of columns, each in runs of rows.  The rows of a strip are
+// halved at any place, its columns at its start; a row of it that does not fit
+// by then is done straight from HBM.
+// No tile of a soup is that crowded, but all of those of a condensed state may
+// be: 1,048,576 beads at density 6 in a corner of a box of mean density 4 take
+// 170 us, and took 1,009 with every such tile straight from HBM (142 in tiles of
+// 8 x 16 cells, which hold that density but are slower for a soup).
+template <bool NEXTKEY, int TPB>
+__device__ __noinline__ void tile_parts(const Bufs &b, int cur, const RepDev *reps, const TileDesc *tiles,
+                                        const RowOut &row) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    TileSmemT<TPB> &SS = *reinterpret_cast<TileSmemT<TPB> *>(smem_raw);
+    const TileDesc td = tiles[blockIdx.x];
+    const RepDev &R = reps[td.rep];
+    const long long step = *b.step;
+    const bool want_row = NEXTKEY && row.rep == td.rep;
+    long long(*rs)[3] = want_row ? SS.rsum : nullptr;
+    uint32_t(*rc)[DPD_MAXT / 2 + 1] = want_row ? SS.rcnt : nullptr;
+    float mb = 0.0f;
+    TileDesc t = td;
+    int sw = td.w, sh = td.h;
+    for (int x = 0; x < td.w; x += t.w) {
+        t.cx0 = td.cx0 + x;
+        t.w = min(sw, td.w - x);
+        for (int y = 0; y < td.h;) {
+            t.cy0 = td.cy0 + y;
+            t.h = min(sh, td.h - y);
+            __syncthreads();  // (the part before is done with the shared memory)
+            if (tile_staged<NEXTKEY, TPB>(b, cur, R, t, SS, step, mb, rs, rc)) {
+                y += t.h;
+            } else if (t.h > 1 && (y > 0 || t.h >= t.w)) {
+                sh = (t.h + 1) / 2;
+            } else if (y == 0 && t.w > 1) {
+                t.w = sw = (t.w + 1) / 2;
+            } else {
+                tile_direct<NEXTKEY>(b, cur, R, t, SS.t.a, step, mb, rs, rc);
+                y += t.h;
+            }
+        }
+    }
+    max_bond_out(b, td.rep, mb);
+    if (NEXTKEY && row.rep >= 0) row_partial(b, row, SS.rsum, SS.rcnt, want_row);
+}
+
+template <bool NEXTKEY, int TPB>
+__global__ void __launch_bounds__(TPB, TILE_MINB * 256 / TPB)
+    k_forces_tile(const __grid_constant__ Bufs b, int cur, const RepDev *__restrict__ reps,
+                  const TileDesc *__restrict__ tiles, const __grid_constant__ RowOut row) {
+    // The successor may be scheduled only once this grid's CTAs reach their
+    // epilogue: scheduled earlier, its waiting CTAs would hold SM slots that
+    // later tiles need (1 % of the step at 1M beads).
+    pdl_wait();
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    TileSmemT<TPB> &SS = *reinterpret_cast<TileSmemT<TPB> *>(smem_raw);
+    const TileDesc td = tiles[blockIdx.x];
+    const RepDev &R = reps[td.rep];
+    const int tid = (int)threadIdx.x, lane = (int)lane_id(), wq = tid >> 5;
+    const long long step = *b.step;
+    if (tid < DPD_MAXT * DPD_MAXT) SS.t.a[tid] = a_at(R, tid, step);
+    const bool want_row = NEXTKEY && row.rep == td.rep;  // this tile's beads enter the step's stats row
+    long long(*rs)[3] = want_row ? SS.rsum : nullptr;
+    uint32_t(*rc)[DPD_MAXT / 2 + 1] = want_row ? SS.rcnt : nullptr;
+    if (want_row && lane == 0) {  // each warp's slot of the row sums (only that warp's lane 0 writes it)
+        SS.rsum[wq][0] = SS.rsum[wq][1] = SS.rsum[wq][2] = 0;
+        for (int k = 0; k < DPD_MAXT / 2 + 1; k++) SS.rcnt[wq][k] = 0;
+    }
+    float mb = 0.0f;
+    if (!tile_staged<NEXTKEY, TPB>(b, cur, R, td, SS, step, mb, rs, rc)) {
+        tile_parts<NEXTKEY, TPB>(b, cur, reps, tiles, row);
+        return;
     }
     max_bond_out(b, td.rep, mb);
     if (NEXTKEY && row.rep >= 0) row_partial(b, row, SS.rsum, SS.rcnt, want_row);
