@@ -36,6 +36,7 @@
 //  7. per cell: centroid, covariance and convex hull of the lumen pixels
 //     (hull from each pixel row's two ends), the bilayer test and the final
 //     numbering (cells.py:539-611).
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -326,7 +327,12 @@ __device__ __forceinline__ void uf_flatten(int *par, int i) {
 // share no bead, so each needs only its own frontier.  The levels are a loop
 // with barriers of the CTA: as three grid-wide passes, a scan and a read-back
 // per level the walks took 4.1 of the 10.9 ms of a snapshot with 49 vesicles.
-constexpr int WALK_TPB = 512;
+// A membrane of WALK_LARGE beads or more has a cluster of CTAS = WALK_CTAS CTAs,
+// each taking its part of the frontier: a sheet of 638,252 beads takes 16.4 ms
+// (53.1 with one CTA), one of 158,252 6.2 (13.2), one of 15,164 0.9 (1.7).
+// Vesicles of a thousand beads have frontiers of a few dozen and are faster with
+// one CTA: 62 us against 146, 49 of them 167 against 628.
+constexpr int WALK_TPB = 512, WALK_CTAS = 8, WALK_LARGE = 16384;
 struct WalkArgs {
     const int *deg, *off, *adj;
     const double *X, *Y;
@@ -336,28 +342,65 @@ struct WalkArgs {
     double *UX, *UY;
 };
 
+struct WalkShared {
+    int counts[WALK_TPB + 1];
+    int own, team[WALK_CTAS];  // beads reached by this CTA's part, and by each CTA's
+};
+
+// all threads of the membrane's CTAs
+template <int CTAS> __device__ __forceinline__ void walk_sync() {
+    if (CTAS == 1) {
+        __syncthreads();
+    } else {
+        __syncwarp();  // (the cluster's barrier takes whole warps)
+        cooperative_groups::this_cluster().sync();
+    }
+}
+
 // one level: from the nf beads of cur to nxt, LP lanes per bead of cur; returns their number
-template <int LP>
-__device__ __forceinline__ int walk_level(const WalkArgs &w, const int *cur, int *nxt, int nf, int d, int *counts) {
+template <int LP, int CTAS>
+__device__ __forceinline__ int walk_level(const WalkArgs &w, const int *cur, int *nxt, int nf, int d, WalkShared &S) {
     constexpr int PER = WALK_TPB / LP;  // frontier entries a round
     const int tid = (int)threadIdx.x, sub = tid % LP, slot = tid / LP, lane = tid & 31;
     const unsigned group = LP == 32 ? 0xffffffffu : ((1u << (LP & 31)) - 1u) << (lane / LP * LP);
-    for (int k = slot; k < nf; k += PER) {
+    int *counts = S.counts;
+    // this CTA's part of the frontier
+    const int rank = CTAS == 1 ? 0 : (int)(blockIdx.x % CTAS), part = (nf + CTAS - 1) / CTAS;
+    const int k_begin = min(rank * part, nf), k_end = min(k_begin + part, nf);
+    if (tid == 0) S.own = 0;
+    for (int k = k_begin + slot; k < k_end; k += PER) {
         const int u = cur[k], o = w.off[u], m = w.deg[u];
         for (int s = sub; s < m; s += LP) {
             const int v = w.adj[o + s];
             if (v >= 0 && w.level[v] < 0) atomicMin(w.key + v, ((unsigned long long)k << 20) | (unsigned)s);
         }
     }
-    __syncthreads();
-    int run = 0;
-    for (int k0 = 0; k0 < nf; k0 += PER) {
-        const int k = k0 + slot, u = k < nf ? cur[k] : 0, o = w.off[u], m = k < nf ? w.deg[u] : 0;
-        auto won = [&](int s) {  // is this entry and place the one that reaches its bead
-            if (s >= m) return -1;
-            const int v = w.adj[o + s];
-            return v >= 0 && w.level[v] < 0 && __ldcg(w.key + v) == (((unsigned long long)k << 20) | (unsigned)s) ? v : -1;
-        };
+    walk_sync<CTAS>();
+    // the bead that place s of frontier entry k reaches, if it is the first to
+    auto reached = [&](int k, int o, int s) {
+        const int v = w.adj[o + s];
+        return v >= 0 && w.level[v] < 0 && __ldcg(w.key + v) == (((unsigned long long)k << 20) | (unsigned)s) ? v : -1;
+    };
+    int run = 0, total = 0;
+    if (CTAS > 1) {  // the places of the parts before this one's in the next frontier
+        int mine = 0;
+        for (int k = k_begin + slot; k < k_end; k += PER) {
+            const int u = cur[k], o = w.off[u], m = w.deg[u];
+            for (int s = sub; s < m; s += LP) mine += reached(k, o, s) >= 0;
+        }
+        mine = (int)__reduce_add_sync(0xffffffffu, (unsigned)mine);
+        if (lane == 0) atomicAdd(&S.own, mine);
+        __syncthreads();
+        if (tid < CTAS) cooperative_groups::this_cluster().map_shared_rank(&S, tid)->team[rank] = S.own;
+        walk_sync<CTAS>();
+        for (int q = 0; q < CTAS; q++) {
+            run += q < rank ? S.team[q] : 0;
+            total += S.team[q];
+        }
+    }
+    for (int k0 = k_begin; k0 < k_end; k0 += PER) {
+        const int k = k0 + slot, u = k < k_end ? cur[k] : 0, o = w.off[u], m = k < k_end ? w.deg[u] : 0;
+        auto won = [&](int s) { return s < m ? reached(k, o, s) : -1; };
         int mine = 0;
         for (int s = sub; s < m; s += LP) mine += won(s) >= 0;
         if (LP > 1)
@@ -403,25 +446,29 @@ __device__ __forceinline__ int walk_level(const WalkArgs &w, const int *cur, int
         run += counts[PER];
         __syncthreads();
     }
-    return run;
+    if (CTAS == 1) return run;
+    walk_sync<CTAS>();
+    return total;
 }
 
+template <int CTAS>
 __global__ void __launch_bounds__(WALK_TPB) k_walk(const int2 *__restrict__ walk, WalkArgs w, int *F, int *Fn) {
-    __shared__ int counts[WALK_TPB + 1];
-    const int r = walk[blockIdx.x].x;
-    int *cur = F + walk[blockIdx.x].y, *nxt = Fn + walk[blockIdx.x].y;
-    if (threadIdx.x == 0) {
+    __shared__ WalkShared S;
+    const int2 start = walk[blockIdx.x / CTAS];
+    const int r = start.x;
+    int *cur = F + start.y, *nxt = Fn + start.y;
+    if (blockIdx.x % CTAS == 0 && threadIdx.x == 0) {
         w.level[r] = 0;
         w.UX[r] = w.X[r];
         w.UY[r] = w.Y[r];
         cur[0] = r;
     }
-    __syncthreads();
+    walk_sync<CTAS>();
     int nf = 1;
     for (int d = 0; nf > 0; d++) {
         // a small frontier is latency: sixteen lanes take a bead's neighbours together
-        nf = nf <= 4 * (WALK_TPB / 16) ? walk_level<16>(w, cur, nxt, nf, d, counts)
-                                       : walk_level<1>(w, cur, nxt, nf, d, counts);
+        nf = nf <= 4 * CTAS * (WALK_TPB / 16) ? walk_level<16, CTAS>(w, cur, nxt, nf, d, S)
+                                              : walk_level<1, CTAS>(w, cur, nxt, nf, d, S);
         int *t = cur;
         cur = nxt;
         nxt = t;
@@ -832,7 +879,7 @@ void detect(const dpd_cells_cfg &cfg, double L, long long n64, const double *hx,
     c.release(co);
     c.release(ci);
 
-    // breadth-first walks from each membrane's lowest bead, a CTA per membrane
+    // breadth-first walks from each membrane's lowest bead, a CTA or a cluster of them per membrane
     int *rootmin = c.fill<int>(std::max(nagg, 1), 0x7f), *nbead = c.zeros<int>(std::max(nagg, 1));
     c.each(n, [=] __device__(long long i) {
         if (mol[i] < 0 || !CAND[bagg[i]]) return;
@@ -840,19 +887,32 @@ void detect(const dpd_cells_cfg &cfg, double L, long long n64, const double *hx,
         agg_inc(nbead, bagg[i]);
     });
     const std::vector<int> hroot = c.download(rootmin, nagg), hbead = c.download(nbead, nagg);
-    std::vector<int2> walk;  // root and first place of its frontier
+    std::vector<int2> walk, large;  // root and first place of its frontier
+    int place = 0;
     for (int a : cand) {
-        const int at = walk.empty() ? 0 : walk.back().y + hbead[cand[walk.size() - 1]];
-        walk.push_back(make_int2(hroot[a], at));
+        (hbead[a] < WALK_LARGE ? walk : large).push_back(make_int2(hroot[a], place));
+        place += hbead[a];
     }
     int *level = c.fill<int>(n, 0xff);
     unsigned long long *key = c.fill<unsigned long long>(n, 0xff);
     double *UX = c.alloc<double>(n), *UY = c.alloc<double>(n);
     int *F = c.alloc<int>(n), *Fn = c.alloc<int>(n);
-    const int2 *WALK = c.upload(walk);
-    if (ncand) {
-        k_walk<<<ncand, WALK_TPB, 0, c.s>>>(WALK, WalkArgs{dtot, aoff, adj, X, Y, L, level, key, UX, UY}, F, Fn);
+    const WalkArgs wargs{dtot, aoff, adj, X, Y, L, level, key, UX, UY};
+    if (!walk.empty()) {
+        k_walk<1><<<(unsigned)walk.size(), WALK_TPB, 0, c.s>>>(c.upload(walk), wargs, F, Fn);
         CU(cudaGetLastError());
+    }
+    if (!large.empty()) {
+        cudaLaunchAttribute cluster;
+        cluster.id = cudaLaunchAttributeClusterDimension;
+        cluster.val.clusterDim = {WALK_CTAS, 1, 1};
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)large.size() * WALK_CTAS);
+        cfg.blockDim = dim3(WALK_TPB);
+        cfg.stream = c.s;
+        cfg.attrs = &cluster;
+        cfg.numAttrs = 1;
+        CU(cudaLaunchKernelEx(&cfg, k_walk<WALK_CTAS>, (const int2 *)c.upload(large), wargs, F, Fn));
     }
     c.release(key);
     c.release(F);
