@@ -832,15 +832,25 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
         cudaMemsetAsync(gsum, 0, (size_t)nrep * sizeof(double), s);
         k_gsum<<<nbch, BEAD_TPB, 0, s>>>(rep, bch, g, gsum);
     }
-    // Lanes per bead and CTAs an SM: as many lanes as keep all tasks on the GPU at once (a small box is latency), then
-    // few, whose lanes wait less for the fullest list.  us a launch with (lanes, CTAs an SM), density 4:
+    // Lanes per bead and CTAs an SM: as many lanes as keep all tasks on the GPU at once (a small box is latency).  A
+    // larger box is rounds of tasks, of 444 with (4, 3) and of 592 with (2, 4), and one of the latter takes 2.5 of the
+    // former: two lanes where that is less in all, and past six rounds of four.  us a launch with (lanes, CTAs an SM),
+    // density 4:
     //   beads      (8, 2)  (4, 2)  (4, 3)  (2, 2)  (2, 4)
     //   4,096         9.6    12.3    12.7    18.8    20.0
-    //   16,384       15.3    13.8    14.2    18.8    20.2
-    //   25,600       20.0    20.7    16.3    20.7    22.1
-    //   36,864       24.4    20.8    24.6    21.0    22.3
-    //   131,044      67.4    52.4    50.5    52.2    48.8
-    //   1,048,576   492     378     342     331     290
+    //   16,384       15.2    14.0    14.6    19.4    21.0
+    //   25,600       20.3    21.4    16.8    22.2    23.6
+    //   36,864       24.2    20.9    25.5    21.3    22.8
+    //   50,176       32.2    26.8    25.1    30.5    24.2
+    //   65,536       37.0    33.6    32.7    32.5    30.5
+    //   82,944       46.8    42.1    35.1    45.2    49.2
+    //   102,400      55.2    46.3    41.7    43.4    52.0
+    //   131,044      67.2    53.3    53.2    53.5    50.6
+    //   144,400      74.0    60.4    57.8    56.1    53.8
+    //   160,000      83.0    70.1    64.0    70.3    65.4
+    //   179,776      89.2    70.1    67.3    65.9    66.1
+    //   204,304     100.8    78.6    75.3    75.1    70.2
+    //   1,048,576   484     375     339     335     287
     const bool update = up && !mol;  // the branched shapes add their share first
     const AdjUpdate none{};
     auto go = [&](auto kern, int lpb, int per_sm) {
@@ -851,7 +861,8 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
     if (nbch * 8 <= 2 * 148) go(update ? k_force_vjp<8, 2, true> : k_force_vjp<8, 2, false>, 8, 2);
     else if (nbch * 4 <= 2 * 148) go(update ? k_force_vjp<4, 2, true> : k_force_vjp<4, 2, false>, 4, 2);
     else if (nbch * 4 > 3 * 148 && nbch * 2 <= 2 * 148) go(update ? k_force_vjp<2, 2, true> : k_force_vjp<2, 2, false>, 2, 2);
-    else if (nbch <= 600) go(update ? k_force_vjp<4, 3, true> : k_force_vjp<4, 3, false>, 4, 3);
+    else if (nbch <= 666 && 5 * ((nbch * 2 + 591) / 592) > 2 * ((nbch * 4 + 443) / 444))
+        go(update ? k_force_vjp<4, 3, true> : k_force_vjp<4, 3, false>, 4, 3);
     else go(update ? k_force_vjp<2, 4, true> : k_force_vjp<2, 4, false>, 2, 4);
     if (mol) {
         k_mol_vjp<<<nbch, BEAD_TPB, 0, s>>>(sv, rep, bch, mol, g, xbar, grad);
