@@ -44,8 +44,6 @@
 
 #define NGRAD DPD_NGRAD
 
-__device__ __forceinline__ float theta_of(const NoiseKey &nk, uint32_t gi, uint32_t gj) { return pair_theta(nk, gi, gj); }
-
 __device__ __forceinline__ float dot2(float2 u, float2 v) { return u.x * v.x + u.y * v.y; }
 
 // dphi/da (pa) and dphi/dc (pc) of phi = D U(a, c)[da, dc] for an angle term
@@ -164,8 +162,10 @@ __device__ __forceinline__ void adj_update(const AdjUpdate &u, const RepDev &R, 
 // the order of its cells and slots and evaluated by its lanes in turn, so that
 // the noise and the derivative run on lanes that have a pair.  Each pair is
 // evaluated by both of its beads: no atomics on floats, and a bead's terms are
-// added in its list's order, as a thread per bead would add them (the same
-// bits).  The sums of the parameters' gradient are FP64: per lane and pair of
+// added in its list's order: as a thread per bead would add them (the same
+// bits) where a lane's part of the slots is at most the 32 of its word, which is
+// up to 64 candidates with two lanes and 128 with four; beyond that, the lanes'
+// next words follow the first.  The sums of the parameters' gradient are FP64: per lane and pair of
 // types in shared memory for the first four types (no two lanes on one word),
 // through an atomic for the others.
 // A CTA takes a run of consecutive tasks (256 / LPB beads of a chunk) and hands
@@ -179,10 +179,9 @@ __device__ __forceinline__ void adj_update(const AdjUpdate &u, const RepDev &R, 
 // one.  And the fullest list of a warp is 1.6 times the mean.  The same boxes
 // took 939 us (and 82 for the update) with a thread per bead and an FP64 shared
 // atomic per pair; one box 31 against 68, of 16,384: 14 against 60, of 4,096: 10
-// against 61.  Tried: one
-// queue of pairs per warp evaluated by full rounds, its terms summed through
-// shared memory, 504 us (more shared memory, 16 warps an SM); the order of the
-// sum left to the lanes, 397 us.
+// against 61.  Tried: one queue of pairs per warp evaluated by full rounds, its
+// terms summed through shared memory, 504 us (more shared memory, 16 warps an
+// SM); the order of the sum left to the lanes, 397 us.
 template <int LPB, int MINB, bool UPDATE>
 __global__ void __launch_bounds__(VJP_TPB, MINB) k_force_vjp(StateView sv, long long step, const RepDev *__restrict__ reps,
                                                        const Chunk *__restrict__ ch, int ntask,
@@ -860,7 +859,8 @@ void launch_force_vjp(const StateView &sv, long long step, const RepDev *rep, co
     };
     if (nbch * 8 <= 2 * 148) go(update ? k_force_vjp<8, 2, true> : k_force_vjp<8, 2, false>, 8, 2);
     else if (nbch * 4 <= 2 * 148) go(update ? k_force_vjp<4, 2, true> : k_force_vjp<4, 2, false>, 4, 2);
-    else if (nbch * 4 > 3 * 148 && nbch * 2 <= 2 * 148) go(update ? k_force_vjp<2, 2, true> : k_force_vjp<2, 2, false>, 2, 2);
+    else if (nbch * 4 > 3 * 148 && nbch * 2 <= 2 * 148)
+        go(update ? k_force_vjp<2, 2, true> : k_force_vjp<2, 2, false>, 2, 2);
     else if (nbch <= 666 && 5 * ((nbch * 2 + 591) / 592) > 2 * ((nbch * 4 + 443) / 444))
         go(update ? k_force_vjp<4, 3, true> : k_force_vjp<4, 3, false>, 4, 3);
     else go(update ? k_force_vjp<2, 4, true> : k_force_vjp<2, 4, false>, 2, 4);

@@ -9,9 +9,9 @@
 // ends with its lowest slot as root whatever the order of the links; full
 // path compression then gives each bead its root.  The neighbour counts are
 // those of the reference: for every bead of type t, the beads of any type and
-// of type t within 1.0 (self excluded).  Distances are FP64 from the FP32
-// positions with the minimum image, as the reference computes them from its
-// snapshot.
+// of type t within 1.0 (self excluded).  Comparisons are those of FP64 distances
+// from the FP32 positions with the minimum image, as the reference computes them
+// from its snapshot.
 #include "dpd_device.cuh"
 
 namespace {
@@ -54,9 +54,10 @@ __device__ __forceinline__ double exact_r2(float2 pi, float2 pj, double L) {
 // take the slots of its 3 x 3 cells in turn (cells are column-major: three
 // contiguous ranges, two each where the rows wrap).  Squared distances are
 // FP32; one within near_eps of a threshold is taken again in FP64 with the
-// reference's minimum image, so every comparison is the FP64 one.  786,432 beads: k_uf_link 115 us against 168, k_agg_link 105 against 128,
-// with a thread per bead and two FP64 divisions per candidate (what is left is the
-// union-find's own chains).
+// reference's minimum image, so every comparison is the FP64 one.  786,432
+// beads: k_uf_link 115 us against 168, k_agg_link 105 against 128, with a thread
+// per bead and two FP64 divisions per candidate (what is left is the union-find's
+// own chains).
 constexpr int NEAR_LANES = 8;
 
 // Bound of the FP32 error of a squared distance up to about 1: a coordinate

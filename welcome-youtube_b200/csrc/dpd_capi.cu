@@ -89,10 +89,10 @@ struct dpd_handle {
     int cur = 0;
     // force kernel: 0 = cell tiles in shared memory (half shell), 1 = one thread per bead (full shell)
     int force_kernel = 0;      // 0 cell tiles, 1 thread per bead, 2 cell tiles staged by bulk copies
-    int sort_mode = 2;
+    int sort_mode = 2;          // see sort_form
     uint32_t *count2[2] = {nullptr, nullptr};  // counts of next positions, one array per buffer parity
-    int32_t *bins = nullptr;    // the cells' rows of beads (see k_binfix), null where the density is too high for them
-    int tile_threads = 256;    // threads per CTA of the tile kernel (256 or 512: tiles of up to that many local cells)         // 0 two scan passes, 1 one scan pass (k_scan_lb), 2 no second pass (block prefixes in place/cellfix)
+    int32_t *bins = nullptr;    // the cells' rows of beads (see k_binfix), null where the boxes have none
+    int tile_threads = 256;     // threads per CTA of the tile kernel (256 or 512: tiles of up to that many local cells)
     int tile_w = 8, tile_h = 16;
     TileDesc *d_tiles = nullptr;
     int ntiles = 0;
@@ -504,7 +504,8 @@ static Bufs plain_counts(const dpd_handle *h) {
     return b;
 }
 
-// clear the counts (both parities, and the crowded cells' lists) and count the current (or the next) positions of buffer cur of b
+// clear the counts (both parities, and the crowded cells' lists) and count the
+// current (or the next) positions of buffer cur of b
 static void enqueue_keys(dpd_handle *h, const Bufs &b0, int cur, bool next) {
     cudaMemsetAsync(h->count2[0], 0, (h->bins ? 3 : 2) * (size_t)(h->C + 64) * sizeof(uint32_t), h->s);
     launch_keys(at_parity(h, b0, cur), cur, h->d_rep, h->d_bch, h->nbch, next, h->s);
@@ -1833,10 +1834,10 @@ static void window_reverse(dpd_handle *h, AdjBufs &A, const Window &w, const flo
                 launch_rdf_vjp(views, ng, h->d_rep, h->d_bch, h->nbch, w.spec->ta, w.spec->tb, w.spec->nbin, rmax, sig,
                                A.wgt, A.G, N, h->s);
             }
-            const AdjUpdate up{A.X[p], A.V[p], A.F[p], A.X[p ^ 1], A.V[p ^ 1], A.F[p ^ 1], A.seg[s - 1].src,
+            const AdjUpdate up{A.X[p], A.V[p], A.X[p ^ 1], A.V[p ^ 1], A.F[p ^ 1], A.seg[s - 1].src,
                                in_loss ? A.G + (size_t)(g0 - s) * N : nullptr, w.spec->ta, w.spec->tb};
-            launch_force_vjp(seg_view(A, sg, s), w.step0 + k, h->d_rep, h->d_bch, h->nbch, A.F[p], A.xb, A.vb, A.grad, A.gsum, h->nrep,
-                             h->any_stir, mol, h->s, base, &up);
+            launch_force_vjp(seg_view(A, sg, s), w.step0 + k, h->d_rep, h->d_bch, h->nbch, A.F[p], A.xb, A.vb, A.grad,
+                             A.gsum, h->nrep, h->any_stir, mol, h->s, base, &up);
             p ^= 1;
         }
     }

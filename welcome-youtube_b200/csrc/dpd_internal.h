@@ -297,12 +297,13 @@ size_t bulk_smem_bytes();
 void launch_forces_bulk(const Bufs &b, int cur, const RepDev *rep, const TileDesc *tiles, int ntiles,
                         bool next_keys, cudaStream_t s);
 // The adjoint of the Groot-Warren update that made a configuration from the
-// one before: (X, V, F) hold x_bar, vh_bar and F_bar in its slots, (X2, V2, F2)
-// take them in the slots of the configuration before (old slot = src[slot],
-// the step's sort).  G (or null): the loss's own x_bar of this configuration,
-// set for the beads of types ta and tb.
+// one before: (X, V) hold x_bar and vh_bar in its slots (F_bar is the cotangent
+// of the force VJP), (X2, V2, F2) take x_bar, vh_bar and F_bar in the slots of
+// the configuration before (old slot = src[slot], the step's sort).  G (or
+// null): the loss's own x_bar of this configuration, set for the beads of types
+// ta and tb.
 struct AdjUpdate {
-    const float2 *X, *V, *F;
+    const float2 *X, *V;
     float2 *X2, *V2, *F2;
     const int32_t *src;
     const float2 *G;

@@ -1087,7 +1087,7 @@ __device__ __noinline__ int pair_hist_bin(float2 pi, float2 pj, double L, double
 // per pair.
 // GROUP lanes share a bead: one for all beads; for beads of two types, which the
 // CTA lists first, eight, so that lanes are not idle for the other types' beads
-// (the tails of the same configuration: 78 us against 172).
+// (the tails of the same configuration: 75 us against 172).
 template <bool LANES, int GROUP>
 __global__ void __launch_bounds__(BEAD_TPB) k_pair_hist(Bufs b, int cur, const RepDev *__restrict__ reps,
                                                         const Chunk *__restrict__ ch, int rep_index, int ta, int tb,
