@@ -513,7 +513,7 @@ __device__ __forceinline__ void bin_cell(const Bufs &b, int cell, int s, int n) 
 }
 
 // a cell of n > BIN_CAP beads: its row, then its list (the last bead to arrive first), which is left empty
-__device__ __noinline__ void crowded_cell(int32_t *src, int32_t *dest, const int32_t *row, int32_t *last,
+__device__ __forceinline__ void crowded_cell(int32_t *src, int32_t *dest, const int32_t *row, int32_t *last,
                                           const int32_t *next, int s, int n, DevStatus *status) {
     for (int k = 0; k < BIN_CAP; k++) src[s + k] = row[k];
     int q = *last;
@@ -576,10 +576,8 @@ __global__ void __launch_bounds__(CELL_TPB) k_binfix(Bufs b, uint32_t *__restric
     if (act) {
         b.cstart[cell] = s;
         if (cell + 1 == C) b.cstart[C] = s + n;
-        if (n > BIN_CAP) {
-            crowded_cell(b.src, b.dest, b.bins + (size_t)cell * BIN_CAP, b.crowd + cell, b.crowd_next, s, n, b.status);
-        } else if (n > 16) {
-            bin_cell<32>(b, cell, s, n);
+        if (n > 16) {
+            if (n <= BIN_CAP) bin_cell<32>(b, cell, s, n);
         } else if (n > 8) {
             bin_cell<16>(b, cell, s, n);
         } else if (n > 4) {
@@ -588,6 +586,8 @@ __global__ void __launch_bounds__(CELL_TPB) k_binfix(Bufs b, uint32_t *__restric
             bin_cell<4>(b, cell, s, n);
         }
     }
+    if (n > BIN_CAP)
+        crowded_cell(b.src, b.dest, b.bins + (size_t)cell * BIN_CAP, b.crowd + cell, b.crowd_next, s, n, b.status);
 }
 
 // ---------------------------------------------------------------- permute (+ integrate)
