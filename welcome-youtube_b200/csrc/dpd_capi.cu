@@ -761,14 +761,15 @@ static int ensure_replica(const dpd_handle *h, int r) {
 
 struct ArrayArg {
     const void *p;
-    size_t bytes;
+    size_t bytes, align;
 };
 
 // Are all of these (null ones aside) arrays in one allocation each on the
 // handle's device, aligned for its kernels?  They can then be read or written
 // in place; anything else goes through the staging arrays and copies that take
 // any pointer, and that refuse an array which is shorter than the replica.
-static bool on_device(const dpd_handle *h, std::initializer_list<ArrayArg> args, size_t align) {
+// An array in the allocation of the one before needs no lookup (0.3 us).
+static bool on_device(const dpd_handle *h, std::initializer_list<ArrayArg> args) {
     static const auto attributes = [] {
         void *f = nullptr;
         cudaDriverEntryPointQueryResult found;
@@ -779,22 +780,25 @@ static bool on_device(const dpd_handle *h, std::initializer_list<ArrayArg> args,
         return (decltype(&cuPointerGetAttributes))f;
     }();
     if (!attributes) return false;
+    CUdeviceptr start = 0;
+    size_t size = 0;
     for (const ArrayArg &a : args) {
         if (!a.p) continue;
+        if ((uintptr_t)a.p % a.align != 0) return false;
+        auto inside = [&] {
+            const size_t at = (size_t)((CUdeviceptr)a.p - start);  // (wraps before the start)
+            return at <= size && size - at >= a.bytes;
+        };
+        if (size && inside()) continue;
         unsigned type = 0, managed = 0;
         int dev = -1;
-        CUdeviceptr start = 0;
-        size_t size = 0;
         CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
                                       CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
                                       CU_POINTER_ATTRIBUTE_RANGE_SIZE};
         void *got[] = {&type, &managed, &dev, &start, &size};
-        if ((uintptr_t)a.p % align != 0 ||
-            attributes(sizeof(what) / sizeof(what[0]), what, got, (CUdeviceptr)a.p) != CUDA_SUCCESS ||
-            type != CU_MEMORYTYPE_DEVICE || managed || dev != h->dev)
+        if (attributes(sizeof(what) / sizeof(what[0]), what, got, (CUdeviceptr)a.p) != CUDA_SUCCESS ||
+            type != CU_MEMORYTYPE_DEVICE || managed || dev != h->dev || !inside())
             return false;
-        const size_t at = (size_t)((CUdeviceptr)a.p - start);
-        if (at > size || size - at < a.bytes) return false;
     }
     return true;
 }
@@ -812,8 +816,8 @@ extern "C" int dpd_set_state(dpd_handle *h, int32_t r, const float *x, const flo
     int32_t *sp = (int32_t *)(p + 5 * a), *sn = (int32_t *)(p + 6 * a);
     uint8_t *st = (uint8_t *)(p + 7 * a);
     const size_t w = n * 4;
-    if (on_device(h, {{x, w}, {y, w}, {vx, w}, {vy, w}, {gid, w}, {prev, w}, {next, w}}, 4) &&
-        on_device(h, {{type, n}}, 1)) {
+    if (on_device(h, {{x, w, 4}, {y, w, 4}, {vx, w, 4}, {vy, w, 4}, {type, n, 1}, {gid, w, 4}, {prev, w, 4},
+                      {next, w, 4}})) {
         launch_pack(h->b, h->cur, R.b0, (int)n, R.L, x, y, vx, vy, type, gid, prev, next, h->s);
     } else {
         CK(cudaMemcpyAsync(sx, x, n * 4, cudaMemcpyDefault, h->s));
@@ -848,9 +852,8 @@ extern "C" int dpd_get_state(dpd_handle *h, int32_t r, float *x, float *y, float
     const RepDev &R = h->rh[r];
     const size_t n = (size_t)R.n, a = ((n * 4 + 255) / 256) * 256;
     const size_t w = n * 4;
-    if (on_device(h, {{x, w}, {y, w}, {vhx, w}, {vhy, w}, {vtx, w}, {vty, w}, {fx, w}, {fy, w}, {gid, w}, {prev, w},
-                      {next, w}}, 4) &&
-        on_device(h, {{type, n}}, 1)) {
+    if (on_device(h, {{x, w, 4}, {y, w, 4}, {vhx, w, 4}, {vhy, w, 4}, {vtx, w, 4}, {vty, w, 4}, {fx, w, 4}, {fy, w, 4},
+                      {type, n, 1}, {gid, w, 4}, {prev, w, 4}, {next, w, 4}})) {
         launch_unpack(h->b, h->cur, R.b0, (int)n, x, y, vhx, vhy, vtx, vty, fx, fy, type, gid, prev, next, h->s);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(h->s));
@@ -2126,7 +2129,7 @@ extern "C" int dpd_force_vjp(dpd_handle *h, int32_t r, int64_t step, const float
     CK(cudaMemsetAsync(A.grad, 0, (size_t)h->nrep * DPD_NGRAD * sizeof(double), h->s));
     if (h->nrep > 1) CK(cudaMemsetAsync(A.F[0], 0, N * sizeof(float2), h->s));  // the other replicas' cotangents
     const float *sx = gx, *sy = gy;
-    if (!on_device(h, {{gx, n * 4}, {gy, n * 4}}, 4)) {
+    if (!on_device(h, {{gx, n * 4, 4}, {gy, n * 4, 4}})) {
         sx = (float *)h->stage;
         sy = (float *)(h->stage + a);
         CK(cudaMemcpyAsync(h->stage, gx, n * 4, cudaMemcpyDefault, h->s));
@@ -2141,7 +2144,8 @@ extern "C" int dpd_force_vjp(dpd_handle *h, int32_t r, int64_t step, const float
     CK(cudaGetLastError());
     float *outs[4] = {xbar_x, xbar_y, vbar_x, vbar_y};
     float *st[4];
-    const bool direct = on_device(h, {{outs[0], n * 4}, {outs[1], n * 4}, {outs[2], n * 4}, {outs[3], n * 4}}, 4);
+    const bool direct =
+        on_device(h, {{outs[0], n * 4, 4}, {outs[1], n * 4, 4}, {outs[2], n * 4, 4}, {outs[3], n * 4, 4}});
     for (int k = 0; k < 4; k++) st[k] = direct ? outs[k] : (float *)(h->stage + k * a);
     Bufs w = h->b;
     w.f[h->cur] = A.xb;
