@@ -507,7 +507,7 @@ static Bufs plain_counts(const dpd_handle *h) {
 // clear the counts (both parities, and the crowded cells' lists) and count the
 // current (or the next) positions of buffer cur of b
 static void enqueue_keys(dpd_handle *h, const Bufs &b0, int cur, bool next) {
-    cudaMemsetAsync(h->count2[0], 0, (h->bins ? 3 : 2) * (size_t)(h->C + 64) * sizeof(uint32_t), h->s);
+    cudaMemsetAsync(h->count2[0], 0, (h->bins ? 3 : 2) * (size_t)CELL_WORDS(h->C) * sizeof(uint32_t), h->s);
     launch_keys(at_parity(h, b0, cur), cur, h->d_rep, h->d_bch, h->nbch, next, h->s);
 }
 
@@ -595,12 +595,9 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
     double dense = 0.0;
     for (int r = 0; r < nrep; r++) dense = std::max(dense, (double)h->rh[r].n / h->rh[r].ncell);
     const bool bins = dense <= 10.0 && C <= 196608;
-    if (bins) {
-        want(&h->bins, C * BIN_CAP);
-        want(&b.crowd_next, N);
-    }
-    // (both parities and the crowded cells in one array, cleared together; each begins on a 16-byte boundary)
-    want(&h->count2[0], (bins ? 3 : 2) * (C + 64));
+    // the counts of both parities and, with bins, the crowded cells' lists (these are cleared together), the rows and
+    // the lists' links: one array, each part on a 16-byte boundary
+    want(&h->count2[0], bins ? 3 * CELL_WORDS(C) + C * BIN_CAP + N : 2 * CELL_WORDS(C));
     want(&b.cstart, C + 4);
     want(&b.bsum, C / SCAN_PER_BLOCK + 2);
     want(&b.scan_state, C / SCAN_PER_BLOCK + 2);
@@ -664,8 +661,9 @@ static int create_impl(dpd_handle *h, const dpd_params *params, int32_t nrep, co
         *q.first = base;
         base += (q.second + 64 + 255) & ~(size_t)255;
     }
-    h->count2[1] = h->count2[0] + (C + 64) / 4 * 4;
-    if (bins) b.crowd = (int32_t *)(h->count2[1] + (C + 64) / 4 * 4);
+    h->count2[1] = h->count2[0] + CELL_WORDS(C);
+    if (bins) h->bins = (int32_t *)(h->count2[1] + 2 * CELL_WORDS(C));
+    b.cells = (int32_t)C;
     b.jump = dj;
     b.mol = dm;
     CK(cudaMemcpy(h->d_rep, h->rh.data(), nrep * sizeof(RepDev), cudaMemcpyHostToDevice));

@@ -341,6 +341,12 @@ __device__ __forceinline__ bool last_cta(unsigned int *done) {
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
+// Beads past the end of their cell's row of bins are in a list of the cell's.
+// Before the rows, per cell: slot + 1 of the last of them to arrive (0: none);
+// behind the rows, per slot: the one that arrived before it.
+__device__ __forceinline__ int32_t *bin_last(const Bufs &b, int cell) { return b.bins - CELL_WORDS(b.cells) + cell; }
+__device__ __forceinline__ int32_t *bin_next(const Bufs &b) { return b.bins + (size_t)b.cells * BIN_CAP; }
+
 // Count a bead (slot) into its next cell and, with bins, put it into the
 // cell's row at the place the count gives (in arrival order; k_binfix puts the
 // row in slot order), or, past the row's end, into the cell's list.  Without
@@ -350,7 +356,7 @@ __device__ __forceinline__ void count_key(const Bufs &b, uint32_t key, int slot,
     if (b.bins) {
         const uint32_t r = atomicAdd(b.count + key, 1u);
         if (r < BIN_CAP) b.bins[(size_t)key * BIN_CAP + r] = slot;
-        else b.crowd_next[slot] = atomicExch(b.crowd + key, slot + 1);
+        else bin_next(b)[slot] = atomicExch(bin_last(b, (int)key), slot + 1);
     } else {
         atomicAdd(b.count + key, 1u);
     }

@@ -31,6 +31,8 @@
 #define SCAN_PER_THREAD 4
 #define SCAN_PER_BLOCK (SCAN_TPB * SCAN_PER_THREAD)
 #define BIN_CAP 32              // beads a cell's row of bins holds
+// elements of one of the handle's arrays of cell counts, and of the crowded cells' lists before the bins
+#define CELL_WORDS(C) (((C) + 64) / 4 * 4)
 
 // status flags raised by kernels (read back once per API call)
 #define DPD_F_OUTSIDE 0x1u      // a bead left [0, L) after integration
@@ -154,6 +156,7 @@ struct StepHead {
     int32_t nstir = 0;
 };
 
+// Most kernels get these by value.  At 448 bytes a call of two launches took 0.8 us more than at 432.
 struct Bufs {
     float2 *pos[2], *vh[2], *vt[2], *f[2];
     uint32_t *tg[2];
@@ -162,8 +165,7 @@ struct Bufs {
     uint32_t *fill;             // per cell: next free slot while beads are placed (cstart + count so far)
     int32_t *src, *dest;
     uint32_t *count;            // the counts the next force kernel makes or the next sort reads (one array per parity)
-    int32_t *bins;              // per cell BIN_CAP slots: the beads counted into it, or null (see k_binfix)
-    int32_t *crowd, *crowd_next;  // per cell: slot + 1 of the last bead past its row (0: none); per slot: the one before
+    int32_t *bins;              // per cell BIN_CAP slots: the beads counted into it, or null (see k_binfix, bin_last)
     int32_t *cstart;            // C + 1
     int32_t *bsum;              // scan block totals
     unsigned long long *scan_state;   // single-pass scan: per block (epoch | flag | value), see k_scan_lb
@@ -174,6 +176,7 @@ struct Bufs {
     int2 *bond_list;            // (slot, replica) of T beads whose bonding draw succeeded
     EventDev *events;
     int32_t evcap;
+    int32_t cells;              // of all replicas
     DevStatus *status;
     long long *step;            // step number of the forces being computed
     unsigned long long *obs;    // OBS_N per replica: the running sums (zero between stats rows)

@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(CELL_TPB) k_binfix(Bufs b, uint32_t *__restric
         }
     }
     if (n > BIN_CAP)
-        crowded_cell(b.src, b.dest, b.bins + (size_t)cell * BIN_CAP, b.crowd + cell, b.crowd_next, s, n, b.status);
+        crowded_cell(b.src, b.dest, b.bins + (size_t)cell * BIN_CAP, bin_last(b, cell), bin_next(b), s, n, b.status);
 }
 
 // ---------------------------------------------------------------- permute (+ integrate)
