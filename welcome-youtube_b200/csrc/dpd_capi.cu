@@ -1724,17 +1724,17 @@ static int window_setup(dpd_handle *h, int ckpt, Window &w, AdjBufs &A) {
     const size_t N = (size_t)h->N, cells = adj_place((size_t)(h->C + 1) * sizeof(int32_t));
     const size_t vec = adj_place(N * sizeof(float2)), word = adj_place(N * sizeof(uint32_t));
     const size_t ck_bytes = 5 * vec + word + cells, seg_bytes = 3 * vec + 2 * word + cells;
-    const size_t g_bytes = N * sizeof(float2);
+    auto g_bytes = [&](int64_t ng) { return adj_place((size_t)ng * N * sizeof(float2)); };
     const int64_t steps = w.nsteps - w.stop(), batch = std::min(rdf_batch(h->nbch), w.spec->last_steps);
     const size_t asked = (size_t)((w.nsteps + ckpt - 1) / ckpt) * ck_bytes + (size_t)ckpt * seg_bytes;
     auto takes = [&](int nseg, int64_t len) {
-        return (size_t)nseg * ck_bytes + (size_t)len * seg_bytes + (size_t)std::min(len, batch) * g_bytes;
+        return (size_t)nseg * ck_bytes + (size_t)len * seg_bytes + g_bytes(std::min(len, batch));
     };
     size_t may = asked, free_now = 0, total = 0;
     if (h->window_mem >= 0) {
         may = std::max(may, (size_t)h->window_mem);
     } else {
-        const size_t scratch = adj_layout(h, nullptr, 0, 0, 0, w.spec->nbin, A);
+        const size_t scratch = adj_layout(h, nullptr, 0, 0, 0, w.spec->nbin, A) - g_bytes(0);
         const size_t held = h->adj_bytes > scratch ? h->adj_bytes - scratch : 0;
         may = std::max(may, held);
         if (takes(1, steps) > may) {
@@ -1749,8 +1749,8 @@ static int window_setup(dpd_handle *h, int ckpt, Window &w, AdjBufs &A) {
             if (len <= ckpt || (len <= INT_MAX && takes(w.nseg, len) <= may)) break;
         }
         const size_t states = (size_t)w.nseg * ck_bytes + (size_t)w.len * seg_bytes;
-        const size_t room = may > states ? (may - states) / g_bytes : 0;
-        const int ng = (int)std::max<size_t>(1, std::min(room, (size_t)std::min<int64_t>(w.len, batch)));
+        int ng = (int)std::min<int64_t>(w.len, batch);
+        while (ng > 1 && states + g_bytes(ng) > may) ng--;
         const int rc = adj_setup(h, w.nseg, w.len, ng, w.spec->nbin, A);
         if (rc != DPD_E_NOMEM || may == asked) return rc;
         cudaGetLastError();  // the failed allocation's
